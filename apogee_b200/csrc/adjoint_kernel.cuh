@@ -3,18 +3,28 @@
 // A reported peak of pair (d, t) in bin b is z = sum_f D[d,f] conj(H[t,f]) W^(f k)
 // with W = exp(2 pi i / n) and k its lag.  With g the upstream gradient of z in
 // torch's convention (dL/dRe z + i dL/dIm z), z is holomorphic in D and
-// antiholomorphic in H, so
+// antiholomorphic in H, so with V_dt[f] = sum_b conj(g_dtb) W^(f k_dtb)
 //
-//   grad_D[d, f] = sum_t sum_b  g_dtb       H[t, f] W^(-f k_dtb)
-//   grad_H[t, f] = sum_d sum_b  conj(g_dtb) D[d, f] W^(+f k_dtb)
+//   grad_D[d, f] = sum_t conj(V_dt[f]) H[t, f]
+//   grad_H[t, f] = sum_d      V_dt[f]  D[d, f]
 //
-// One kernel serves both: "own" rows are the ones written (d for grad_D, t for
-// grad_H), "other" rows are summed over.  Each thread owns frequencies f and
-// f + n/2, whose twiddles differ by (-1)^k, and OC own rows; the (lag,
-// gradient) entries of the CTA's rows are staged in shared memory in rounds,
-// read as broadcasts.  Twiddles come from FP64-built hi/lo tables in shared
-// memory: W^m = hi[m >> lo_bits] * lo[m & (2^lo_bits - 1)].  The lags are the
-// forward pass's argmax lags; nothing of the correlation series is stored.
+// V is the transform of a sequence with one entry per peak.  A thread owns
+// the 16 frequencies f0 + j n/16, for which W^(f k) = W^(f0 k) e^(2 pi i j k/16):
+// the entries are summed into 16 buckets by k mod 16, each entry costing one
+// twiddled add whatever the number of frequencies, and one 16-point transform
+// of the buckets gives V at all 16.  (Evaluating every entry at every
+// frequency, two frequencies per twiddle, is about five times the arithmetic
+// at 16 entries per pair.)
+//
+// One kernel serves both gradients: "own" rows are the ones written (d for
+// grad_D, t for grad_H), "other" rows are summed over.  A CTA covers F =
+// min(n/16, 256) values of f0 for 256/F own rows.  Entries are staged in
+// rounds: a warp sorts one (own, other) row's entries by bucket, then the CTA
+// tabulates W^(l k) for the 32 lanes l and conj(g) W^((F x + 32 a) k) for its
+// groups a of 32 lanes, so the inner loop is two shared-memory reads (the
+// second a broadcast) and four FMAs per entry.  Rows without a peak are
+// skipped.  The lags are the forward pass's argmax lags; nothing of the
+// correlation series is stored.
 #pragma once
 #include <cstdint>
 #include "fft_radix.cuh"
@@ -22,8 +32,10 @@
 namespace mfb {
 
 constexpr int ADJ_THREADS = 256;
-constexpr int ADJ_CAP = 2048;   // staged (lag, gradient) entries per round
-constexpr int ADJ_TW = 1024;    // entries of each twiddle half-table (n <= 2^20)
+constexpr int ADJ_R = 16;              // frequencies per thread = buckets
+constexpr int ADJ_CHUNK = 32;          // entries of one (own, other) row sorted at a time
+constexpr int ADJ_TAB = 40960;         // bytes of staged twiddles per round
+constexpr int ADJ_ITEMS = 1024;        // (own, other, chunk) lists per round
 
 struct AdjArgs {
   const float2 *src;      // other rows [other][n]: templates (grad_D) or data (grad_H)
@@ -32,110 +44,168 @@ struct AdjArgs {
   float2 *out;            // [own][n]
   int n, nd, nt, nb;
   int own, other;
-  int rows_per_round, bins_per_round;
-  int other_per_split;    // other rows per blockIdx.z
-  const float2 *tw_hi, *tw_lo;
-  int lo_bits, hi_count;
-  int accumulate;         // 1: atomicAdd into a zeroed out (other split over blockIdx.z)
+  int fblk, slots;        // f0 values and own rows per CTA (fblk * slots = 256)
+  int fx;                 // blocks of fblk f0 values
+  int chunk;              // entries per list, <= ADJ_CHUNK
+  int chunks;             // lists per (own, other) row: ceil(nb / chunk)
+  int rows_per_round;     // other rows per round when chunks == 1, else 1
+  int lists_per_round;    // lists of one row per round when chunks > 1, else 1
+  int other_per_split;    // other rows per blockIdx.y
+  int accumulate;         // 1: atomicAdd into a zeroed out (other split over blockIdx.y)
 };
 
-template <int OC, bool GRAD_DATA>
-__global__ void __launch_bounds__(ADJ_THREADS) adjoint_kernel(const AdjArgs a) {
-  __shared__ float2 s_hi[ADJ_TW], s_lo[ADJ_TW];
-  __shared__ int s_k[ADJ_CAP];
-  __shared__ float2 s_g[ADJ_CAP];
-  const int half = a.n >> 1;
-  const int f = blockIdx.x * ADJ_THREADS + threadIdx.x;
-  const int j0 = blockIdx.y * OC;
-  const int ob = blockIdx.z * a.other_per_split;
+// Bytes of staged twiddles per entry: min(fblk, 32) lane values, one value
+// per group of 32 f0.
+__host__ __device__ constexpr int adj_entry_bytes(int fblk) {
+  return 8 * ((fblk < 32 ? fblk : 32) + (fblk + 31) / 32);
+}
+
+__device__ __forceinline__ cf adj_root(unsigned m, float two_over_n) {   // W^m, m < n: exact argument
+  cf w;
+  sincospif((float)m * two_over_n, &w.y, &w.x);
+  return w;
+}
+
+template <bool GRAD_DATA>
+__global__ void __launch_bounds__(ADJ_THREADS, 2) adjoint_kernel(const AdjArgs a) {
+  extern __shared__ __align__(16) unsigned char adj_smem[];
+  const int L = a.fblk < 32 ? a.fblk : 32, A = (a.fblk + 31) >> 5;
+  const int per_item = a.chunk;
+  const int cap = ADJ_TAB / adj_entry_bytes(a.fblk);          // entries per round
+  float2 *lane_tw = reinterpret_cast<float2 *>(adj_smem);      // [cap][L]
+  float2 *group_tw = lane_tw + cap * L;                        // [cap][A]
+  float2 *s_g = group_tw + cap * A;                            // [cap] conj(g), sorted
+  int *s_k = reinterpret_cast<int *>(s_g + cap);               // [cap] lags, sorted
+  uint4 *s_end = reinterpret_cast<uint4 *>(                    // [items] bucket ends, one byte each
+      (reinterpret_cast<uintptr_t>(s_k + cap) + 15) & ~uintptr_t(15));
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int fb = blockIdx.x % a.fx, oc = blockIdx.x / a.fx;
+  const int i = tid & (a.fblk - 1), slot = tid / a.fblk;       // fblk is a power of two
+  const int l = i & 31, grp = i >> 5;
+  const int own_row = oc * a.slots + slot;
+  const int sixteenth = a.n >> 4;
+  const int f0 = fb * a.fblk + i;
+  const int ob = blockIdx.y * a.other_per_split;
   const int oe = min(a.other, ob + a.other_per_split);
-  const unsigned mask_n = (unsigned)a.n - 1u, lo_mask = (1u << a.lo_bits) - 1u;
-  for (int i = threadIdx.x; i < a.hi_count; i += ADJ_THREADS) s_hi[i] = a.tw_hi[i];
-  for (int i = threadIdx.x; i <= (int)lo_mask; i += ADJ_THREADS) s_lo[i] = a.tw_lo[i];
-  cf acc0[OC], acc1[OC];
+  const unsigned mask_n = (unsigned)a.n - 1u;
+  const float two_over_n = 2.0f / (float)a.n;
+  const bool live = own_row < a.own;
+
+  cf acc[ADJ_R];
 #pragma unroll
-  for (int j = 0; j < OC; j++) acc0[j] = acc1[j] = cf{0.f, 0.f};
+  for (int j = 0; j < ADJ_R; j++) acc[j] = {0.f, 0.f};
 
   for (int o0 = ob; o0 < oe; o0 += a.rows_per_round) {
     const int rr = min(a.rows_per_round, oe - o0);
-    for (int b0 = 0; b0 < a.nb; b0 += a.bins_per_round) {
-      const int bc = min(a.bins_per_round, a.nb - b0);
-      const int per_row = OC * bc, total = rr * per_row;
-      __syncthreads();   // the previous round's readers are done (and the tables are in)
-      for (int e = threadIdx.x; e < total; e += ADJ_THREADS) {
-        const int ol = e / per_row, rem = e - ol * per_row;
-        const int jj = rem / bc, bl = rem - jj * bc;
-        int k = 0;
+    cf S[ADJ_R];
+    int seen = 0;                       // entries of the row so far (rows of several rounds)
+    for (int c0 = 0; c0 < a.chunks; c0 += a.lists_per_round) {
+      const int lc = min(a.lists_per_round, a.chunks - c0);
+      const int items = rr * lc * a.slots;             // list (o, chunk, slot): slot fastest
+      __syncthreads();                                 // the previous round's readers are done
+      // ---- each warp sorts whole lists by k mod 16 --------------------------------
+      for (int it = warp; it < items; it += ADJ_THREADS / 32) {
+        const int s = it % a.slots, oq = it / a.slots;
+        const int cl = oq % lc, o = o0 + oq / lc, mine = oc * a.slots + s;
+        const int b = (c0 + cl) * a.chunk + lane;
+        int k = -1;
         float2 g = make_float2(0.f, 0.f);
-        const int own_row = j0 + jj;
-        if (own_row < a.own) {
-          const int o = o0 + ol;
-          const int d = GRAD_DATA ? own_row : o, t = GRAD_DATA ? o : own_row;
-          const long long i = ((long long)d * a.nt + t) * a.nb + b0 + bl;
-          const long long kk = a.idx[i];
+        if (lane < a.chunk && b < a.nb && mine < a.own) {
+          const int d = GRAD_DATA ? mine : o, t = GRAD_DATA ? o : mine;
+          const long long at = ((long long)d * a.nt + t) * a.nb + b;
+          const long long kk = a.idx[at];
           if (kk >= 0) {
-            k = (int)kk;
-            g = a.gz[i];
-            if (!GRAD_DATA) g.y = -g.y;   // conj(g)
+            k = (int)(kk & mask_n);
+            g = a.gz[at];
+            g.y = -g.y;
           }
         }
-        s_k[e] = k;
-        s_g[e] = g;
+        const int c = k >= 0 ? (k & (ADJ_R - 1)) : ADJ_R;
+        unsigned ends[4] = {0u, 0u, 0u, 0u};
+        int before = 0, pos = 0;
+#pragma unroll
+        for (int q = 0; q < ADJ_R; q++) {
+          const unsigned m = __ballot_sync(0xffffffffu, c == q);
+          if (c == q) pos = before + __popc(m & ((1u << lane) - 1u));
+          before += __popc(m);
+          ends[q >> 2] |= (unsigned)before << (8 * (q & 3));
+        }
+        if (k >= 0) {
+          s_k[it * per_item + pos] = k;
+          s_g[it * per_item + pos] = g;
+        }
+        if (lane >= before && lane < a.chunk) s_k[it * per_item + lane] = -1;
+        if (lane == 0) s_end[it] = make_uint4(ends[0], ends[1], ends[2], ends[3]);
       }
       __syncthreads();
-      if (f < half) {
-        for (int ol = 0; ol < rr; ol++) {
-          const float2 *sp = a.src + (long long)(o0 + ol) * a.n;
-          const float2 s0 = __ldg(sp + f), s1 = __ldg(sp + f + half);
+      // ---- twiddle tables of every staged entry ------------------------------------
+      for (int x = tid; x < items * per_item * L; x += ADJ_THREADS) {
+        const int e = x / L, j = x & (L - 1);
+        const int k = s_k[e];
+        if (k < 0) continue;
+        const cf w = adj_root(((unsigned)j * (unsigned)k) & mask_n, two_over_n);
+        lane_tw[x] = make_float2(w.x, w.y);
+      }
+      for (int x = tid; x < items * per_item * A; x += ADJ_THREADS) {
+        const int e = x / A, j = x & (A - 1);
+        const int k = s_k[e];
+        if (k < 0) continue;
+        const float2 g = s_g[e];
+        const cf w = cmul(cf{g.x, g.y}, adj_root(((unsigned)(fb * a.fblk + 32 * j) * (unsigned)k) & mask_n,
+                                                 two_over_n));
+        group_tw[x] = make_float2(w.x, w.y);
+      }
+      __syncthreads();
+      // ---- V at this thread's 16 frequencies, times the other row ---------------------
+      for (int ol = 0; ol < rr; ol++) {
+        if (c0 == 0) {
+          seen = 0;
 #pragma unroll
-          for (int jj = 0; jj < OC; jj++) {
-            cf u0 = {0.f, 0.f}, u1 = {0.f, 0.f};
-            const int eb = (ol * OC + jj) * bc;
-            for (int bl = 0; bl < bc; bl++) {
-              const int k = s_k[eb + bl];
-              const float2 g = s_g[eb + bl];
-              const unsigned m = ((unsigned)f * (unsigned)k) & mask_n;
-              const float2 wh = s_hi[m >> a.lo_bits], wl = s_lo[m & lo_mask];
-              const float wr = fmaf(wh.x, wl.x, -wh.y * wl.y);
-              const float wi = fmaf(wh.x, wl.y, wh.y * wl.x);
-              float tr, ti;
-              if (GRAD_DATA) {           // g * conj(W^(fk))
-                tr = fmaf(g.x, wr, g.y * wi);
-                ti = fmaf(g.y, wr, -g.x * wi);
-              } else {                   // conj(g) * W^(fk)
-                tr = fmaf(g.x, wr, -g.y * wi);
-                ti = fmaf(g.x, wi, g.y * wr);
-              }
-              const float sgn = (k & 1) ? -1.f : 1.f;   // W^((f + n/2) k) = (-1)^k W^(fk)
-              u0.x += tr;
-              u0.y += ti;
-              u1.x = fmaf(sgn, tr, u1.x);
-              u1.y = fmaf(sgn, ti, u1.y);
+          for (int j = 0; j < ADJ_R; j++) S[j] = {0.f, 0.f};
+        }
+        for (int cl = 0; cl < lc; cl++) {
+          const int it = (ol * lc + cl) * a.slots + slot;
+          const uint4 ends = s_end[it];
+          const unsigned ew[4] = {ends.x, ends.y, ends.z, ends.w};
+          const float2 *p1 = lane_tw + (it * per_item) * L + l;
+          const float2 *p2 = group_tw + (it * per_item) * A + grp;
+          int e = 0;
+#pragma unroll
+          for (int q = 0; q < ADJ_R; q++) {
+            const int end = (int)((ew[q >> 2] >> (8 * (q & 3))) & 255u);
+            for (; e < end; e++) {
+              const float2 w = p1[e * L], h = p2[e * A];
+              S[q].x = fmaf(w.x, h.x, fmaf(-w.y, h.y, S[q].x));
+              S[q].y = fmaf(w.x, h.y, fmaf(w.y, h.x, S[q].y));
             }
-            acc0[jj].x = fmaf(s0.x, u0.x, fmaf(-s0.y, u0.y, acc0[jj].x));
-            acc0[jj].y = fmaf(s0.x, u0.y, fmaf(s0.y, u0.x, acc0[jj].y));
-            acc1[jj].x = fmaf(s1.x, u1.x, fmaf(-s1.y, u1.y, acc1[jj].x));
-            acc1[jj].y = fmaf(s1.x, u1.y, fmaf(s1.y, u1.x, acc1[jj].y));
+          }
+          seen += e;
+        }
+        if (c0 + lc < a.chunks || !live || seen == 0) continue;   // more of this row to come, or nothing
+        dft16(S);
+        const float2 *sp = a.src + (long long)(o0 + ol) * a.n + f0;
+#pragma unroll
+        for (int j = 0; j < ADJ_R; j++) {
+          const float2 h = __ldg(sp + j * sixteenth);
+          if (GRAD_DATA) {                // conj(V) * H
+            acc[j].x = fmaf(S[j].x, h.x, fmaf(S[j].y, h.y, acc[j].x));
+            acc[j].y = fmaf(S[j].x, h.y, fmaf(-S[j].y, h.x, acc[j].y));
+          } else {                        // V * D
+            acc[j].x = fmaf(S[j].x, h.x, fmaf(-S[j].y, h.y, acc[j].x));
+            acc[j].y = fmaf(S[j].x, h.y, fmaf(S[j].y, h.x, acc[j].y));
           }
         }
       }
     }
   }
-  if (f < half) {
+  if (!live) return;
+  float2 *op = a.out + (long long)own_row * a.n + f0;
 #pragma unroll
-    for (int jj = 0; jj < OC; jj++) {
-      if (j0 + jj >= a.own) break;
-      float2 *op = a.out + (long long)(j0 + jj) * a.n;
-      if (a.accumulate) {
-        atomicAdd(&op[f].x, acc0[jj].x);
-        atomicAdd(&op[f].y, acc0[jj].y);
-        atomicAdd(&op[f + half].x, acc1[jj].x);
-        atomicAdd(&op[f + half].y, acc1[jj].y);
-      } else {
-        op[f] = make_float2(acc0[jj].x, acc0[jj].y);
-        op[f + half] = make_float2(acc1[jj].x, acc1[jj].y);
-      }
-    }
+  for (int j = 0; j < ADJ_R; j++) {
+    const float2 v = make_float2(acc[j].x, acc[j].y);
+    if (a.accumulate) atomicAdd(op + j * sixteenth, v);
+    else op[j * sixteenth] = v;
   }
 }
 

@@ -1815,7 +1815,7 @@ extern "C" int mfb_run_large_static(int device, size_t n, const void *data, int 
 }
 
 // ---------------------------------------------------------------- adjoint
-// W_n^m twiddles for the adjoint kernel: hi[m >> lo_bits] * lo[m & mask],
+// W_n^m twiddles for the batched four-step: hi[m >> lo_bits] * lo[m & mask],
 // built once per (device, n) from FP64 roots.
 struct AdjTables {
   float2 *hi = nullptr, *lo = nullptr;
@@ -1843,51 +1843,51 @@ static int get_adj_tables(int device, int n, AdjTables **out) {
   return MFB_OK;
 }
 
-template <bool GD>
-static cudaError_t launch_adjoint(int oc, dim3 grid, const AdjArgs &a, cudaStream_t s) {
-  switch (oc) {
-    case 8: adjoint_kernel<8, GD><<<grid, ADJ_THREADS, 0, s>>>(a); break;
-    case 4: adjoint_kernel<4, GD><<<grid, ADJ_THREADS, 0, s>>>(a); break;
-    case 2: adjoint_kernel<2, GD><<<grid, ADJ_THREADS, 0, s>>>(a); break;
-    default: adjoint_kernel<1, GD><<<grid, ADJ_THREADS, 0, s>>>(a); break;
-  }
-  return cudaGetLastError();
+// Dynamic shared memory of adjoint_kernel: the staged twiddles, the sorted
+// entries and the lists' bucket ends.
+static size_t adjoint_smem(int fblk, int items) {
+  const int cap = ADJ_TAB / adj_entry_bytes(fblk);
+  return (size_t)ADJ_TAB + (size_t)cap * 12 + 16 + (size_t)items * sizeof(uint4);
 }
 
-// One side of the adjoint: own rows per CTA (OC) shrink, and then the summed
-// rows split over blockIdx.z with atomic accumulation, until the grid covers
-// the device about twice.
+// One side of the adjoint: a CTA covers 256 (own row, f0) and all other rows;
+// when that leaves the device less than ADJ_FILL CTAs per SM, the summed rows
+// split over blockIdx.y with atomic accumulation.
+constexpr int ADJ_FILL = 4;
 static int adjoint_side(bool grad_data, int n, int nd, int nt, int nb, const float2 *src,
-                        const int64_t *idx, const float2 *gz, float2 *out, const AdjTables &tw,
-                        int sms, cudaStream_t st) {
+                        const int64_t *idx, const float2 *gz, float2 *out, int sms,
+                        cudaStream_t st) {
   AdjArgs a;
   memset(&a, 0, sizeof a);
   a.src = src; a.idx = idx; a.gz = gz; a.out = out;
   a.n = n; a.nd = nd; a.nt = nt; a.nb = nb;
   a.own = grad_data ? nd : nt;
   a.other = grad_data ? nt : nd;
-  a.tw_hi = tw.hi; a.tw_lo = tw.lo; a.lo_bits = tw.lo_bits; a.hi_count = tw.hi_count;
-  const long long fx = ((n >> 1) + ADJ_THREADS - 1) / ADJ_THREADS;
-  const long long target = 2LL * sms;
-  int oc = 8;
-  while (oc > 1 && fx * ((a.own + oc - 1) / oc) < target) oc >>= 1;
-  const long long chunks = (a.own + oc - 1) / oc;
-  if (chunks > 65535) return fail(MFB_ERR_UNSUPPORTED, "adjoint: too many rows (%d)", a.own);
+  if ((a.own + 7LL) / 8 > 65535) return fail(MFB_ERR_UNSUPPORTED, "adjoint: too many rows (%d)", a.own);
+  a.fblk = std::min(n / ADJ_R, ADJ_THREADS);
+  a.slots = ADJ_THREADS / a.fblk;
+  a.fx = n / ADJ_R / a.fblk;
+  const int cap = ADJ_TAB / adj_entry_bytes(a.fblk);
+  a.chunk = std::min(std::min(nb, ADJ_CHUNK), cap / a.slots);
+  a.chunks = (nb + a.chunk - 1) / a.chunk;
+  const int lists = std::min(cap / (a.chunk * a.slots), ADJ_ITEMS / a.slots);   // per own row and round
+  a.rows_per_round = a.chunks == 1 ? lists : 1;
+  a.lists_per_round = a.chunks == 1 ? 1 : std::min(lists, a.chunks);
+  const long long tiles = (long long)a.fx * ((a.own + a.slots - 1) / a.slots);
+  const long long target = (long long)ADJ_FILL * sms;
   long long split = 1;
-  if (fx * chunks < target) split = std::min<long long>(a.other, (target + fx * chunks - 1) / (fx * chunks));
+  if (tiles < target) split = std::min<long long>(a.other, std::max<long long>(1, target / tiles));
   a.other_per_split = (int)((a.other + split - 1) / split);
   split = (a.other + a.other_per_split - 1) / a.other_per_split;
-  if ((long long)oc * nb <= ADJ_CAP) {
-    a.bins_per_round = nb;
-    a.rows_per_round = ADJ_CAP / (oc * nb);
-  } else {
-    a.bins_per_round = ADJ_CAP / oc;
-    a.rows_per_round = 1;
-  }
   a.accumulate = split > 1;
   if (a.accumulate) CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)a.own * n * sizeof(float2), st));
-  const dim3 grid((unsigned)fx, (unsigned)chunks, (unsigned)split);
-  CUDA_TRY(grad_data ? launch_adjoint<true>(oc, grid, a, st) : launch_adjoint<false>(oc, grid, a, st));
+  const size_t smem = adjoint_smem(a.fblk, lists * a.slots);
+  const dim3 grid((unsigned)tiles, (unsigned)split);
+  // one limit for every shape, so that callers on several threads set the same value
+  auto kernel = grad_data ? adjoint_kernel<true> : adjoint_kernel<false>;
+  CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 << 10));
+  kernel<<<grid, ADJ_THREADS, smem, st>>>(a);
+  CUDA_TRY(cudaGetLastError());
   return MFB_OK;
 }
 
@@ -1901,20 +1901,17 @@ extern "C" int mfb_adjoint(int device, size_t n, const void *data, int nd, const
   CUDA_TRY(cudaGetDeviceCount(&ndev));
   if (device < 0 || device >= ndev) return fail(MFB_ERR_ARG, "no device %d", device);
   DeviceGuard dg(device);
-  AdjTables *tw = nullptr;
-  int r = get_adj_tables(device, (int)n, &tw);
-  if (r) return r;
-  int sms = 0;
+  int r = MFB_OK, sms = 0;
   CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   cudaStream_t st = (cudaStream_t)stream;
   if (grad_data) {
     r = adjoint_side(true, (int)n, nd, nt, (int)nb, (const float2 *)templates, idx,
-                     (const float2 *)gz, (float2 *)grad_data, *tw, sms, st);
+                     (const float2 *)gz, (float2 *)grad_data, sms, st);
     if (r) return r;
   }
   if (grad_tmpl) {
     r = adjoint_side(false, (int)n, nd, nt, (int)nb, (const float2 *)data, idx,
-                     (const float2 *)gz, (float2 *)grad_tmpl, *tw, sms, st);
+                     (const float2 *)gz, (float2 *)grad_tmpl, sms, st);
     if (r) return r;
   }
   return MFB_OK;

@@ -163,3 +163,60 @@ def test_template_parameter_gradient():
     ga, gt = alpha.grad.cpu().numpy(), tc.grad.cpu().numpy()
     np.testing.assert_allclose(ga, fd_a, rtol=0, atol=1e-3 * np.abs(fd_a).max())
     np.testing.assert_allclose(gt, fd_t, rtol=0, atol=1e-3 * np.abs(fd_t).max())
+
+
+def _adjoint_direct(n, nd, nt, nb, seed, peaks):
+    """mfb_adjoint on random lags; both gradients and the FP64 sums they
+    stand for, with the sum of absolute terms behind every output."""
+    import torch
+    from apogee_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    def cplx(*shape):
+        return torch.randn(*shape, dtype=torch.complex64, device="cuda", generator=g)
+    D, H, gz = cplx(nd, n), cplx(nt, n), cplx(nd, nt, nb)
+    idx = torch.randint(0, n, (nd, nt, nb), device="cuda", generator=g)
+    idx[torch.rand(nd, nt, nb, device="cuda", generator=g) >= peaks] = -1
+    gd, gh = torch.full_like(D, float("nan")), torch.full_like(H, float("nan"))
+    _lib.check(_lib.lib().mfb_adjoint(0, n, D.data_ptr(), nd, H.data_ptr(), nt, nb, idx.data_ptr(),
+                                      gz.data_ptr(), gd.data_ptr(), gh.data_ptr(),
+                                      torch.cuda.current_stream().cuda_stream))
+    live = idx >= 0
+    g64 = torch.where(live, gz.to(torch.complex128), torch.zeros((), dtype=torch.complex128, device="cuda"))
+    wd, wh = torch.zeros(nd, n, dtype=torch.complex128, device="cuda"), []
+    ad = torch.zeros(nd, n, dtype=torch.float64, device="cuda")
+    ah = []
+    D64, H64 = D.to(torch.complex128), H.to(torch.complex128)
+    for t in range(nt):
+        s = torch.zeros(nd, n, dtype=torch.complex128, device="cuda")
+        s.scatter_add_(1, idx[:, t].clamp(min=0), g64[:, t])
+        u = torch.fft.fft(s, dim=1)
+        a = g64[:, t].abs().sum(1, keepdim=True)
+        wd += u * H64[t]
+        ad += a * H64[t].abs()
+        wh.append((u.conj() * D64).sum(0))
+        ah.append((a * D64.abs()).sum(0))
+    return (gd, wd, ad), (gh, torch.stack(wh), torch.stack(ah))
+
+
+@pytest.mark.parametrize("n, nd, nt, nb, peaks", [
+    (64, 3, 70, 1, 1.0),        # 4 frequencies per row: 64 own rows per CTA, a ragged last one
+    (64, 65, 2, 64, 0.5),       # every lag a bin: many lists per row
+    (256, 7, 3, 33, 1.0),       # one entry more than a list
+    (512, 2, 5, 32, 0.9),       # lists exactly full
+    (1024, 9, 2, 100, 0.7),     # four own rows per CTA, several lists per row
+    (4096, 1, 1, 1, 1.0),       # one row, one entry
+    (4096, 5, 200, 16, 0.05),   # rows without a peak among the summed ones
+    (8192, 2, 3, 300, 1.0),     # a row's lists in several rounds
+    (16384, 3, 40, 16, 0.0),    # no peak at all
+    (1 << 20, 1, 2, 3, 1.0),    # the longest transform
+])
+def test_adjoint_kernel_edges(n, nd, nt, nb, peaks):
+    """Both gradients against FP64 at the edges of the kernel's lists, rounds
+    and row blocks.  Every output is a sum of g * row * W terms: two twiddles
+    within 2 ulp and three products (12 roundings of at most 2^-24 each),
+    a 16-point transform (8), and as many additions as a row has entries and
+    there are rows -- the bound below, relative to the sum of |g| |row|."""
+    for got, want, scale in _adjoint_direct(n, nd, nt, nb, n + nb, peaks):
+        bound = (24 + nb + max(nd, nt)) * 2.0 ** -24 * scale
+        err = (got.to(want.dtype) - want).abs()
+        assert bool((err <= bound + 1e-30).all()), (n, nd, nt, nb, float((err / scale.clamp(min=1e-30)).max()))
