@@ -234,6 +234,18 @@ __device__ __forceinline__ void inverse_passes(cf *v, float2 *buf, const float2 
   }
 }
 
+// Whether any of the pair slot's threads in this warp (gmask) holds a candidate,
+// |z|^2 > t2.  Above a threshold the usual answer is no, found with three
+// instructions a point; the per-bin reduction then has nothing to do.  At
+// threshold 0 there is always one, and nothing is computed.
+__device__ __forceinline__ bool any_candidate(const cf *v, float t2, bool live, unsigned gmask) {
+  if (!(t2 > 0.f)) return true;
+  float mx = 0.f;
+#pragma unroll
+  for (int q = 0; q < 16; q++) mx = fmaxf(mx, fmaf(v[q].x, v[q].x, v[q].y * v[q].y));
+  return __any_sync(gmask, live && mx > t2);
+}
+
 // Items [ibeg, iend) of one launch's pairs (item i = pairs i*G .. i*G+G-1 of
 // the dense block or the list), processed by one CTA of FlatGeo<N>::CTA
 // threads with `smem` its dynamic shared memory.  CACHE_D keeps a data row
@@ -363,9 +375,10 @@ __device__ __forceinline__ void flat_range(const FlatArgs &a, long long ibeg, lo
     // values that close the lower lag wins.  The same truncation is used for
     // every comparison, across warps too, so the result is deterministic.
     unsigned cand = 0u;
+    const bool want = any_candidate(v, a.t2, live, gmask);
     if (fast) {
       // Whole window, bins a multiple of 32 lags: every warp slot is one bin.
-      if (live) {
+      if (live && want) {
         unsigned mxs[16];
 #pragma unroll
         for (int q = 0; q < 16; q++) {
@@ -393,9 +406,10 @@ __device__ __forceinline__ void flat_range(const FlatArgs &a, long long ibeg, lo
         }
       }
     } else if (small_keys) {
-      // Fast path: one redux per slot and warp; the winning lane parks z[k]
+      // One redux per slot and warp; the winning lane parks z[k]
       // at buf[k] (free after the last pass); 16 lanes then publish the warp's
       // 16 slot winners to the per-bin keys with parallel atomics.
+      if (want) {
       unsigned mxs[16];
 #pragma unroll
       for (int q = 0; q < 16; q++) {
@@ -426,7 +440,8 @@ __device__ __forceinline__ void flat_range(const FlatArgs &a, long long ibeg, lo
           atomicMax(keys + bin, ((unsigned long long)(my & ~31u) << 32) | (unsigned)(~k));
         }
       }
-    } else {
+      }
+    } else if (want) {
       // Many bins (keys occupy buf): per-lane atomics, winners write back below.
 #pragma unroll
       for (int q = 0; q < 16; q++) {
@@ -541,7 +556,12 @@ flat_kernel(const FlatArgs a) {
   const long long ibeg = blockIdx.x * per + (blockIdx.x < extra ? blockIdx.x : extra);
   const long long iend = ibeg + per + (blockIdx.x < extra ? 1 : 0);
 
-  cf dreg[16];
+  // The data row stays in registers while consecutive pairs share it; 1024
+  // threads have 64 registers each, too few for it beside the transform (kept, it
+  // spilled: 149 us for 6 x 300 pairs at n = 16384, threshold 4.5, against 126 us
+  // reloaded from L2).
+  constexpr bool CACHE_D = Geo::CTA <= 512;
+  cf dreg[CACHE_D ? 16 : 1];
   int cur_d = -1;
   const int lane = threadIdx.x & 31;
 
@@ -595,22 +615,25 @@ flat_kernel(const FlatArgs a) {
     // ---- pass 0: load, conjugate product, radix-R0 butterflies ----------
     cf v[16];
     if (live) {
-      if (d != cur_d) {
-        const float2 *dp = a.data + (long long)(a.d0 + d) * a.data_stride;
+      const float2 *dp = a.data + (long long)(a.d0 + d) * a.data_stride;
+      const float2 *hp = a.tmpl + (long long)(a.t0 + tt) * a.tmpl_stride;
+      if (CACHE_D && d != cur_d) {
 #pragma unroll
         for (int s = 0; s < 16; s++) {
           float2 x = __ldg(dp + t + T * s);
-          dreg[s] = {x.x, x.y};
+          dreg[CACHE_D ? s : 0] = {x.x, x.y};
         }
         cur_d = d;
       }
-      const float2 *hp = a.tmpl + (long long)(a.t0 + tt) * a.tmpl_stride;
 #pragma unroll
       for (int s = 0; s < 16; s++) {
         float2 h = __ldg(hp + t + T * s);
+        cf x;
+        if constexpr (CACHE_D) x = dreg[s];
+        else { const float2 y = __ldg(dp + t + T * s); x = {y.x, y.y}; }
         // D * conj(H)
-        v[s].x = fmaf(dreg[s].x, h.x, dreg[s].y * h.y);
-        v[s].y = fmaf(dreg[s].y, h.x, -dreg[s].x * h.y);
+        v[s].x = fmaf(x.x, h.x, x.y * h.y);
+        v[s].y = fmaf(x.y, h.x, -x.x * h.y);
       }
     } else {
 #pragma unroll
@@ -634,9 +657,10 @@ flat_kernel(const FlatArgs a) {
     // values that close the lower lag wins.  The same truncation is used for
     // every comparison, across warps too, so the result is deterministic.
     unsigned cand = 0u;
+    const bool want = any_candidate(v, a.t2, live, gmask);
     if (fast) {
       // Whole window, bins a multiple of 32 lags: every warp slot is one bin.
-      if (live) {
+      if (live && want) {
         unsigned mxs[16];
 #pragma unroll
         for (int q = 0; q < 16; q++) {
@@ -664,9 +688,10 @@ flat_kernel(const FlatArgs a) {
         }
       }
     } else if (small_keys) {
-      // Fast path: one redux per slot and warp; the winning lane parks z[k]
+      // One redux per slot and warp; the winning lane parks z[k]
       // at buf[k] (free after the last pass); 16 lanes then publish the warp's
       // 16 slot winners to the per-bin keys with parallel atomics.
+      if (want) {
       unsigned mxs[16];
 #pragma unroll
       for (int q = 0; q < 16; q++) {
@@ -697,7 +722,8 @@ flat_kernel(const FlatArgs a) {
           atomicMax(keys + bin, ((unsigned long long)(my & ~31u) << 32) | (unsigned)(~k));
         }
       }
-    } else {
+      }
+    } else if (want) {
       // Many bins (keys occupy buf): per-lane atomics, winners write back below.
 #pragma unroll
       for (int q = 0; q < 16; q++) {
