@@ -102,9 +102,11 @@ struct NConst {
   int grid_peaks = 0, grid_gate = 0, grid_fwd = 0;
   int cta = 0, smem = 0, g = 0;
   int grid_rows = 0;
-  // n = 4096: the two-pairs-per-thread kernel (flat2_kernel.cuh)
-  float4 *twid2 = nullptr;      // Flat2Geo::TW records (wr, wr, wi, wi)
-  int grid2 = 0;
+  // two pairs per thread (flat2_kernel.cuh at n = 4096, the transforms of
+  // large2_kernel.cuh at 128 ... 1024): the tables as (wr, wr, wi, wi) records
+  float4 *twid2 = nullptr;
+  float4 *twid2w = nullptr;     // flat2w_kernel: pass 2 in its thread order
+  int grid2 = 0, grid2w = 0;    // flat2_kernel, flat2w_kernel
 };
 static std::mutex g_const_mu;
 static std::map<std::pair<int, int>, NConst> g_const;
@@ -138,20 +140,37 @@ static int make_const(int device, NConst &c) {
                                                          Geo::SMEM));
   if (b1 < 1 || b2 < 1 || b3 < 1 || b4 < 1)
     return fail(MFB_ERR_CUDA, "kernel for n=%d cannot be resident on this device", N);
-  if constexpr (N == Flat2Geo::N) {
+  if constexpr (N == Flat2Geo::N || (N >= 128 && N <= 1024)) {
     // the scalar tables' values, duplicated for the two lanes
-    std::vector<float4> tw2(Flat2Geo::TW);
-    for (int i = 0; i < Flat2Geo::TW; i++) tw2[i] = make_float4(tw[i].x, tw[i].x, tw[i].y, tw[i].y);
+    std::vector<float4> tw2(tw.size());
+    for (size_t i = 0; i < tw.size(); i++) tw2[i] = make_float4(tw[i].x, tw[i].x, tw[i].y, tw[i].y);
     CUDA_TRY(cudaMalloc(&c.twid2, tw2.size() * sizeof(float4)));
     CUDA_TRY(cudaMemcpy(c.twid2, tw2.data(), tw2.size() * sizeof(float4), cudaMemcpyHostToDevice));
     CUDA_TRY(cudaFuncSetAttribute(flat2_kernel<MODE_PEAKS>,
+  }
+  if constexpr (N == Flat2Geo::N) {
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, Flat2Geo::SMEM));
     int b5 = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b5, flat2_kernel<MODE_PEAKS>,
                                                            Flat2Geo::T, Flat2Geo::SMEM));
-    if (b5 < 1) return fail(MFB_ERR_CUDA, "packed kernel for n=%d cannot be resident", N);
+    std::vector<float4> tww(Flat2wGeo::TW);
+    for (int i = 0; i < 240; i++) tww[i] = make_float4(tw[i].x, tw[i].x, tw[i].y, tw[i].y);
+    for (int q = 0; q < 15; q++)
+      for (int t = 0; t < 256; t++) {   // thread K1 + 16 K0 takes entry K0 + 16 K1
+        const float2 w = tw[240 + q * 256 + (t >> 4) + 16 * (t & 15)];
+        tww[240 + q * 256 + t] = make_float4(w.x, w.x, w.y, w.y);
+      }
+    CUDA_TRY(cudaMalloc(&c.twid2w, tww.size() * sizeof(float4)));
+    CUDA_TRY(cudaMemcpy(c.twid2w, tww.data(), tww.size() * sizeof(float4), cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaFuncSetAttribute(flat2w_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  Flat2wGeo::SMEM));
+    int b6 = 0;
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b6, flat2w_kernel, Flat2wGeo::T,
+                                                           Flat2wGeo::SMEM));
+    if (b5 < 1 || b6 < 1) return fail(MFB_ERR_CUDA, "packed kernel for n=%d cannot be resident", N);
     c.grid2 = b5 * sms;
   }
+    c.grid2w = b6 * sms;
   c.grid_rows = b4 * sms;
   c.grid_peaks = b1 * sms;
   c.grid_gate = b2 * sms;
@@ -200,12 +219,20 @@ static cudaError_t launch_flat(int n, const NConst &c, const FlatArgs &a, cudaSt
 // window with bins a multiple of 32 lags and at most KEYCAP bins, dense or
 // listed; it gives the same bits as flat_kernel / rows_kernel.
 static bool flat2_applies(int n, const NConst &c, const FlatArgs &a) {
-  return n == Flat2Geo::N && c.twid2 && a.ws == 0 && a.we == n && (a.binsize & 31) == 0 &&
-         a.nb <= KEYCAP;
+static bool flat2w_applies(int n, const FlatArgs &a) {
+  return n == Flat2wGeo::N && (a.ws & 255) == 0 && (a.we & 255) == 0 && (a.binsize & 255) == 0;
+}
+  return flat2w_applies(n, a) || (n == Flat2Geo::N && c.twid2 && a.ws == 0 && a.we == n &&
+                                  (a.binsize & 31) == 0 && a.nb <= KEYCAP);
 }
 
 static cudaError_t launch_flat2(const NConst &c, FlatArgs a, cudaStream_t s) {
   a.twid = reinterpret_cast<const float2 *>(c.twid2);
+  if (flat2w_applies(Flat2wGeo::N, a)) {
+    a.twid = reinterpret_cast<const float2 *>(c.twid2w);
+    flat2w_kernel<<<c.grid2w, Flat2wGeo::T, Flat2wGeo::SMEM, s>>>(a);
+    return cudaGetLastError();
+  }
   flat2_kernel<MODE_PEAKS><<<c.grid2, Flat2Geo::T, Flat2Geo::SMEM, s>>>(a);
   return cudaGetLastError();
 }
@@ -684,10 +711,7 @@ static int run_impl(mfb_plan *p, int d0, int nd, int t0, int nt, size_t binsize,
   if (is_large(p->n))
     return run_large(p, d0, nd, t0, nt, nullptr, 0, binsize, threshold, start, end, nb, idx, val,
                      counts, rs);
-  if (p->packed && flat2_applies((int)p->n, *p->c, a))
-    CUDA_TRY(launch_flat2(*p->c, a, p->stream));
-  else
-    CUDA_TRY(launch_flat<MODE_PEAKS>((int)p->n, *p->c, a, p->stream));
+  CUDA_TRY(launch_peaks(p, a));
   return MFB_OK;
 }
 
@@ -765,6 +789,12 @@ static int run_rows_impl(mfb_plan *p, int d0, int nd, int t0, int nt, const int3
   } else {
     CUDA_TRY(launch_rows((int)p->n, *p->c, a, p->stream));
   }
+// The dense block of `a` at n <= 16384.
+static cudaError_t launch_peaks(const mfb_plan *p, const FlatArgs &a) {
+  if (p->packed && flat2_applies((int)p->n, *p->c, a)) return launch_flat2(*p->c, a, p->stream);
+  return launch_flat<MODE_PEAKS>((int)p->n, *p->c, a, p->stream);
+}
+
   if (added) *added = trig_total != nullptr;
   return MFB_OK;
 }
@@ -885,7 +915,7 @@ extern "C" int mfb_run_series(mfb_plan *p, const void *series, size_t nseries,
     a.out_val = (float2 *)val + (size_t)b0 * nt * nb0;
     a.rs = 1;
     a.out_cnt = counts ? counts + (size_t)b0 * nt : nullptr;
-    CUDA_TRY(launch_flat<MODE_PEAKS>((int)p->n, *p->c, a, p->stream));
+    CUDA_TRY(launch_peaks(p, a));
     b0 += g;
   }
   return MFB_OK;

@@ -355,3 +355,55 @@ def test_packed_kernel_matches_one_pair_kernel_and_oracle(nd, nt, binsize, thres
     np.testing.assert_array_equal(got_v[rows], out[1][3].reshape(nd * nt, nb)[rows])
     untouched = np.setdiff1d(np.arange(nd * nt), rows)
     assert (got_i[untouched] == -7).all()
+
+
+@pytest.mark.parametrize("nd, nt, binsize, win", [
+    (1, 1, 4096, None),                 # one pair: the second lane is dead
+    (3, 5, 256, None),                  # odd pair count, data rows change inside an item
+    (2, 301, 256, (1024, 3072)),        # a window of whole blocks (block-wise series filtering)
+    (5, 7, 768, (256, 4096)),           # bins of three blocks
+    (1, 2, 2048, (0, 256)),             # one block
+])
+@pytest.mark.parametrize("thr", [0.0, 350.0, 1e6])
+def test_block_bins_kernel_is_bit_identical(nd, nt, binsize, win, thr):
+    """n = 4096 with bins and window in multiples of 256 lags (the kernel whose
+    second exchange stays within half-warps) against the one-pair kernel:
+    same bits; and against the FP64 oracle.  Thresholds: every bin reports,
+    some do (z has deviation 128 per component), none does."""
+    mf = _mf()
+    from apogee_b200 import _lib
+    rng = np.random.default_rng(nd * 1000 + nt)
+    D, H = noise(rng, (nd, 4096)), noise(rng, (nt, 4096))
+    f = mf.MatchedFilter(4096, nd, nt)
+    f.set_data(D)
+    f.set_templates(H)
+    out, cnt = f.run(binsize=binsize, threshold=thr, window=win, counts=True)
+    out, cnt = out.copy(), cnt.copy()
+    _lib.check(_lib.lib().mfb_set_packed(f._plan, 0))
+    ref, rcnt = f.run(binsize=binsize, threshold=thr, window=win, counts=True)
+    np.testing.assert_array_equal(out["index"], ref["index"])
+    np.testing.assert_array_equal(out["value"], ref["value"])
+    np.testing.assert_array_equal(cnt, rcnt)
+    z = oracle.correlate(D, H[:8])
+    assert not parity.compare(out["index"][:, :8], out["value"][:, :8], z, binsize, thr, win)
+
+
+@pytest.mark.parametrize("n", [64, 256, 1024, 2048, 8192, 16384])
+@pytest.mark.parametrize("win", [None, (3, -5)])
+def test_threshold_skips_only_pairs_without_candidates(n, win):
+    """Above a threshold a warp whose points are all below it skips the per-bin
+    reduction: one loud pair among quiet ones (in one warp with it where
+    several pairs share a warp), bins on and off the 32-lag grid, many bins."""
+    mf = _mf()
+    rng = np.random.default_rng(n)
+    D, H = noise(rng, (3, n)), noise(rng, (9, n))
+    D[1] += (2.0 * H[4] * np.exp(-2j * np.pi * np.arange(n) * (n // 3) / n)).astype(np.complex64)
+    w = None if win is None else (win[0], n + win[1])
+    f = mf.MatchedFilter(n, 3, 9)
+    f.set_data(D)
+    f.set_templates(H)
+    thr = float(n)
+    for binsize in (n // 8, n // 16 + 1, max(1, n // 128)):
+        out = check(f, D, H, binsize, thr, w)
+        assert (out["index"][1, 4] >= 0).any()
+        assert (out["index"] >= 0).any(-1).sum() < 27
