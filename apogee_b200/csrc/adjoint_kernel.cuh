@@ -21,8 +21,9 @@
 // min(n/16, 256) values of f0 for 256/F own rows.  Entries are staged in
 // rounds: a warp sorts one (own, other) row's entries by bucket, then the CTA
 // tabulates W^(l k) for the 32 lanes l and conj(g) W^((F x + 32 a) k) for its
-// groups a of 32 lanes, so the inner loop is two shared-memory reads (the
-// second a broadcast) and four FMAs per entry.  Rows without a peak are
+// groups a of 32 lanes (W^m = hi[m >> lo_bits] * lo[m & mask], FP64-built halves),
+// so the inner loop is two shared-memory reads (the second a broadcast) and
+// four FMAs per entry.  Rows without a peak are
 // skipped.  The lags are the forward pass's argmax lags; nothing of the
 // correlation series is stored.
 #pragma once
@@ -36,6 +37,7 @@ constexpr int ADJ_R = 16;              // frequencies per thread = buckets
 constexpr int ADJ_CHUNK = 32;          // entries of one (own, other) row sorted at a time
 constexpr int ADJ_TAB = 40960;         // bytes of staged twiddles per round
 constexpr int ADJ_ITEMS = 1024;        // (own, other, chunk) lists per round
+
 
 struct AdjArgs {
   const float2 *src;      // other rows [other][n]: templates (grad_D) or data (grad_H)
@@ -52,6 +54,9 @@ struct AdjArgs {
   int lists_per_round;    // lists of one row per round when chunks > 1, else 1
   int other_per_split;    // other rows per blockIdx.y
   int accumulate;         // 1: atomicAdd into a zeroed out (other split over blockIdx.y)
+  int lsh, ash;           // log2 of the lane and group values per entry
+  const float2 *tw_hi, *tw_lo;
+  int lo_bits, hi_count;
 };
 
 // Bytes of staged twiddles per entry: min(fblk, 32) lane values, one value
@@ -60,24 +65,21 @@ __host__ __device__ constexpr int adj_entry_bytes(int fblk) {
   return 8 * ((fblk < 32 ? fblk : 32) + (fblk + 31) / 32);
 }
 
-__device__ __forceinline__ cf adj_root(unsigned m, float two_over_n) {   // W^m, m < n: exact argument
-  cf w;
-  sincospif((float)m * two_over_n, &w.y, &w.x);
-  return w;
-}
-
 template <bool GRAD_DATA>
 __global__ void __launch_bounds__(ADJ_THREADS, 2) adjoint_kernel(const AdjArgs a) {
   extern __shared__ __align__(16) unsigned char adj_smem[];
-  const int L = a.fblk < 32 ? a.fblk : 32, A = (a.fblk + 31) >> 5;
+  const int L = 1 << a.lsh, A = 1 << a.ash;
   const int per_item = a.chunk;
   const int cap = ADJ_TAB / adj_entry_bytes(a.fblk);          // entries per round
   float2 *lane_tw = reinterpret_cast<float2 *>(adj_smem);      // [cap][L]
   float2 *group_tw = lane_tw + cap * L;                        // [cap][A]
   float2 *s_g = group_tw + cap * A;                            // [cap] conj(g), sorted
   int *s_k = reinterpret_cast<int *>(s_g + cap);               // [cap] lags, sorted
-  uint4 *s_end = reinterpret_cast<uint4 *>(                    // [items] bucket ends, one byte each
+  float2 *s_hi = reinterpret_cast<float2 *>(                   // twiddle halves
       (reinterpret_cast<uintptr_t>(s_k + cap) + 15) & ~uintptr_t(15));
+  float2 *s_lo = s_hi + a.hi_count;
+  uint4 *s_end = reinterpret_cast<uint4 *>(                    // [items] bucket ends, one byte each
+      (reinterpret_cast<uintptr_t>(s_lo + (1 << a.lo_bits)) + 15) & ~uintptr_t(15));
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int fb = blockIdx.x % a.fx, oc = blockIdx.x / a.fx;
@@ -89,8 +91,15 @@ __global__ void __launch_bounds__(ADJ_THREADS, 2) adjoint_kernel(const AdjArgs a
   const int ob = blockIdx.y * a.other_per_split;
   const int oe = min(a.other, ob + a.other_per_split);
   const unsigned mask_n = (unsigned)a.n - 1u;
-  const float two_over_n = 2.0f / (float)a.n;
+  const unsigned lo_mask = (1u << a.lo_bits) - 1u;
   const bool live = own_row < a.own;
+  for (int x = tid; x < a.hi_count; x += ADJ_THREADS) s_hi[x] = a.tw_hi[x];
+  for (int x = tid; x <= (int)lo_mask; x += ADJ_THREADS) s_lo[x] = a.tw_lo[x];
+  auto root = [&](unsigned m) {   // W^(m mod n)
+    m &= mask_n;
+    const float2 h = s_hi[m >> a.lo_bits], w = s_lo[m & lo_mask];
+    return cmul(cf{h.x, h.y}, cf{w.x, w.y});
+  };
 
   cf acc[ADJ_R];
 #pragma unroll
@@ -141,19 +150,18 @@ __global__ void __launch_bounds__(ADJ_THREADS, 2) adjoint_kernel(const AdjArgs a
       __syncthreads();
       // ---- twiddle tables of every staged entry ------------------------------------
       for (int x = tid; x < items * per_item * L; x += ADJ_THREADS) {
-        const int e = x / L, j = x & (L - 1);
+        const int e = x >> a.lsh, j = x & (L - 1);
         const int k = s_k[e];
         if (k < 0) continue;
-        const cf w = adj_root(((unsigned)j * (unsigned)k) & mask_n, two_over_n);
+        const cf w = root((unsigned)j * (unsigned)k);
         lane_tw[x] = make_float2(w.x, w.y);
       }
       for (int x = tid; x < items * per_item * A; x += ADJ_THREADS) {
-        const int e = x / A, j = x & (A - 1);
+        const int e = x >> a.ash, j = x & (A - 1);
         const int k = s_k[e];
         if (k < 0) continue;
         const float2 g = s_g[e];
-        const cf w = cmul(cf{g.x, g.y}, adj_root(((unsigned)(fb * a.fblk + 32 * j) * (unsigned)k) & mask_n,
-                                                 two_over_n));
+        const cf w = cmul(cf{g.x, g.y}, root((unsigned)(fb * a.fblk + 32 * j) * (unsigned)k));
         group_tw[x] = make_float2(w.x, w.y);
       }
       __syncthreads();
@@ -168,14 +176,14 @@ __global__ void __launch_bounds__(ADJ_THREADS, 2) adjoint_kernel(const AdjArgs a
           const int it = (ol * lc + cl) * a.slots + slot;
           const uint4 ends = s_end[it];
           const unsigned ew[4] = {ends.x, ends.y, ends.z, ends.w};
-          const float2 *p1 = lane_tw + (it * per_item) * L + l;
-          const float2 *p2 = group_tw + (it * per_item) * A + grp;
+          const float2 *p1 = lane_tw + ((it * per_item) << a.lsh) + l;
+          const float2 *p2 = group_tw + ((it * per_item) << a.ash) + grp;
           int e = 0;
 #pragma unroll
           for (int q = 0; q < ADJ_R; q++) {
             const int end = (int)((ew[q >> 2] >> (8 * (q & 3))) & 255u);
-            for (; e < end; e++) {
-              const float2 w = p1[e * L], h = p2[e * A];
+            for (; e < end; e++, p1 += L, p2 += A) {
+              const float2 w = *p1, h = *p2;
               S[q].x = fmaf(w.x, h.x, fmaf(-w.y, h.y, S[q].x));
               S[q].y = fmaf(w.x, h.y, fmaf(w.y, h.x, S[q].y));
             }

@@ -1845,7 +1845,7 @@ extern "C" int mfb_run_large_static(int device, size_t n, const void *data, int 
 }
 
 // ---------------------------------------------------------------- adjoint
-// W_n^m twiddles for the batched four-step: hi[m >> lo_bits] * lo[m & mask],
+// W_n^m twiddles for the adjoint and the batched four-step: hi[m >> lo_bits] * lo[m & mask],
 // built once per (device, n) from FP64 roots.
 struct AdjTables {
   float2 *hi = nullptr, *lo = nullptr;
@@ -1874,10 +1874,10 @@ static int get_adj_tables(int device, int n, AdjTables **out) {
 }
 
 // Dynamic shared memory of adjoint_kernel: the staged twiddles, the sorted
-// entries and the lists' bucket ends.
-static size_t adjoint_smem(int fblk, int items) {
+// entries, the twiddle halves and the lists' bucket ends.
+static size_t adjoint_smem(int fblk, int items, int roots) {
   const int cap = ADJ_TAB / adj_entry_bytes(fblk);
-  return (size_t)ADJ_TAB + (size_t)cap * 12 + 16 + (size_t)items * sizeof(uint4);
+  return (size_t)ADJ_TAB + (size_t)cap * 12 + 32 + (size_t)roots * 8 + (size_t)items * sizeof(uint4);
 }
 
 // One side of the adjoint: a CTA covers 256 (own row, f0) and all other rows;
@@ -1885,8 +1885,8 @@ static size_t adjoint_smem(int fblk, int items) {
 // split over blockIdx.y with atomic accumulation.
 constexpr int ADJ_FILL = 4;
 static int adjoint_side(bool grad_data, int n, int nd, int nt, int nb, const float2 *src,
-                        const int64_t *idx, const float2 *gz, float2 *out, int sms,
-                        cudaStream_t st) {
+                        const int64_t *idx, const float2 *gz, float2 *out, const AdjTables &tw,
+                        int sms, cudaStream_t st) {
   AdjArgs a;
   memset(&a, 0, sizeof a);
   a.src = src; a.idx = idx; a.gz = gz; a.out = out;
@@ -1911,11 +1911,11 @@ static int adjoint_side(bool grad_data, int n, int nd, int nt, int nb, const flo
   split = (a.other + a.other_per_split - 1) / a.other_per_split;
   a.accumulate = split > 1;
   if (a.accumulate) CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)a.own * n * sizeof(float2), st));
-  const size_t smem = adjoint_smem(a.fblk, lists * a.slots);
+  const size_t smem = adjoint_smem(a.fblk, lists * a.slots, tw.hi_count + (1 << tw.lo_bits));
   const dim3 grid((unsigned)tiles, (unsigned)split);
   // one limit for every shape, so that callers on several threads set the same value
   auto kernel = grad_data ? adjoint_kernel<true> : adjoint_kernel<false>;
-  CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 << 10));
+  CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 88 << 10));
   kernel<<<grid, ADJ_THREADS, smem, st>>>(a);
   CUDA_TRY(cudaGetLastError());
   return MFB_OK;
@@ -1931,17 +1931,20 @@ extern "C" int mfb_adjoint(int device, size_t n, const void *data, int nd, const
   CUDA_TRY(cudaGetDeviceCount(&ndev));
   if (device < 0 || device >= ndev) return fail(MFB_ERR_ARG, "no device %d", device);
   DeviceGuard dg(device);
-  int r = MFB_OK, sms = 0;
+  AdjTables *tw = nullptr;
+  int r = get_adj_tables(device, (int)n, &tw);
+  if (r) return r;
+  int sms = 0;
   CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   cudaStream_t st = (cudaStream_t)stream;
   if (grad_data) {
     r = adjoint_side(true, (int)n, nd, nt, (int)nb, (const float2 *)templates, idx,
-                     (const float2 *)gz, (float2 *)grad_data, sms, st);
+                     (const float2 *)gz, (float2 *)grad_data, *tw, sms, st);
     if (r) return r;
   }
   if (grad_tmpl) {
     r = adjoint_side(false, (int)n, nd, nt, (int)nb, (const float2 *)data, idx,
-                     (const float2 *)gz, (float2 *)grad_tmpl, sms, st);
+                     (const float2 *)gz, (float2 *)grad_tmpl, *tw, sms, st);
     if (r) return r;
   }
   return MFB_OK;
@@ -1992,6 +1995,9 @@ extern "C" int mfb_batch_create(mfb_batch **out, int device, const mfb_job *jobs
   CUDA_TRY(cudaGetDeviceCount(&ndev));
   if (device < 0 || device >= ndev) return fail(MFB_ERR_ARG, "no device %d", device);
   const size_t slot_bytes = (opts && opts->slot_bytes) ? opts->slot_bytes : ((size_t)64 << 20);
+  while ((1 << a.lsh) < a.fblk && a.lsh < 5) a.lsh++;
+  while ((32 << a.ash) < a.fblk) a.ash++;
+  a.tw_hi = tw.hi; a.tw_lo = tw.lo; a.lo_bits = tw.lo_bits; a.hi_count = tw.hi_count;
   const int nslots = (opts && opts->slots) ? opts->slots : 3;
   if (nslots < 2 || nslots > 64) return fail(MFB_ERR_ARG, "slots must be 2 .. 64");
   DeviceGuard dg(device);
