@@ -6,29 +6,33 @@
 // reference runs the flat filter at length m).  Here the m = 512 point DFT is
 // factored m = 16 x 32 (f = 32 f1 + f2, j = j1 + 16 j2):
 //
-//   stage 1  Y[j1, f2] = sum_f1 W16^(f1 j1) P[32 f1 + f2]          (GEMM)
-//   twiddle  Y'[j1, f2] = Y[j1, f2] W512^(f2 j1)                      (CUDA cores)
-//   stage 2  Z[j1 + 16 j2] = sum_f2 W32^(f2 j2) Y'[j1, f2]           (GEMM)
+//   stage 1  Y[j1, f2] = sum_f1 W16^(f1 j1) P[32 f1 + f2]      (CUDA cores, FP32)
+//   twiddle  Y'[j1, f2] = Y[j1, f2] W512^(f2 j1)
+//   stage 2  Z[j1 + 16 j2] = sum_f2 W32^(f2 j2) Y'[j1, f2]       (GEMM)
 //
-// Both stages are real GEMMs on the 5th-generation tensor cores: complex
-// values are realified (re, im interleaved along K), and every operand is
-// split into hi + lo halves of BF16 (or FP16) with the products
-// hi*hi + hi*lo + lo*hi accumulated in FP32 in tensor memory, which keeps
-// about 16 significant bits (BF16) of the FP32 inputs.  Pairs are batched
-// along M: stage 1 rows are (pair, f2) -- 4 pairs per 128-row tile -- and
-// stage 2 rows are (pair, j1) -- 8 pairs per tile.
+// Stage 1 stays in registers: lane f2 of a warp holds the 16 products
+// P[32 f1 + f2] of a pair, and the 16-point transform costs it about ten FP32
+// operations a point, five in packed FP32x2 form with two pairs per thread --
+// less than staging it as a tensor-core operand (a hi/lo split, a store, and
+// the accumulator read back), and with FP32 rounding.  Stage 2 is a real GEMM on
+// the 5th-generation tensor cores: complex values are realified (re, im
+// interleaved along K), and both operands are split into hi + lo halves of BF16
+// (or FP16) with the products hi*hi + hi*lo + lo*hi accumulated in FP32 in tensor
+// memory, which keeps about 16 significant bits (BF16) of the FP32 inputs.  Rows
+// are (pair, j1): 8 pairs per 128-row tile.
 //
-// Per item (8 pairs): the conjugate product and its split are written by the
-// CUDA cores as the stage-1 A operand (K-major, no swizzle); one thread
-// issues 12 MMAs (M128 N32 K16) into TMEM; the accumulators come back with
-// tcgen05.ld, are twiddled, split and written transposed as the stage-2 A
-// operand (K-major, 128-byte swizzle, so a warp's 32 stores to one row hit 32
-// different banks); 12 more MMAs (M128 N64 K16); then |z|^2 over the window,
-// max over the pair's 16 rows, and the gate of src/hmf.c:264-300.  The three
-// steps run in separate warp roles on consecutive items (see
-// coarse_tc_ws_kernel).  The DFT matrices (B operands) and the 512-point
-// twiddles are built once on the host in FP64 and copied into shared memory
-// at kernel start.
+// Per item (8 pairs): four warps of two pairs each form the conjugate products,
+// stage 1, the twiddle and the split, and store the stage-2 A operand (K-major,
+// 128-byte swizzle; a warp stores one row per instruction, 32 different banks);
+// one thread issues 12 MMAs (M128 N64 K16); the same warps then read the previous
+// item's |z|^2 over the window from tensor memory, its maximum over the pair's 16
+// rows, and apply the gate of src/hmf.c:264-300 (see coarse_tc_ws_kernel).  The
+// DFT matrix (B operand) and the 512-point twiddles are built once on the host in
+// FP64 and copied into shared memory at kernel start.
+//
+// Measured on a B200, 16 x 1024 pairs, BF16: 33.5 -> 26.8 us against both stages as
+// GEMMs in three roles; 14.3 -> 11.2 M warp instructions.  FP32 work and the split, at
+// 16 warps per SM, bound it (issue ~46%, tensor pipe ~10%).
 //
 // Every wait on an mbarrier is bounded; on timeout the kernel records an
 // error flag, stops issuing work, releases its tensor memory and returns.
@@ -40,17 +44,17 @@
 #include <cstring>
 #include <vector>
 #include "hier_kernels.cuh"
+#include "packed_passes.cuh"
 
 namespace mfb {
 
 namespace tc {
 constexpr int BAND = 512;
-constexpr int PAIRS = 8;          // pairs per item; producer warp w works on pair w
+constexpr int PAIRS = 8;          // pairs per item; warp w of a team works on pairs 2w, 2w + 1
 // constant operands at the start of shared memory (1024-byte aligned base)
 constexpr int OFF_B2 = 0;         // 2 splits x 8 KB, 128B swizzle (64 rows x 128 B)
-constexpr int OFF_B1 = 16384;     // 2 splits x 2 k-steps x 1 KB, no swizzle
-constexpr int OFF_TW = 20480;     // 512 float2 twiddles W512^(f2 j1), [j1][f2]
-constexpr int CONST_BYTES = 24576;
+constexpr int OFF_TW = 16384;     // 512 float2 twiddles W512^(f2 j1), [j1][f2]
+constexpr int CONST_BYTES = 20480;
 constexpr unsigned SPIN_LIMIT = 1u << 22;
 
 __host__ __device__ constexpr uint32_t idesc(int n, int fp16) {
@@ -113,14 +117,6 @@ __device__ __forceinline__ void tc_after_sync() {
                  "=r"(r[30]), "=r"(r[31])                                                          \
                : "r"(taddr))
 
-#define MFB_TMEM_LD16(taddr, r)                                                                    \
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "                                            \
-               "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"                     \
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),          \
-                 "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),        \
-                 "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])                                \
-               : "r"(taddr))
-
 __device__ __forceinline__ void tmem_wait_ld() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -152,7 +148,7 @@ struct TcKernelArgs {
   const float2 *data;        // full-length rows, stride n; first BAND bins used
   long long data_stride;
   const float2 *ct;          // coarse templates [nt][BAND]
-  const uint4 *consts;       // CONST_BYTES image: B2 | B1 | twiddles
+  const uint4 *consts;       // CONST_BYTES image: B2 | twiddles
   int d0, nd, t0, nt;
   int ws, we;
   float t2, gate;
@@ -170,43 +166,35 @@ struct TcKernelArgs {
   int rows_n2, cs, ce;
 };
 
-// Warp-specialised form of the same pass: three roles in one 512-thread CTA
-// (one per SM) work on consecutive items at once, handing operands over
-// through NSLOT shared-memory and tensor-memory slots per stage:
-//   warps 0-7   producers: warp w owns pair w of the item (lane = f2); the
-//               conjugate product and split -> stage-1 A (slot k), inputs for
-//               the next item already in flight; thread 0 issues the stage-1
-//               MMAs into TMEM S1[k];
-//   warps 8-11  stage-1 epilogue: quadrant q reads pairs q and 4 + q from
-//               S1[k] -> twiddle, split, transposed store -> stage-2 A
-//               (slot k); thread 256 issues the stage-2 MMAs into S2[k];
-//   warps 12-15 stage-2 epilogue: S2[k] -> |z|^2 over the window, max per
-//               pair with warp shuffles, gate.
-// Hand-offs are mbarriers: full_s1[k] / full_s2[k] (MMA commits) and
-// free_s1[k] / free_s2[k] (the epilogue warps have read the accumulators).
-// A slot is reused every NSLOT items, so each wait is on the phase of the
-// item NSLOT back and no role can run two phases ahead of a waiter.  Waits
-// are bounded; a failed wait sets the error flag, every later wait returns
-// at once and the roles run out their loops without issuing MMAs (no thread
-// leaves a loop early, so the role barriers always fill).
+// One 512-thread CTA per SM: four teams of four warps, team T on items T, T + 4,
+// ... of the CTA, warp w of a team on pairs 2w and 2w + 1 (lane = f2).  A team's
+// step: products, 16-point transforms and twiddles in packed FP32x2; the split ->
+// the team's stage-2 operand (free once the previous item's MMAs have
+// committed); a team barrier; its first thread issues the item's MMAs into one
+// of the team's two accumulators; the next item's loads; and the previous item's
+// accumulators -> |z|^2 over the window, maximum per pair with warp shuffles,
+// gate.  Every warp does the same work, so no role waits for another: as
+// producer and epilogue roles (12 + 4 warps) the epilogue warps took ~1850 cycles
+// an item and bounded the pass, and hand-offs by mbarrier with a separate
+// issuing thread were slower still.  The MMAs of an item run while the team reads the previous
+// one's accumulators and forms the next one's products.  Waits are bounded; a
+// failed wait sets the error flag, every later wait returns at once and the teams
+// run out their loops without issuing MMAs (no thread leaves a loop early, so the
+// team barriers always fill).
 namespace tcw {
-constexpr int NSLOT = 2;
-constexpr int THREADS = 512;
-constexpr int TMEM_COLS = 256;                      // S1[2] x 64 + S2[2] x 64
-constexpr int S2_COL = NSLOT * 64;
-constexpr int SLOT = 32768;
-constexpr int OFF_A2 = 24576;                       // NSLOT x 32 KB (2 splits x 16 KB, 128B swizzle)
-constexpr int OFF_A1 = OFF_A2 + NSLOT * SLOT;       // NSLOT x 32 KB (2 tiles x 2 splits x 2 k-steps x 4 KB)
-constexpr int OFF_BAR = OFF_A1 + NSLOT * SLOT;      // 4 NSLOT mbarriers, TMEM slot, abort flag
+constexpr int TEAMS = 4;
+constexpr int THREADS = TEAMS * 128;
+constexpr int NACC = 2 * TEAMS;                     // accumulators, 64 columns each
+constexpr int TMEM_COLS = NACC * 64;
+constexpr int SLOT = 32768;                         // 2 splits x 16 KB, 128B swizzle
+constexpr int OFF_A2 = 20480;
+constexpr int OFF_BAR = OFF_A2 + TEAMS * SLOT;      // NACC mbarriers (MMA commits), TMEM slot, abort flag
 constexpr int SMEM_BYTES = OFF_BAR + 128 + 1024;
-constexpr int B_FULL1 = 0, B_FULL2 = NSLOT, B_FREE1 = 2 * NSLOT, B_FREE2 = 3 * NSLOT;
+static_assert(OFF_A2 % 1024 == 0 && OFF_A2 >= tc::CONST_BYTES, "swizzled slots are 1024-byte aligned");
 }  // namespace tcw
 
 __device__ __forceinline__ void role_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" :: "r"(id), "r"(nthreads) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(bar) : "memory");
 }
 // Bounded wait that gives up at once when another thread has given up.
 __device__ __forceinline__ bool mbar_wait_ab(uint32_t bar, uint32_t phase, volatile int *abort_flag,
@@ -223,25 +211,24 @@ __device__ __forceinline__ bool mbar_wait_ab(uint32_t bar, uint32_t phase, volat
   return false;
 }
 
-template <int FP16>
+template <int FP16, bool ROWS>
 __global__ void __launch_bounds__(tcw::THREADS, 1)
 coarse_tc_ws_kernel(const TcKernelArgs a) {
   using namespace tc;
-  using tcw::NSLOT;
+  using tcw::NACC;
+  using tcw::TEAMS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *sm = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t sbase = smem_u32(sm);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   uint64_t *bars = reinterpret_cast<uint64_t *>(sm + tcw::OFF_BAR);
-  uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + tcw::OFF_BAR + 8 * 4 * NSLOT);
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(sm + tcw::OFF_BAR + 8 * 4 * NSLOT + 8);
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + tcw::OFF_BAR + 8 * NACC);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(sm + tcw::OFF_BAR + 8 * NACC + 8);
   for (int i = tid; i < CONST_BYTES / 16; i += tcw::THREADS)
     reinterpret_cast<uint4 *>(sm)[i] = a.consts[i];
   if (tid == 0) {
-    for (int i = 0; i < 4 * NSLOT; i++) {   // commits: 1 arrival; epilogue reads: 1 per warp (4)
-      const int cnt = i < tcw::B_FREE1 ? 1 : 4;
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&bars[i])), "r"(cnt));
-    }
+    for (int i = 0; i < NACC; i++)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&bars[i])));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     *abort_flag = 0;
   }
@@ -255,215 +242,194 @@ coarse_tc_ws_kernel(const TcKernelArgs a) {
   __syncthreads();
   tc_after_sync();
   const uint32_t tmem = *tslot;
-  const float2 *tw512 = reinterpret_cast<const float2 *>(sm + OFF_TW);
-  const uint32_t id1 = idesc(32, FP16), id2 = idesc(64, FP16);
+  const uint32_t id2 = idesc(64, FP16);
   const long long total = (long long)a.nd * a.nt;
   const long long items = (total + PAIRS - 1) / PAIRS;
   const long long per = items / gridDim.x, extra = items % gridDim.x;
   const long long ibeg = blockIdx.x * per + (blockIdx.x < extra ? blockIdx.x : extra);
   const int nit = (int)(per + (blockIdx.x < extra ? 1 : 0));
-  auto bar = [&](int i) { return smem_u32(&bars[i]); };
+  const int team = warp >> 2, w = warp & 3, f2 = lane;
+  auto full = [&](int u) { return smem_u32(&bars[team * 2 + (u & 1)]); };   // commit of the team's item u
 
-  if (warp < 8) {
-    // ---- producers: warp w owns pair w of the item, lane = f2 ----------------
-    const int prow = 32 * (warp & 3) + lane, ptile = warp >> 2;
-    float2 pd[16], ph[16];
-    auto issue_loads = [&](int it) {
-      const long long pi = (ibeg + it) * PAIRS + warp;
-      if (it < nit && pi < total && a.rows_n2 > 0) {
-        // rows mode: the product is already formed (times conj(1) below, exact)
-        const float2 *dp = a.data + pi * (long long)a.data_stride;
+  const float2 *tw512 = reinterpret_cast<const float2 *>(sm + OFF_TW) + f2;
+  uint8_t *a2 = sm + tcw::OFF_A2 + team * tcw::SLOT;
+  const uint32_t a2s = sbase + tcw::OFF_A2 + team * tcw::SLOT;
+  // Inputs of the team's next item: the data row of pair A (pair B's, where it
+  // differs, is loaded at its use) and both templates; in rows mode pa, pb are the
+  // products.  Pairs past the end repeat the last one; their results are dropped.
+  float2 pd[16], pa[16], pb[16];
+  bool same_d = true;
+  auto pair0 = [&](int it) { return min((ibeg + min(it, nit - 1)) * PAIRS + 2 * w, total - 1); };
+  auto load_a = [&](int it) {
+    const long long p0 = pair0(it);
+    if constexpr (ROWS) {
+      const float2 *ra = a.data + p0 * (long long)a.data_stride + f2;
 #pragma unroll
-        for (int f1 = 0; f1 < 16; f1++) { pd[f1] = __ldg(dp + 32 * f1 + lane); ph[f1] = make_float2(1.f, 0.f); }
-      } else if (it < nit && pi < total) {
-        const int d = (int)(pi / a.nt), t = (int)(pi - (long long)d * a.nt);
-        const float2 *dp = a.data + (long long)(a.d0 + d) * a.data_stride;
-        const float2 *hp = a.ct + (long long)(a.t0 + t) * BAND;
+      for (int f1 = 0; f1 < 16; f1++) pa[f1] = __ldg(ra + 32 * f1);
+    } else {
+      const int d = (int)((unsigned)p0 / (unsigned)a.nt), t = (int)(p0 - (long long)d * a.nt);
+      const float2 *dp = a.data + (long long)(a.d0 + d) * a.data_stride + f2;
+      const float2 *hp = a.ct + (long long)(a.t0 + t) * BAND + f2;
 #pragma unroll
-        for (int f1 = 0; f1 < 16; f1++) { pd[f1] = __ldg(dp + 32 * f1 + lane); ph[f1] = __ldg(hp + 32 * f1 + lane); }
+      for (int f1 = 0; f1 < 16; f1++) { pd[f1] = __ldg(dp + 32 * f1); pa[f1] = __ldg(hp + 32 * f1); }
+    }
+  };
+  auto load_b = [&](int it) {
+    const long long p0 = pair0(it), p1 = min(p0 + 1, total - 1);
+    if constexpr (ROWS) {
+      const float2 *rb = a.data + p1 * (long long)a.data_stride + f2;
+#pragma unroll
+      for (int f1 = 0; f1 < 16; f1++) pb[f1] = __ldg(rb + 32 * f1);
+    } else {
+      const int t = (int)((unsigned)p0 % (unsigned)a.nt);
+      same_d = p1 == p0 || t + 1 < a.nt;       // else pair B is template 0 of the next row
+      const int v = !same_d ? 0 : p1 > p0 ? t + 1 : t;
+      const float2 *hq = a.ct + (long long)(a.t0 + v) * BAND + f2;
+#pragma unroll
+      for (int f1 = 0; f1 < 16; f1++) pb[f1] = __ldg(hq + 32 * f1);
+    }
+  };
+
+  // Rows R = 32 w + lane of an item's accumulators = (pair R / 16, j1 = R % 16);
+  // lags j1 + 16 J of the window: J in [J0, J1).
+  const int R = 32 * w + lane, j1 = R & 15;
+  auto first_J = [&](int edge) { return edge > j1 ? min(32, (edge - j1 + 15) >> 4) : 0; };
+  int J0 = first_J(a.ws), J1 = first_J(a.we);
+  auto epilogue = [&](int it, int u) {
+    const long long pi = (ibeg + it) * PAIRS + (R >> 4);
+    if constexpr (ROWS) {
+      // lags rows_n2 * j + k2 of the longer band inside [cs, ce)
+      const int k2 = (int)(pi % a.rows_n2);
+      J0 = first_J(a.cs > k2 ? (a.cs - k2 + a.rows_n2 - 1) / a.rows_n2 : 0);
+      J1 = first_J(a.ce > k2 ? (a.ce - k2 + a.rows_n2 - 1) / a.rows_n2 : 0);
+    }
+    const bool whole = __all_sync(0xffffffffu, J0 == 0 && J1 == 32);
+    const uint32_t acc = tmem + ((uint32_t)(32 * w) << 16) + (team * 2 + (u & 1)) * 64;
+    tc_after_sync();
+    float best = 0.f;
+#pragma unroll
+    for (int half = 0; half < 2; half++) {
+      uint32_t v[32];
+      MFB_TMEM_LD32(acc + 32 * half, v);
+      tmem_wait_ld();
+      float m[2] = {0.f, 0.f};
+      auto m2 = [&](int jj) {
+        const float zr = __uint_as_float(v[2 * jj]), zi = __uint_as_float(v[2 * jj + 1]);
+        return fmaf(zr, zr, zi * zi);
+      };
+      if (whole) {
+#pragma unroll
+        for (int jj = 0; jj < 16; jj++) m[jj & 1] = fmaxf(m[jj & 1], m2(jj));
       } else {
 #pragma unroll
-        for (int f1 = 0; f1 < 16; f1++) { pd[f1] = make_float2(0.f, 0.f); ph[f1] = make_float2(0.f, 0.f); }
+        for (int jj = 0; jj < 16; jj++)
+          if (16 * half + jj >= J0 && 16 * half + jj < J1) m[jj & 1] = fmaxf(m[jj & 1], m2(jj));
       }
-    };
-    int last = -1;
-    issue_loads(0);
-    for (int it = 0; it < nit; it++) {
-      const int k = it % NSLOT;
-      const uint32_t u = (uint32_t)(it / NSLOT);
-      if (it >= NSLOT) mbar_wait_ab(bar(tcw::B_FULL1 + k), (u - 1) & 1, abort_flag, a.err);  // A1[k] consumed
-      uint8_t *a1 = sm + tcw::OFF_A1 + k * tcw::SLOT;
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        uint32_t hh[4], ll[4];
-#pragma unroll
-        for (int v = 0; v < 4; v++) {
-          const float2 x = pd[4 * q + v], h = ph[4 * q + v];
-          split2<FP16>(fmaf(x.x, h.x, x.y * h.y), fmaf(x.y, h.x, -x.x * h.y), hh[v], ll[v]);
-        }
-        const int ks = q >> 1, cc = q & 1;
-        const int off = (prow >> 3) * 256 + cc * 128 + (prow & 7) * 16;
-        *reinterpret_cast<uint4 *>(a1 + ((ptile * 2 + 0) * 2 + ks) * 4096 + off) = make_uint4(hh[0], hh[1], hh[2], hh[3]);
-        *reinterpret_cast<uint4 *>(a1 + ((ptile * 2 + 1) * 2 + ks) * 4096 + off) = make_uint4(ll[0], ll[1], ll[2], ll[3]);
-      }
-      issue_loads(it + 1);
-      fence_async_smem();
-      tc_before_sync();
-      role_sync(1, 256);
-      if (tid == 0) {
-        bool ok = !*abort_flag;
-        if (ok && it >= NSLOT)
-          ok = mbar_wait_ab(bar(tcw::B_FREE1 + k), (u - 1) & 1, abort_flag, a.err);   // S1[k] read
-        if (ok) {
-          tc_after_sync();
-          const uint32_t a1s = sbase + tcw::OFF_A1 + k * tcw::SLOT;
-#pragma unroll
-          for (int s = 0; s < 2; s++) {
-            int first = 1;
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-              const int ha = (c == 2) ? 1 : 0, hb = (c == 1) ? 1 : 0;
-#pragma unroll
-              for (int ks = 0; ks < 2; ks++) {
-                const uint64_t ad = sdesc(a1s + ((s * 2 + ha) * 2 + ks) * 4096, 128, 256, 0);
-                const uint64_t bd = sdesc(sbase + OFF_B1 + (hb * 2 + ks) * 1024, 128, 256, 0);
-                mma(tmem + k * 64 + s * 32, ad, bd, id1, first ? 0u : 1u);
-                first = 0;
-              }
-            }
-          }
-          commit(bar(tcw::B_FULL1 + k));
-          last = it;
-        }
-      }
+      best = fmaxf(best, fmaxf(m[0], m[1]));
     }
-    if (tid == 0 && last >= 0)   // own MMAs complete before the accumulators are freed
-      mbar_wait(bar(tcw::B_FULL1 + last % NSLOT), (uint32_t)(last / NSLOT) & 1);
-  } else if (warp < 12) {
-    // ---- stage-1 epilogue: quadrant q, pairs q (tile 0) and 4 + q (tile 1), f2 = lane
-    const int q = warp & 3, f2 = lane;
-    float2 tw[16];                 // W512^(f2 j1), j1 = 0..15: the same for every item
 #pragma unroll
-    for (int j1 = 0; j1 < 16; j1++) tw[j1] = tw512[j1 * 32 + f2];
-    int last = -1;
-    for (int it = 0; it < nit; it++) {
-      const int k = it % NSLOT;
-      const uint32_t u = (uint32_t)(it / NSLOT);
-      mbar_wait_ab(bar(tcw::B_FULL1 + k), u & 1, abort_flag, a.err);                       // S1[k] full
-      tc_after_sync();
-      uint32_t vv[16];
-      if (it >= NSLOT) mbar_wait_ab(bar(tcw::B_FULL2 + k), (u - 1) & 1, abort_flag, a.err);  // A2[k] consumed
-      uint8_t *a2 = sm + tcw::OFF_A2 + k * tcw::SLOT;
-#pragma unroll
-      for (int hh = 0; hh < 4; hh++) {
-        // 16 accumulator columns (8 values j1 of one tile) at a time: few
-        // registers live, so the compiler can overlap the elements' chains
-        const int s = hh >> 1, p = 4 * s + q;
-        MFB_TMEM_LD16(tmem + ((uint32_t)(32 * q) << 16) + k * 64 + 16 * hh, vv);
-        tmem_wait_ld();
-        if (hh == 3) {   // both tiles read: S1[k] is free
-          tc_before_sync();
-          if (lane == 0) mbar_arrive(bar(tcw::B_FREE1 + k));
-        }
-#pragma unroll
-        for (int jj = 0; jj < 8; jj++) {
-          const int j1 = 8 * (hh & 1) + jj;
-          const float yr = __uint_as_float(vv[2 * jj]), yi = __uint_as_float(vv[2 * jj + 1]);
-          const float2 w = tw[j1];
-          const float zr = fmaf(yr, w.x, -yi * w.y), zi = fmaf(yr, w.y, yi * w.x);
-          uint32_t hi, lo;
-          split2<FP16>(zr, zi, hi, lo);
-          const int R = p * 16 + j1;
-          const int off = (R >> 3) * 1024 + (R & 7) * 128 + (((f2 >> 2) ^ (R & 7)) << 4) + (f2 & 3) * 4;
-          *reinterpret_cast<uint32_t *>(a2 + off) = hi;
-          *reinterpret_cast<uint32_t *>(a2 + 16384 + off) = lo;
-        }
-      }
-      fence_async_smem();
-      tc_before_sync();
-      role_sync(2, 128);
-      if (tid == 256) {
-        bool ok = !*abort_flag;
-        if (ok && it >= NSLOT)
-          ok = mbar_wait_ab(bar(tcw::B_FREE2 + k), (u - 1) & 1, abort_flag, a.err);   // S2[k] read
-        if (ok) {
-          tc_after_sync();
-          const uint32_t a2s = sbase + tcw::OFF_A2 + k * tcw::SLOT;
-          int first = 1;
-#pragma unroll
-          for (int c = 0; c < 3; c++) {
-            const int ha = (c == 2) ? 1 : 0, hb = (c == 1) ? 1 : 0;
-#pragma unroll
-            for (int ks = 0; ks < 4; ks++) {
-              const uint64_t ad = sdesc(a2s + ha * 16384 + ks * 32, 16, 1024, 2);
-              const uint64_t bd = sdesc(sbase + OFF_B2 + hb * 8192 + ks * 32, 16, 1024, 2);
-              mma(tmem + tcw::S2_COL + k * 64, ad, bd, id2, first ? 0u : 1u);
-              first = 0;
-            }
-          }
-          commit(bar(tcw::B_FULL2 + k));
-          last = it;
-        }
-      }
-    }
-    if (tid == 256 && last >= 0)
-      mbar_wait(bar(tcw::B_FULL2 + last % NSLOT), (uint32_t)(last / NSLOT) & 1);
-  } else {
-    // ---- stage-2 epilogue: quadrant q, rows R = 32 q + lane = (pair R / 16, j1 = R % 16)
-    const int q = warp & 3, R = 32 * q + lane, j1 = R & 15;
-    for (int it = 0; it < nit; it++) {
-      const int k = it % NSLOT;
-      const uint32_t u = (uint32_t)(it / NSLOT);
-      mbar_wait_ab(bar(tcw::B_FULL2 + k), u & 1, abort_flag, a.err);                       // S2[k] full
-      tc_after_sync();
-      int ws = a.ws, we = a.we;
-      if (a.rows_n2 > 0) {
-        // lags rows_n2 * j + k2 of the longer band inside [cs, ce)
-        const long long pi = (ibeg + it) * PAIRS + (R >> 4);
-        const int k2 = (int)(pi % a.rows_n2);
-        ws = a.cs > k2 ? (a.cs - k2 + a.rows_n2 - 1) / a.rows_n2 : 0;
-        we = a.ce > k2 ? (a.ce - k2 + a.rows_n2 - 1) / a.rows_n2 : 0;
-      }
-      float best = 0.f;
-#pragma unroll
-      for (int half = 0; half < 2; half++) {
-        uint32_t v[32];
-        MFB_TMEM_LD32(tmem + ((uint32_t)(32 * q) << 16) + tcw::S2_COL + k * 64 + 32 * half, v);
-        tmem_wait_ld();
-#pragma unroll
-        for (int jj = 0; jj < 16; jj++) {
-          const float zr = __uint_as_float(v[2 * jj]), zi = __uint_as_float(v[2 * jj + 1]);
-          const int j = j1 + 16 * (16 * half + jj);
-          const float m2 = fmaf(zr, zr, zi * zi);
-          if (j >= ws && j < we && m2 > best) best = m2;
-        }
-      }
-      tc_before_sync();
-      if (lane == 0) mbar_arrive(bar(tcw::B_FREE2 + k));
-#pragma unroll
-      for (int o = 8; o; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
-      const int pr = R >> 4;
-      const long long pi = (ibeg + it) * PAIRS + pr;
-      if (pi < total && !*abort_flag) {
-        const int row = (int)pi;
-        if (a.rows_n2 > 0) {
-          if ((lane & 15) == 0) a.coarse_out[pi] = best;
-        } else if (a.coarse_out) {
-          if ((lane & 15) == 0) a.coarse_out[row] = sqrtf(best);
+    for (int o = 8; o; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
+    if (pi < total && !*abort_flag) {
+      const int row = (int)pi;
+      if constexpr (ROWS) {
+        if ((lane & 15) == 0) a.coarse_out[pi] = best;
+      } else if (a.coarse_out) {
+        if ((lane & 15) == 0) a.coarse_out[row] = sqrtf(best);
+      } else {
+        const bool fire = best > a.t2 && sqrtf(best) >= a.gate;
+        if (fire) {
+          if ((lane & 15) == 0) a.fire_list[atomicAdd(a.fire_count, 1)] = row;
         } else {
-          const bool fire = best > a.t2 && sqrtf(best) >= a.gate;
-          if (fire) {
-            if ((lane & 15) == 0) a.fire_list[atomicAdd(a.fire_count, 1)] = row;
-          } else {
-            const long long obase = (long long)row * a.full_nb;
-            for (int b = lane & 15; b < a.full_nb; b += 16) {
-              a.out_idx[(obase + b) * a.rs] = -1;
-              a.out_val[(obase + b) * a.rs] = make_float2(0.f, 0.f);
-            }
+          const long long obase = (long long)row * a.full_nb;
+          for (int b = lane & 15; b < a.full_nb; b += 16) {
+            a.out_idx[(obase + b) * a.rs] = -1;
+            a.out_val[(obase + b) * a.rs] = make_float2(0.f, 0.f);
           }
         }
       }
     }
+  };
+
+  int last = -1;               // the team's last item with MMAs issued (first thread)
+  int u = 0;                   // the team's items so far
+  if (team < nit) { load_a(team); load_b(team); }
+  for (int it = team; it < nit; it += TEAMS, u++) {
+    float2 X[16], Y[16];
+    if constexpr (ROWS) {
+#pragma unroll
+      for (int f1 = 0; f1 < 16; f1++) {
+        X[f1] = make_float2(pa[f1].x, pb[f1].x);
+        Y[f1] = make_float2(pa[f1].y, pb[f1].y);
+      }
+    } else {
+#pragma unroll
+      for (int f1 = 0; f1 < 16; f1++) {
+        const float2 d = pd[f1], h = pa[f1], g = pb[f1];
+        X[f1].x = fmaf(d.x, h.x, d.y * h.y);
+        Y[f1].x = fmaf(d.y, h.x, -d.x * h.y);
+        X[f1].y = fmaf(d.x, g.x, d.y * g.y);
+        Y[f1].y = fmaf(d.y, g.x, -d.x * g.y);
+      }
+      if (!same_d) {   // pair B opens the next data row
+        const unsigned p1 = (unsigned)((ibeg + it) * PAIRS + 2 * w + 1);
+        const float2 *dp = a.data + (long long)(a.d0 + (int)(p1 / (unsigned)a.nt)) * a.data_stride + f2;
+        const float2 *hp = a.ct + (long long)a.t0 * BAND + f2;
+#pragma unroll
+        for (int f1 = 0; f1 < 16; f1++) {
+          const float2 d = __ldg(dp + 32 * f1), g = __ldg(hp + 32 * f1);
+          X[f1].y = fmaf(d.x, g.x, d.y * g.y);
+          Y[f1].y = fmaf(d.y, g.x, -d.x * g.y);
+        }
+      }
+    }
+    p2::dft16(X, Y);
+#pragma unroll
+    for (int j = 1; j < 16; j++) {
+      const float2 tw = tw512[j * 32];
+      p2::twiddle(X[j], Y[j], make_float4(tw.x, tw.x, tw.y, tw.y));
+    }
+    if (u >= 1) mbar_wait_ab(full(u - 1), ((u - 1) >> 1) & 1, abort_flag, a.err);   // operand consumed
+#pragma unroll
+    for (int p = 0; p < 2; p++)
+#pragma unroll
+      for (int j = 0; j < 16; j++) {
+        uint32_t hi, lo;
+        split2<FP16>(p ? X[j].y : X[j].x, p ? Y[j].y : Y[j].x, hi, lo);
+        const int r = (2 * w + p) * 16 + j;
+        const int off = (r >> 3) * 1024 + (r & 7) * 128 + (((f2 >> 2) ^ (r & 7)) << 4) + (f2 & 3) * 4;
+        *reinterpret_cast<uint32_t *>(a2 + off) = hi;
+        *reinterpret_cast<uint32_t *>(a2 + 16384 + off) = lo;
+      }
+    fence_async_smem();
+    tc_before_sync();
+    role_sync(1 + team, 128);
+    if ((tid & 127) == 0 && !*abort_flag) {
+      tc_after_sync();
+      int first = 1;
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const int ha = (c == 2) ? 1 : 0, hb = (c == 1) ? 1 : 0;
+#pragma unroll
+        for (int ks = 0; ks < 4; ks++) {
+          const uint64_t ad = sdesc(a2s + ha * 16384 + ks * 32, 16, 1024, 2);
+          const uint64_t bd = sdesc(sbase + OFF_B2 + hb * 8192 + ks * 32, 16, 1024, 2);
+          mma(tmem + (team * 2 + (u & 1)) * 64, ad, bd, id2, first ? 0u : 1u);
+          first = 0;
+        }
+      }
+      commit(full(u));
+      last = u;
+    }
+    __syncwarp();
+    load_a(it + TEAMS);
+    if (u >= 1) epilogue(it - TEAMS, u - 1);   // its commit was waited for above
+    load_b(it + TEAMS);
+  }
+  if (u >= 1) {
+    mbar_wait_ab(full(u - 1), ((u - 1) >> 1) & 1, abort_flag, a.err);
+    epilogue(team + (u - 1) * TEAMS, u - 1);
+    // after a failed wait: own MMAs complete before the accumulators are freed
+    if (last >= 0 && *abort_flag) mbar_wait(full(last), (last >> 1) & 1);
   }
   tc_before_sync();
   __syncthreads();
@@ -524,17 +490,6 @@ static void build_consts(std::vector<uint8_t> &img) {
                            (((kb >> 4) ^ (n & 7)) << 4) + (kb & 15);
         put(off, v);
       }
-    // B1: 32 rows (n = 2 j1 + co) x 32 K (k = 2 f1 + ci), 2 k-steps, no swizzle
-    for (int n = 0; n < 32; n++)
-      for (int k = 0; k < 32; k++) {
-        const double x = realified(n >> 1, n & 1, k >> 1, k & 1, 16);
-        const uint16_t hi = to16<FP16>(x);
-        const uint16_t v = h == 0 ? hi : to16<FP16>(x - from16<FP16>(hi));
-        const int ks = k >> 4, kk = k & 15;
-        const size_t off = OFF_B1 + (h * 2 + ks) * 1024 + (n >> 3) * 256 + (kk >> 3) * 128 +
-                           (n & 7) * 16 + (kk & 7) * 2;
-        put(off, v);
-      }
   }
   // twiddles W512^(f2 j1) laid out [j1][f2], so a warp (f2 = lane) reads 32
   // consecutive entries
@@ -558,10 +513,10 @@ int tc_coarse_create(TcCoarse **out, int m, int ntmpl, int ndata, int fp16) {
   if (e == cudaSuccess) e = cudaMemcpy(c->consts, img.data(), img.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMalloc(&c->err, sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(c->err, 0, sizeof(int));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(coarse_tc_ws_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, tcw::SMEM_BYTES);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(coarse_tc_ws_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tcw::SMEM_BYTES);
+  for (auto k : {coarse_tc_ws_kernel<0, false>, coarse_tc_ws_kernel<0, true>,
+                 coarse_tc_ws_kernel<1, false>, coarse_tc_ws_kernel<1, true>})
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, tcw::SMEM_BYTES);
   int dev = 0, sms = 0, smem_sm = 0;
   if (e == cudaSuccess) e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -571,7 +526,7 @@ int tc_coarse_create(TcCoarse **out, int m, int ntmpl, int ndata, int fp16) {
     tc_coarse_destroy(c);
     return -1;
   }
-  // One 512-thread CTA per SM (all 128 registers x 512 threads; 256 TMEM columns).
+  // One 512-thread CTA per SM (all 128 registers x 512 threads; all TMEM columns).
   c->grid = sms;
   c->blocks_per_sm = 1;
   *out = c;
@@ -607,8 +562,8 @@ int tc_coarse_run(TcCoarse *c, const TcRunArgs &r, cudaStream_t s) {
   a.fire_count = r.fire_count;
   a.coarse_out = r.coarse_out;
   a.err = c->err;
-  if (c->fp16) coarse_tc_ws_kernel<1><<<c->grid, tcw::THREADS, tcw::SMEM_BYTES, s>>>(a);
-  else coarse_tc_ws_kernel<0><<<c->grid, tcw::THREADS, tcw::SMEM_BYTES, s>>>(a);
+  if (c->fp16) coarse_tc_ws_kernel<1, false><<<c->grid, tcw::THREADS, tcw::SMEM_BYTES, s>>>(a);
+  else coarse_tc_ws_kernel<0, false><<<c->grid, tcw::THREADS, tcw::SMEM_BYTES, s>>>(a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { g_tc_err = cudaGetErrorString(e); return -1; }
   return 0;
@@ -627,8 +582,8 @@ int tc_coarse_rows(TcCoarse *c, const float2 *rows, long long nrows, int n2, int
   a.coarse_out = m2_out;
   a.err = c->err;
   a.rows_n2 = n2; a.cs = cs; a.ce = ce;
-  if (c->fp16) coarse_tc_ws_kernel<1><<<c->grid, tcw::THREADS, tcw::SMEM_BYTES, s>>>(a);
-  else coarse_tc_ws_kernel<0><<<c->grid, tcw::THREADS, tcw::SMEM_BYTES, s>>>(a);
+  if (c->fp16) coarse_tc_ws_kernel<1, true><<<c->grid, tcw::THREADS, tcw::SMEM_BYTES, s>>>(a);
+  else coarse_tc_ws_kernel<0, true><<<c->grid, tcw::THREADS, tcw::SMEM_BYTES, s>>>(a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { g_tc_err = cudaGetErrorString(e); return -1; }
   return 0;

@@ -42,9 +42,9 @@ N, ND, NT, BINSIZE, BAND = 4096, 16, 1024, 256, 512
 SNR, FD, THRESHOLD = 5.5, 1e-2, 5.5
 FLOPS_PER_PAIR = lambda n: 5 * n * int(np.log2(n)) + 9 * n   # the reference's own convention
 # Tensor-core flops the coarse pass executes per pair at band 512: per 8 pairs,
-# stage 1 = 12 MMAs of M128 x N32 x K16 and stage 2 = 12 MMAs of M128 x N64 x K16
-# (hi*hi + hi*lo + lo*hi included), 2 flops per multiply-add.
-TC_FLOPS_PER_PAIR = (12 * 128 * 32 * 16 * 2 + 12 * 128 * 64 * 16 * 2) / 8
+# 12 MMAs of M128 x N64 x K16 (hi*hi + hi*lo + lo*hi included), 2 flops per
+# multiply-add; the 16-point first stage runs on the CUDA cores.
+TC_FLOPS_PER_PAIR = 12 * 128 * 64 * 16 * 2 / 8
 # DRAM bytes per launch from one ncu capture of the same kernels on this workload
 # (profiles/coarse_tc_ws_band512_16x1024.md, profiles/flat_kernel_n4096_16x1024.md).
 TRAFFIC_COARSE_TC = 4.347e6

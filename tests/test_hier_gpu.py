@@ -226,3 +226,39 @@ def test_band_selected_by_measured_cost():
     # the choice is kept until the bank or the reference changes
     hf.run(binsize=1024, threshold=5.5)
     assert hf.selection is sel
+
+
+@pytest.mark.parametrize("kind", ["bf16x3", "fp16x3"])
+@pytest.mark.parametrize("nd, nt", [(1, 1), (9, 1), (1, 2), (7, 3), (3, 5), (40, 31), (2, 600)])
+def test_tensor_core_coarse_pairing(kind, nd, nt):
+    """The band-512 pass takes pairs two to a warp and eight to an item: odd
+    counts, one template (every pair opens a data row), items across rows, fewer
+    items than teams and more; whole and partial windows.  Coarse maxima against FP64.
+    Bound: with f = 32 f1 + f2 the tensor cores sum Y[j1, f2] W over f2, Y the 16-point
+    transforms; a BF16 hi + lo pair is within 2^-17 of its value and the lo * lo
+    products (2^-16 at most) are left out, so z is within 4 * 2^-17 of sum |Y[j1, f2]|
+    (FP16: 2^-22 each and as much again for the FP32 sums, 8 * 2^-22), and so is a
+    maximum, however small the window makes it."""
+    mf = _mf()
+    n, band = 4096, 512
+    rng = np.random.default_rng(nd * 1000 + nt)
+    D, H = noise(rng, (nd, n)), noise(rng, (nt, n))
+    P = (np.abs(H) ** 2).mean(0).astype(np.float32)
+    hf = mf.HierarchicalFilter(n, nd, nt, band=band, coarse=kind)
+    hf.set_reference(P)
+    hf.set_coarse_threshold(1.0)
+    hf.set_data(D)
+    hf.set_templates(H)
+    for window in (None, (n // 3, n // 2), (0, 8)):
+        lo, hi = (0, n) if window is None else window
+        cs, ce = max(0, lo // 8 - 1 if lo >= 8 else 0), min(band, -(-hi // 8))
+        f = float(np.float32(P[:band].astype(np.float64).sum() / P.astype(np.float64).sum()))
+        want, scale = np.empty((nd, nt)), np.empty((nd, nt))
+        for d in range(nd):
+            P64 = D[d, :band].astype(np.complex128) * np.conj(H[:, :band])
+            z = np.fft.ifft(P64, axis=1) * band
+            Y = np.fft.ifft(P64.reshape(nt, 16, 32), axis=1) * 16
+            want[d] = np.abs(z[:, cs:ce]).max(1) / np.sqrt(f)
+            scale[d] = np.abs(Y).sum(2).max(1) / np.sqrt(f)
+        bound = scale * (2.0 ** -15 if kind == "bf16x3" else 2.0 ** -19)
+        assert (np.abs(hf.coarse_values(window=window) - want) <= bound).all()
