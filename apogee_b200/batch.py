@@ -38,6 +38,10 @@ PEAK_DTYPE = np.dtype([("index", "<i8"), ("value", "<c8")])
 #: other jobs' work (microseconds; B200 measurement order of magnitude).
 DEDICATED_LAUNCH_US = 10.0
 
+#: Pairs up to which a job of n = 32768 runs on thread-block clusters (as the
+#: library's own rule has it for runs that are not captured).
+CLUSTER_PAIRS = 64
+
 
 def dedicated(job, cfg):
     """True if ``job`` runs as its own launches under configuration ``cfg``."""
@@ -215,6 +219,9 @@ class BatchedFilter:
         own = {"index": i, "plan": plan, "keep": []}
         try:
             _lib.check(L.mfb_set_stream(plan, self._stream()))
+            if j.n == 32768 and j.pairs > CLUSTER_PAIRS:
+                # the plan is this job's alone: its runs never overlap, captured or not
+                _lib.check(L.mfb_set_cluster(plan, 0))
             h = _device_complex(j.templates, self._dev)
             _lib.check(L.mfb_set_templates(plan, 0, j.nt, h.data_ptr()))
             own["keep"].append(h)             # until the copy is done (constructor syncs)

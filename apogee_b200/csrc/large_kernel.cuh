@@ -67,7 +67,7 @@ __device__ __forceinline__ void large_pair(const LargeArgs &a, long long pi, int
     d = row / a.nt;
     t = row - d * a.nt;
   } else {
-    t = (int)(pi / a.nd);
+    t = (pi >> 32) ? (int)(pi / a.nd) : (int)((unsigned)pi / (unsigned)a.nd);
     d = (int)(pi - (long long)t * a.nd);
     row = d * a.nt + t;
   }

@@ -26,6 +26,7 @@
 #include "band_kernels.cuh"
 #include "large_kernel.cuh"
 #include "cluster_kernel.cuh"
+#include "large2_kernel.cuh"
 #include "adjoint_kernel.cuh"
 #include "batch_kernel.cuh"
 #include "gate_kernels.cuh"
@@ -146,9 +147,9 @@ static int make_const(int device, NConst &c) {
     for (size_t i = 0; i < tw.size(); i++) tw2[i] = make_float4(tw[i].x, tw[i].x, tw[i].y, tw[i].y);
     CUDA_TRY(cudaMalloc(&c.twid2, tw2.size() * sizeof(float4)));
     CUDA_TRY(cudaMemcpy(c.twid2, tw2.data(), tw2.size() * sizeof(float4), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaFuncSetAttribute(flat2_kernel<MODE_PEAKS>,
   }
   if constexpr (N == Flat2Geo::N) {
+    CUDA_TRY(cudaFuncSetAttribute(flat2_kernel<MODE_PEAKS>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, Flat2Geo::SMEM));
     int b5 = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b5, flat2_kernel<MODE_PEAKS>,
@@ -169,8 +170,8 @@ static int make_const(int device, NConst &c) {
                                                            Flat2wGeo::SMEM));
     if (b5 < 1 || b6 < 1) return fail(MFB_ERR_CUDA, "packed kernel for n=%d cannot be resident", N);
     c.grid2 = b5 * sms;
-  }
     c.grid2w = b6 * sms;
+  }
   c.grid_rows = b4 * sms;
   c.grid_peaks = b1 * sms;
   c.grid_gate = b2 * sms;
@@ -218,21 +219,21 @@ static cudaError_t launch_flat(int n, const NConst &c, const FlatArgs &a, cudaSt
 // The two-pairs-per-thread kernel covers n = 4096 peaks over the whole lag
 // window with bins a multiple of 32 lags and at most KEYCAP bins, dense or
 // listed; it gives the same bits as flat_kernel / rows_kernel.
-static bool flat2_applies(int n, const NConst &c, const FlatArgs &a) {
 static bool flat2w_applies(int n, const FlatArgs &a) {
   return n == Flat2wGeo::N && (a.ws & 255) == 0 && (a.we & 255) == 0 && (a.binsize & 255) == 0;
 }
+static bool flat2_applies(int n, const NConst &c, const FlatArgs &a) {
   return flat2w_applies(n, a) || (n == Flat2Geo::N && c.twid2 && a.ws == 0 && a.we == n &&
                                   (a.binsize & 31) == 0 && a.nb <= KEYCAP);
 }
 
 static cudaError_t launch_flat2(const NConst &c, FlatArgs a, cudaStream_t s) {
-  a.twid = reinterpret_cast<const float2 *>(c.twid2);
   if (flat2w_applies(Flat2wGeo::N, a)) {
     a.twid = reinterpret_cast<const float2 *>(c.twid2w);
     flat2w_kernel<<<c.grid2w, Flat2wGeo::T, Flat2wGeo::SMEM, s>>>(a);
     return cudaGetLastError();
   }
+  a.twid = reinterpret_cast<const float2 *>(c.twid2);
   flat2_kernel<MODE_PEAKS><<<c.grid2, Flat2Geo::T, Flat2Geo::SMEM, s>>>(a);
   return cudaGetLastError();
 }
@@ -280,8 +281,38 @@ struct LargeConst {
   // n = 32768 / 65536: one thread-block cluster per pair (cluster_kernel);
   // cl[0]: 256-thread CTAs, cl[1]: 512-thread CTAs
   ClusterCfg cl[2];
+  // large2_kernel: pass-A twiddle anchors, units per item of both kinds, and its grid
+  float2 *anchors = nullptr;
+  int units_a = 0, units_b = 0, grid2 = 0;
 };
 static std::map<std::pair<int, int>, LargeConst> g_large;
+
+// large2_kernel at every supported split.
+#define LARGE2_SPLITS(X) X(128, 256) X(256, 256) X(256, 512) X(512, 512) X(512, 1024) X(1024, 1024)
+
+constexpr int large2_smem(int nb) { return LARGE2_BUF * 16 + 2 * nb * 8; }
+
+template <int N1, int N2>
+static int large2_attr(LargeConst &c, int sms) {
+  CUDA_TRY(cudaFuncSetAttribute(large2_kernel<N1, N2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                large2_smem(LARGE_MAX_BINS)));
+  int b = 0;
+  CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, large2_kernel<N1, N2>, 256,
+                                                         large2_smem(LARGE_MAX_BINS)));
+  if (b < 1) return fail(MFB_ERR_CUDA, "large kernel (%d x %d) cannot be resident", N1, N2);
+  c.units_a = N1 / large2_cols<N2>();
+  c.units_b = N2 / (256 / (N1 / 16));
+  c.grid2 = 2 * sms;      // two CTAs per SM (registers and shared memory at up to ~2700 bins)
+  LargeArgs a;
+  memset(&a, 0, sizeof a);
+  a.n = N1 * N2;
+  a.tw_hi = c.tw_hi; a.tw_lo = c.tw_lo; a.lo_bits = c.lo_bits;
+  CUDA_TRY(cudaMalloc(&c.anchors, (size_t)c.units_a * 5 * 256 * sizeof(float2)));
+  large2_anchors<N2><<<c.units_a, 256>>>(a, c.anchors);
+  CUDA_TRY(cudaGetLastError());
+  CUDA_TRY(cudaDeviceSynchronize());
+  return MFB_OK;
+}
 
 template <int N2>
 static int large_a_attr(int *grid, int *smem, int *cta, int sms) {
@@ -416,6 +447,10 @@ static int get_large(int device, int n, LargeConst **out) {
     default: return fail(MFB_ERR_UNSUPPORTED, "no four-step split for n=%d", n);
   }
   if (r) return r;
+#define L2_CASE(A, B) if (c.N1 == A && c.N2 == B) r = large2_attr<A, B>(c, sms);
+  LARGE2_SPLITS(L2_CASE)
+#undef L2_CASE
+  if (r) return r;
   if (n == 32768) {
     r = cluster_attr<128, 256, 8>(c.cl[0]);
     if (r == MFB_OK) r = cluster_attr<128, 256, 4>(c.cl[1]);
@@ -453,6 +488,14 @@ static cudaError_t launch_large(const LargeConst &c, const LargeArgs &a, cudaStr
   return cudaGetLastError();
 }
 
+static cudaError_t launch_large2(const LargeConst &c, const Large2Args &g, int grid, cudaStream_t s) {
+  const int smem = large2_smem(g.a.nb);
+#define L2_CASE(A, B) if (c.N1 == A && c.N2 == B) large2_kernel<A, B><<<grid, 256, smem, s>>>(g);
+  LARGE2_SPLITS(L2_CASE)
+#undef L2_CASE
+  return cudaGetLastError();
+}
+
 static cudaError_t launch_large_fwd(const LargeConst &c, const LargeArgs &a, const LargeFwd &f,
                                     cudaStream_t s) {
   switch (c.N2) {
@@ -479,6 +522,42 @@ extern "C" size_t mfb_nbins(size_t n, size_t binsize, size_t start, size_t end) 
 }
 
 // ---------------------------------------------------------------- flat plan
+// large2_kernel's scratch: rows, candidate records and counters (both zero
+// between launches) of `ring` items, and the mapped error word.
+struct LargeScratch {
+  float4 *Y = nullptr;      // one allocation: Y, then rec, then ctl
+  uint4 *rec = nullptr;
+  Large2Ctl *ctl = nullptr;
+  int *err = nullptr;       // from g_err_words
+  cudaEvent_t used = nullptr;   // after the last use outside a capture
+  int ring = 0;
+};
+
+// Mapped host words for the error flags of large2_kernel launches, a page at a
+// time and given back with the scratch that held them: page-locking memory for
+// every plan would cost it about a millisecond.
+static std::mutex g_err_mu;
+static std::vector<int *> g_err_words;
+static cudaError_t take_err_word(int **out) {
+  std::lock_guard<std::mutex> lk(g_err_mu);
+  if (g_err_words.empty()) {
+    constexpr int WORDS = 1024;
+    int *page = nullptr;
+    cudaError_t e = cudaHostAlloc(&page, WORDS * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
+    if (e != cudaSuccess) return e;
+    for (int i = 0; i < WORDS; i++) g_err_words.push_back(page + i);
+  }
+  *out = g_err_words.back();
+  g_err_words.pop_back();
+  **out = 0;
+  return cudaSuccess;
+}
+static void give_err_word(int *w) {
+  if (!w) return;
+  std::lock_guard<std::mutex> lk(g_err_mu);
+  g_err_words.push_back(w);
+}
+
 struct mfb_plan {
   int device = 0;
   size_t n = 0;
@@ -492,13 +571,12 @@ struct mfb_plan {
   int starts_cap = 0;
   float2 *sspec = nullptr;
   int sspec_rows = 0;
-  // large-n (two-pass) state: constants, L2-sized scratch, candidate records
+  // large-n state: constants and scratch (with rings outgrown by later runs)
   LargeConst *lc = nullptr;
-  float2 *lY = nullptr;
-  uint4 *lrec = nullptr;
-  int lbatch = 0;
+  LargeScratch ls;
+  std::vector<LargeScratch> ls_old;
   int packed = 1;           // use flat2_kernel where it applies (mfb_set_packed)
-  int cluster = 0;          // cluster_kernel geometry where it applies (mfb_set_cluster)
+  int cluster = -1;         // mfb_set_cluster's choice; -1: cluster_mode's rule
 };
 
 struct DeviceGuard {
@@ -509,6 +587,9 @@ struct DeviceGuard {
   }
   ~DeviceGuard() { if (prev >= 0 && prev != dev_) cudaSetDevice(prev); }
 };
+
+static int large_scratch(mfb_plan *p, long long pairs);
+extern "C" int mfb_destroy(mfb_plan *p);
 
 extern "C" int mfb_create(mfb_plan **out, size_t n, int ndata, int ntmpl, int device) {
   if (!out) return fail(MFB_ERR_ARG, "null output handle");
@@ -524,7 +605,6 @@ extern "C" int mfb_create(mfb_plan **out, size_t n, int ndata, int ntmpl, int de
   mfb_plan *p = new mfb_plan;
   p->device = device;
   p->n = n;
-  p->cluster = n == 32768 ? 1 : 0;   // the faster kernel at each length (mfb_set_cluster)
   p->nd = ndata;
   p->nt = ntmpl;
   int r = is_large(n) ? get_large(device, (int)n, &p->lc) : get_const(device, (int)n, &p->c);
@@ -541,9 +621,16 @@ extern "C" int mfb_create(mfb_plan **out, size_t n, int ndata, int ntmpl, int de
   cudaMemset(p->data, 0, (size_t)ndata * n * sizeof(float2));
   cudaMemset(p->tmpl, 0, (size_t)ntmpl * n * sizeof(float2));
   CUDA_TRY(cudaDeviceSynchronize());
+  if (n == 32768) {
+    // runs at this length never allocate (they may be captured at the first call)
+    r = large_scratch(p, (long long)ndata * ntmpl);
+    if (r != MFB_OK) { mfb_destroy(p); return r; }
+  }
   *out = p;
   return MFB_OK;
 }
+
+static void large_free(LargeScratch &s);
 
 extern "C" int mfb_destroy(mfb_plan *p) {
   if (!p) return MFB_OK;
@@ -553,8 +640,8 @@ extern "C" int mfb_destroy(mfb_plan *p) {
   cudaFree(p->tmpl);
   cudaFree(p->starts_dev);
   cudaFree(p->sspec);
-  cudaFree(p->lY);
-  cudaFree(p->lrec);
+  large_free(p->ls);
+  for (LargeScratch &s : p->ls_old) large_free(s);
   delete p;
   return MFB_OK;
 }
@@ -618,39 +705,101 @@ static FlatArgs base_args(const mfb_plan *p, int d0, int nd, int t0, int nt, siz
   return a;
 }
 
-// Two-pass path for n > 16384.  list/nlist: listed output rows (host count),
-// or nullptr for the dense block.  Scratch is allocated on first use.
-#ifndef MFB_LARGE_SCRATCH_MB
-#define MFB_LARGE_SCRATCH_MB 64
-#endif
-static int large_scratch(mfb_plan *p) {
-  if (!p->lY) {
-    const size_t per = p->n * sizeof(float2);
-    int b = (int)std::max<size_t>(1, ((size_t)MFB_LARGE_SCRATCH_MB << 20) / per);
-    CUDA_TRY(cudaMalloc(&p->lY, (size_t)b * per));
-    CUDA_TRY(cudaMalloc(&p->lrec, (size_t)b * LARGE_MAX_BINS * sizeof(uint4)));
-    p->lbatch = b;
+static bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
   }
+  return cs != cudaStreamCaptureStatusNone;
+}
+// Scratch of the large-n kernel, allocated on first use: a ring of item slots
+// (two pairs each), two and a half times the kernel's delay between an item's two
+// passes, or as many as the run has items if those are fewer (two at least).  A run
+// with more items (run_series over many blocks) gets a larger ring; the smaller
+// one is kept until the plan goes, because captured graphs may hold it.
+static size_t large_rec_bytes(int ring) { return (size_t)ring * 2 * LARGE_MAX_BINS * sizeof(uint4); }
+static size_t large_ctl_bytes(int ring) { return sizeof(Large2Ctl) + (size_t)ring * 3 * sizeof(unsigned); }
+
+static void large_free(LargeScratch &s) {
+  cudaFree(s.Y);
+  if (s.used) cudaEventDestroy(s.used);
+  give_err_word(s.err);
+  s = LargeScratch();
+}
+static int large_scratch(mfb_plan *p, long long pairs) {
+  LargeScratch &cur = p->ls;
+  if (cur.ring && *(volatile int *)cur.err) {   // an earlier launch gave up half-way: start afresh
+    CUDA_TRY(cudaDeviceSynchronize());
+    CUDA_TRY(cudaMemset(cur.rec, 0, large_rec_bytes(cur.ring) + large_ctl_bytes(cur.ring)));
+    CUDA_TRY(cudaDeviceSynchronize());
+    *cur.err = 0;
+    return fail(MFB_ERR_CUDA, "an earlier run at n=%zu timed out on a dependency; its outputs are invalid", p->n);
+  }
+  pairs = std::max(pairs, (long long)p->nd * p->nt);
+  const int per = (p->lc->units_a + p->lc->units_b) / LARGE2_GROUP;
+  const long long most = large2_delay(p->lc->grid2, per) * 5 / 2;
+  const int ring = (int)std::max<long long>(2, std::min((pairs + 1) / 2, most));
+  if (cur.ring >= ring) return MFB_OK;
+  LargeScratch s;
+  s.ring = ring;
+  const size_t rows = (size_t)ring * p->n * sizeof(float4), rest = large_rec_bytes(ring) + large_ctl_bytes(ring);
+  cudaError_t e = cudaMalloc(&s.Y, rows + rest);
+  if (e == cudaSuccess) {
+    s.rec = reinterpret_cast<uint4 *>(reinterpret_cast<char *>(s.Y) + rows);
+    s.ctl = reinterpret_cast<Large2Ctl *>(reinterpret_cast<char *>(s.rec) + large_rec_bytes(ring));
+    e = cudaMemset(s.rec, 0, rest);
+  }
+  if (e == cudaSuccess) e = take_err_word(&s.err);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s.used, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();   // before any stream uses them
+  if (e != cudaSuccess) {
+    large_free(s);
+    return fail(MFB_ERR_CUDA, "large-n scratch for n=%zu: %s", p->n, cudaGetErrorString(e));
+  }
+  if (cur.ring) p->ls_old.push_back(cur);
+  cur = s;
   return MFB_OK;
 }
+// Runs of one plan enqueued on different streams share its scratch: each waits
+// for the one before.  (A captured run is ordered by whoever launches its graph.)
+static cudaError_t scratch_begin(const mfb_plan *p) {
+  return capturing(p->stream) ? cudaSuccess : cudaStreamWaitEvent(p->stream, p->ls.used, 0);
+}
+static cudaError_t scratch_end(const mfb_plan *p) {
+  return capturing(p->stream) ? cudaSuccess : cudaEventRecord(p->ls.used, p->stream);
+}
+// Series blocks that fit the scratch.
+static int large_rows(const mfb_plan *p) { return p->ls.ring * 2; }
 
-// data: the rows to filter (default the plan's data rows).
-static bool cluster_applies(const mfb_plan *p) {
-  return p->cluster > 0 && p->lc && p->lc->cl[p->cluster - 1].C > 0;
+// The cluster kernel's geometry for a run (1 or 2), or 0 for large2_kernel.  At
+// n = 32768, unless mfb_set_cluster says otherwise, lists and dense runs of up to
+// CLUSTER_PAIRS pairs take the cluster kernel (one cluster per pair has the
+// shorter latency: 1 pair 16 against 19 us, 16 pairs 20 against 21, 51 listed rows
+// of 4096 56 against 62), larger blocks large2_kernel (128 pairs 34 against
+// 38 us, 1024 pairs 152 against 258).  A captured run at that length keeps to the
+// cluster kernel, which has no scratch: its graph may run beside other runs of the
+// plan.
+constexpr long long CLUSTER_PAIRS = 64;
+static int cluster_mode(const mfb_plan *p, bool listed, long long pairs) {
+  int mode = p->cluster;
+  if (mode < 0)
+    mode = p->n == 32768 && (listed || pairs <= CLUSTER_PAIRS || capturing(p->stream)) ? 1 : 0;
+  return mode > 0 && p->lc && p->lc->cl[mode - 1].C > 0 ? mode : 0;
 }
 
-// list: listed rows, nlist of them (counted on the host for the two-pass
-// batches), or list_count on the device (the cluster kernel reads it itself).
+// list: listed rows; list_count: how many, on the device.  data: the rows to
+// filter (default the plan's data rows).
 static int run_large(mfb_plan *p, int d0, int nd, int t0, int nt, const int32_t *list,
-                     long long nlist, size_t binsize, float threshold, size_t start, size_t end,
-                     size_t nb, int64_t *idx, void *val, int32_t *counts, int rs,
-                     const float2 *data = nullptr, const int32_t *list_count = nullptr) {
+                     const int32_t *list_count, size_t binsize, float threshold, size_t start,
+                     size_t end, size_t nb, int64_t *idx, void *val, int32_t *counts, int rs,
+                     const float2 *data = nullptr) {
   if (nb > (size_t)LARGE_MAX_BINS)
     return fail(MFB_ERR_UNSUPPORTED, "n=%zu supports at most %d bins per pair", p->n, LARGE_MAX_BINS);
   const LargeConst &c = *p->lc;
-  const bool cl = cluster_applies(p) && (!list || list_count);
+  const int cl = cluster_mode(p, list != nullptr, (long long)nd * nt);
   if (!cl) {
-    int sr = large_scratch(p);
+    int sr = large_scratch(p, (long long)nd * nt);
     if (sr) return sr;
   }
   if (end > p->n) end = p->n;
@@ -661,9 +810,8 @@ static int run_large(mfb_plan *p, int d0, int nd, int t0, int nt, const int32_t 
   a.n = (int)p->n; a.N1 = c.N1; a.N2 = c.N2;
   a.d0 = d0; a.nd = nd; a.t0 = t0; a.nt = nt;
   a.list = list;
-  a.total = list ? nlist : (long long)nd * nt;
-  a.Y = p->lY;
-  a.rec = p->lrec;
+  a.list_count = list ? list_count : nullptr;
+  a.total = (long long)nd * nt;
   a.tw1 = c.c1->twid;
   a.tw2 = c.c2->twid;
   a.tw_hi = c.tw_hi;
@@ -679,17 +827,31 @@ static int run_large(mfb_plan *p, int d0, int nd, int t0, int nt, const int32_t 
   a.rs = rs;
   a.out_cnt = counts;
   if (cl) {
-    a.list_count = list ? list_count : nullptr;
-    CUDA_TRY(launch_cluster(c, p->cluster, a, list ? 0 : a.total, p->stream));
+    CUDA_TRY(launch_cluster(c, cl, a, list ? 0 : a.total, p->stream));
     return MFB_OK;
   }
-  for (long long p0 = 0; p0 < a.total; p0 += p->lbatch) {
-    a.pair0 = p0;
-    a.batch = (int)std::min<long long>(p->lbatch, a.total - p0);
-    CUDA_TRY(cudaMemsetAsync(p->lrec, 0, (size_t)a.batch * nb * sizeof(uint4), p->stream));
-    CUDA_TRY(launch_large(c, a, p->stream));
-  }
+  Large2Args g;
+  g.a = a;
+  g.tw1 = c.c1->twid2;
+  g.tw2 = c.c2->twid2;
+  g.anchors = c.anchors;
+  g.Y = p->ls.Y;
+  g.rec = p->ls.rec;
+  g.ctl = p->ls.ctl;
+  CUDA_TRY(cudaHostGetDevicePointer((void **)&g.err, p->ls.err, 0));
+  g.ring = p->ls.ring;
+  const long long items = (a.total + 1) / 2;
+  const int grid = (int)std::min<long long>(c.grid2, std::max<long long>(1, items * c.units_a));
+  CUDA_TRY(scratch_begin(p));
+  CUDA_TRY(launch_large2(c, g, grid, p->stream));
+  CUDA_TRY(scratch_end(p));
   return MFB_OK;
+}
+
+// The dense block of `a` at n <= 16384.
+static cudaError_t launch_peaks(const mfb_plan *p, const FlatArgs &a) {
+  if (p->packed && flat2_applies((int)p->n, *p->c, a)) return launch_flat2(*p->c, a, p->stream);
+  return launch_flat<MODE_PEAKS>((int)p->n, *p->c, a, p->stream);
 }
 
 static int run_impl(mfb_plan *p, int d0, int nd, int t0, int nt, size_t binsize,
@@ -709,7 +871,7 @@ static int run_impl(mfb_plan *p, int d0, int nd, int t0, int nt, size_t binsize,
   a.out_cnt = counts;
   if (counts) CUDA_TRY(cudaMemsetAsync(counts, 0, (size_t)nd * nt * sizeof(int32_t), p->stream));
   if (is_large(p->n))
-    return run_large(p, d0, nd, t0, nt, nullptr, 0, binsize, threshold, start, end, nb, idx, val,
+    return run_large(p, d0, nd, t0, nt, nullptr, nullptr, binsize, threshold, start, end, nb, idx, val,
                      counts, rs);
   CUDA_TRY(launch_peaks(p, a));
   return MFB_OK;
@@ -765,20 +927,9 @@ static int run_rows_impl(mfb_plan *p, int d0, int nd, int t0, int nt, const int3
   a.out_val = (float2 *)val;
   a.rs = rs;
   a.out_cnt = counts;   // rows not listed keep whatever the caller put there
-  if (is_large(p->n) && cluster_applies(p)) {
-    if (added) *added = false;
-    return run_large(p, d0, nd, t0, nt, rows, 0, binsize, threshold, start, end, nb, idx, val,
-                     counts, rs, nullptr, nrows);
-  }
-  if (is_large(p->n)) {
-    // the two-pass path sizes its batches on the host: read the row count
-    int32_t cnt = 0;
-    CUDA_TRY(cudaMemcpyAsync(&cnt, nrows, sizeof cnt, cudaMemcpyDeviceToHost, p->stream));
-    CUDA_TRY(cudaStreamSynchronize(p->stream));
-    if (cnt > max_rows) return fail(MFB_ERR_ARG, "row count %d exceeds max_rows %d", cnt, max_rows);
-    return run_large(p, d0, nd, t0, nt, rows, cnt, binsize, threshold, start, end, nb, idx, val,
+  if (is_large(p->n))
+    return run_large(p, d0, nd, t0, nt, rows, nrows, binsize, threshold, start, end, nb, idx, val,
                      counts, rs);
-  }
   a.trig_total = trig_total;
   if (p->packed && flat2_applies((int)p->n, *p->c, a)) {
     if (host_rec && rs == 2) {
@@ -789,12 +940,6 @@ static int run_rows_impl(mfb_plan *p, int d0, int nd, int t0, int nt, const int3
   } else {
     CUDA_TRY(launch_rows((int)p->n, *p->c, a, p->stream));
   }
-// The dense block of `a` at n <= 16384.
-static cudaError_t launch_peaks(const mfb_plan *p, const FlatArgs &a) {
-  if (p->packed && flat2_applies((int)p->n, *p->c, a)) return launch_flat2(*p->c, a, p->stream);
-  return launch_flat<MODE_PEAKS>((int)p->n, *p->c, a, p->stream);
-}
-
   if (added) *added = trig_total != nullptr;
   return MFB_OK;
 }
@@ -802,6 +947,14 @@ static cudaError_t launch_peaks(const mfb_plan *p, const FlatArgs &a) {
 extern "C" int mfb_run_rows(mfb_plan *p, int d0, int nd, int t0, int nt, const int32_t *rows,
                             const int32_t *nrows, int max_rows, size_t binsize, float threshold,
                             size_t start, size_t end, int64_t *idx, void *val, int32_t *counts) {
+  if (p && is_large(p->n) && !cluster_mode(p, true, 0) && rows && nrows && max_rows >= 0) {
+    // this length checks the list's length against max_rows: read it on the host
+    DeviceGuard dg(p->device);
+    int32_t cnt = 0;
+    CUDA_TRY(cudaMemcpyAsync(&cnt, nrows, sizeof cnt, cudaMemcpyDeviceToHost, p->stream));
+    CUDA_TRY(cudaStreamSynchronize(p->stream));
+    if (cnt > max_rows) return fail(MFB_ERR_ARG, "row count %d exceeds max_rows %d", cnt, max_rows);
+  }
   return run_rows_impl(p, d0, nd, t0, nt, rows, nrows, max_rows, binsize, threshold, start, end,
                        idx, val, counts, 1);
 }
@@ -813,14 +966,14 @@ extern "C" int mfb_forward(mfb_plan *p, const void *series, size_t nseries,
     return fail(MFB_ERR_ARG, "invalid forward-transform arguments");
   DeviceGuard dg(p->device);
   if (is_large(p->n)) {
-    int sr = large_scratch(p);
+    int sr = large_scratch(p, std::max<long long>(nblocks, (long long)p->nd * p->nt));
     if (sr) return sr;
     const LargeConst &c = *p->lc;
     LargeArgs a;
     memset(&a, 0, sizeof a);
     a.n = (int)p->n; a.N1 = c.N1; a.N2 = c.N2;
     a.total = nblocks;
-    a.Y = p->lY;
+    a.Y = reinterpret_cast<float2 *>(p->ls.Y);
     a.tw1 = c.c1->twid; a.tw2 = c.c2->twid;
     a.tw_hi = c.tw_hi; a.tw_lo = c.tw_lo; a.lo_bits = c.lo_bits;
     LargeFwd f;
@@ -829,11 +982,13 @@ extern "C" int mfb_forward(mfb_plan *p, const void *series, size_t nseries,
     f.starts = (const unsigned long long *)starts_dev;
     f.spectra = (float2 *)spectra;
     f.scale = 1.0f / (float)p->n;
-    for (long long p0 = 0; p0 < nblocks; p0 += p->lbatch) {
+    CUDA_TRY(scratch_begin(p));
+    for (long long p0 = 0; p0 < nblocks; p0 += large_rows(p)) {
       a.pair0 = p0;
-      a.batch = (int)std::min<long long>(p->lbatch, nblocks - p0);
+      a.batch = (int)std::min<long long>(large_rows(p), nblocks - p0);
       CUDA_TRY(launch_large_fwd(c, a, f, p->stream));
     }
+    CUDA_TRY(scratch_end(p));
     return MFB_OK;
   }
   SeriesArgs s;
@@ -902,7 +1057,7 @@ extern "C" int mfb_run_series(mfb_plan *p, const void *series, size_t nseries,
     if (r) return r;
     size_t lo = win_start[b0], hi = win_end[b0];
     if (is_large(p->n)) {
-      r = run_large(p, 0, g, t0, nt, nullptr, 0, binsize, threshold, lo, hi, nb0,
+      r = run_large(p, 0, g, t0, nt, nullptr, nullptr, binsize, threshold, lo, hi, nb0,
                     idx + (size_t)b0 * nt * nb0, (float2 *)val + (size_t)b0 * nt * nb0,
                     counts ? counts + (size_t)b0 * nt : nullptr, 1, p->sspec);
       if (r) return r;
@@ -1477,9 +1632,8 @@ extern "C" int mfb_hier_run_host(mfb_hplan *h, int d0, int nd, int t0, int nt, s
     return fail(MFB_ERR_ARG, "info must be pinned (page-locked, mapped) host memory");
   }
   // A graph may hold copies from pinned host memory only (a pageable copy is
-  // synchronous and cannot be captured), and the two-pass large-n refine
-  // sizes its batches on the host.
-  bool graphable = !is_large(h->n) || cluster_applies(h->full);
+  // synchronous and cannot be captured).
+  bool graphable = true;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(h->full->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
     cudaGetLastError();
@@ -1896,6 +2050,9 @@ static int adjoint_side(bool grad_data, int n, int nd, int nt, int nb, const flo
   if ((a.own + 7LL) / 8 > 65535) return fail(MFB_ERR_UNSUPPORTED, "adjoint: too many rows (%d)", a.own);
   a.fblk = std::min(n / ADJ_R, ADJ_THREADS);
   a.slots = ADJ_THREADS / a.fblk;
+  while ((1 << a.lsh) < a.fblk && a.lsh < 5) a.lsh++;
+  while ((32 << a.ash) < a.fblk) a.ash++;
+  a.tw_hi = tw.hi; a.tw_lo = tw.lo; a.lo_bits = tw.lo_bits; a.hi_count = tw.hi_count;
   a.fx = n / ADJ_R / a.fblk;
   const int cap = ADJ_TAB / adj_entry_bytes(a.fblk);
   a.chunk = std::min(std::min(nb, ADJ_CHUNK), cap / a.slots);
@@ -1995,9 +2152,6 @@ extern "C" int mfb_batch_create(mfb_batch **out, int device, const mfb_job *jobs
   CUDA_TRY(cudaGetDeviceCount(&ndev));
   if (device < 0 || device >= ndev) return fail(MFB_ERR_ARG, "no device %d", device);
   const size_t slot_bytes = (opts && opts->slot_bytes) ? opts->slot_bytes : ((size_t)64 << 20);
-  while ((1 << a.lsh) < a.fblk && a.lsh < 5) a.lsh++;
-  while ((32 << a.ash) < a.fblk) a.ash++;
-  a.tw_hi = tw.hi; a.tw_lo = tw.lo; a.lo_bits = tw.lo_bits; a.hi_count = tw.hi_count;
   const int nslots = (opts && opts->slots) ? opts->slots : 3;
   if (nslots < 2 || nslots > 64) return fail(MFB_ERR_ARG, "slots must be 2 .. 64");
   DeviceGuard dg(device);

@@ -88,26 +88,24 @@ int mfb_run_records(mfb_plan *p, int d0, int nd, int t0, int nt, size_t binsize,
 int mfb_set_packed(mfb_plan *p, int on);
 /* Kernel choice for n = 32768 and 65536 (no counterpart in the reference,
    whose CPU engine always runs its four-step plan through memory): mode 0
-   runs the two-pass kernels through the plan's L2-sized scratch; mode 1 runs
+   runs the persistent four-step kernel through the plan's scratch; mode 1 runs
    each pair on one thread-block cluster whose distributed shared memory
    holds the whole spectrum between the two passes of the four-step split --
    8 (n = 32768) or 16 (n = 65536) CTAs of 256 threads, three CTAs per SM --
-   in one launch with no scratch and no host decision (listed runs read their
-   row count on the device, so a hierarchical run at these lengths is
-   replayed as one CUDA graph); mode 2 the same with 4 / 8 CTAs of 512
-   threads, one per SM.  Same arithmetic, identical results.  The default is
-   the faster on a B200: mode 1 at n = 32768 (on a par with mode 0 on dense
-   blocks, faster on short row lists), mode 0 at 65536 (mode 1 is 1.3x
-   slower there). */
+   in one launch with no scratch; mode 2 the same with 4 / 8 CTAs of 512
+   threads, one per SM.  Same arithmetic, identical results.  Without a call, a
+   run takes the faster on a B200: at n = 32768 mode 1 for row lists, dense blocks
+   of up to 64 pairs and captured runs, mode 0 for larger blocks (1.7x faster
+   at 1024 pairs); at 65536 mode 0. */
 int mfb_set_cluster(mfb_plan *p, int mode);
 /* Replaces ap_mf_run_sel (src/matchfilt.c:492-503) in list form: run only the
    output rows rows[0..*nrows) of the block [d0,d0+nd) x [t0,t0+nt), where a row
    is (d-d0)*nt + (t-t0) and the row count lives in DEVICE memory (nrows), so a
    survivor list made on the GPU needs no host round trip.  The caller keeps
-   *nrows <= max_rows.  Every kernel reads the count on the device, except the
-   two-pass kernels (n >= 65536, and n = 32768 in cluster mode 0), which size
-   their batches on the host: there the call reads the count, synchronises the
-   plan's stream and refuses a count above max_rows. */
+   *nrows <= max_rows.  Every kernel reads the count on the device; where the
+   persistent four-step kernel runs (n >= 65536, and n = 32768 in cluster mode 0)
+   the call also reads it on the host, synchronising the plan's stream, and refuses
+   a count above max_rows. */
 int mfb_run_rows(mfb_plan *p, int d0, int nd, int t0, int nt, const int32_t *rows,
                  const int32_t *nrows, int max_rows, size_t binsize, float threshold,
                  size_t start, size_t end, int64_t *idx, void *val, int32_t *counts);

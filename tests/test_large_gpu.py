@@ -148,3 +148,107 @@ def test_band_16384_tensor_core_coarse(coarse, nd, nt, window):
     np.testing.assert_array_equal(fired, cv >= gate)
     np.testing.assert_array_equal(out[fired], ref[fired])
     assert (out["index"][~fired] == -1).all() and (out["value"][~fired] == 0).all()
+
+
+@pytest.mark.parametrize("n, nd, nt", [
+    (32768, 1, 1),       # one pair: half an item
+    (65536, 3, 141),     # odd pair count, data rows change inside items, more items than ring slots
+    (131072, 2, 3),
+    (262144, 2, 75),     # the ring of item slots is reused
+    (524288, 1, 4),
+])
+@pytest.mark.parametrize("bins", ["even", "ragged", "one"])
+def test_persistent_kernel_equals_two_pass(n, nd, nt, bins):
+    """The persistent four-step kernel (two pairs per thread, items through a ring of
+    scratch slots) against the two-pass kernels of the entry point without
+    allocation: same arithmetic, same bits; run twice, the second run on the
+    counters and records the first left behind."""
+    import torch
+    mf = _mf()
+    from apogee_b200 import _lib
+    L = _lib.lib()
+    g = torch.Generator(device="cuda").manual_seed(n + nt)
+    D = torch.randn(nd, n, dtype=torch.complex64, device="cuda", generator=g)
+    H = torch.randn(nt, n, dtype=torch.complex64, device="cuda", generator=g)
+    f = mf.MatchedFilter(n, nd, nt)
+    _lib.check(L.mfb_set_cluster(f._plan, 0))
+    f.set_data(D)
+    f.set_templates(H)
+    binsize, win = {"even": (n // 16, (0, n)), "ragged": (n // 50 + 3, (17, n - 9)),
+                    "one": (n, (0, n))}[bins]
+    for thr in (0.0, 3.3 * np.sqrt(n)):
+        nb = L.mfb_nbins(n, binsize, *win)
+        idx = torch.full((nd, nt, nb), -7, dtype=torch.int64, device="cuda")
+        val = torch.zeros(nd, nt, nb, dtype=torch.complex64, device="cuda")
+        cnt = torch.zeros(nd, nt, dtype=torch.int32, device="cuda")
+        _lib.check(L.mfb_run_large_static(0, n, D.data_ptr(), nd, H.data_ptr(), nt, binsize, thr,
+                                          *win, idx.data_ptr(), val.data_ptr(), cnt.data_ptr(),
+                                          torch.cuda.current_stream().cuda_stream))
+        for _ in range(2):
+            i2, v2 = f.run_device(binsize=binsize, threshold=thr, window=win)
+            assert torch.equal(i2, idx) and torch.equal(v2, val)
+        out, c2 = f.run(binsize=binsize, threshold=thr, window=win, counts=True)
+        np.testing.assert_array_equal(c2, cnt.cpu().numpy())
+
+
+def test_persistent_kernel_lists_and_streams():
+    """Listed rows (odd count, arbitrary order, none) give the dense run's rows;
+    runs of one plan enqueued on two streams do not disturb one another."""
+    import torch
+    mf = _mf()
+    from apogee_b200 import _lib
+    L = _lib.lib()
+    n, nd, nt = 65536, 4, 60
+    g = torch.Generator(device="cuda").manual_seed(9)
+    f = mf.MatchedFilter(n, nd, nt)
+    f.set_data(torch.randn(nd, n, dtype=torch.complex64, device="cuda", generator=g))
+    f.set_templates(torch.randn(nt, n, dtype=torch.complex64, device="cuda", generator=g))
+    ref_i, ref_v = f.run_device(binsize=n // 16)
+    ref_w, _ = f.run_device(binsize=n // 64, threshold=800.0)
+    torch.cuda.synchronize()
+    rows = torch.from_numpy(np.random.default_rng(3).permutation(nd * nt)[:77].astype(np.int32)).cuda()
+    for k in (0, 1, 77):
+        idx = torch.full((nd * nt, 16), -7, dtype=torch.int64, device="cuda")
+        val = torch.zeros(nd * nt, 16, dtype=torch.complex64, device="cuda")
+        cnt = torch.tensor([k], dtype=torch.int32, device="cuda")
+        f._bind_stream()
+        _lib.check(L.mfb_run_rows(f._plan, 0, nd, 0, nt, rows.data_ptr(), cnt.data_ptr(), 77, n // 16,
+                                  0.0, 0, n, idx.data_ptr(), val.data_ptr(), None))
+        r = rows[:k].long()
+        assert torch.equal(idx[r], ref_i.view(-1, 16)[r]) and torch.equal(val[r], ref_v.view(-1, 16)[r])
+        assert int((idx == -7).all(1).sum()) == nd * nt - k
+    cnt = torch.tensor([78], dtype=torch.int32, device="cuda")
+    assert L.mfb_run_rows(f._plan, 0, nd, 0, nt, rows.data_ptr(), cnt.data_ptr(), 77, n // 16, 0.0, 0,
+                          n, idx.data_ptr(), val.data_ptr(), None) < 0
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    got = []
+    for i in range(6):
+        with torch.cuda.stream(streams[i & 1]):
+            got.append(f.run_device(binsize=n // 16) if i % 3 else f.run_device(binsize=n // 64, threshold=800.0))
+    torch.cuda.synchronize()
+    for i, (a, b) in enumerate(got):
+        if i % 3:
+            assert torch.equal(a, ref_i) and torch.equal(b, ref_v)
+        else:
+            assert torch.equal(a, ref_w)
+
+
+def test_series_ring_grows_beyond_the_plan():
+    """run_series over more blocks than the plan has data rows: the scratch grows,
+    and the spectra and peaks stay those of the blocks."""
+    mf = _mf()
+    n, nt, blocks = 65536, 2, 40
+    rng = np.random.default_rng(5)
+    x = noise(rng, n // 2 * (blocks + 1))
+    H = noise(rng, (nt, n))
+    f = mf.MatchedFilter(n, 1, nt)
+    f.set_templates(H)
+    f.set_data(noise(rng, (1, n)))
+    f.run(binsize=n)                          # sizes the ring for one pair of rows
+    starts = np.arange(blocks) * (n // 2)
+    out = f.run_series(x, starts, np.full(blocks, n // 4), np.full(blocks, 3 * n // 4), binsize=n // 8)
+    for b in (0, 7, 39):
+        D = np.fft.fft(x[starts[b]:starts[b] + n].astype(np.complex128) / n)
+        z = oracle.correlate(D[None], H)
+        assert not parity.compare(out["index"][b][None], out["value"][b][None], z, n // 8, 0.0,
+                                  (n // 4, 3 * n // 4))
