@@ -10,17 +10,18 @@
 //  * Stockham autosort FFT, radix 16 (first pass radix 2/4/8/16), one
 //    butterfly per thread per pass.  A thread keeps 16 complex values in
 //    registers; passes exchange through padded shared memory.
-//  * The conjugate product is formed while the first pass loads: the
-//    template spectrum streams from HBM/L2 with coalesced 8-byte loads, the
-//    data spectrum a thread needs sits in its registers for as long as the
-//    CTA stays on that data row.
+//  * The conjugate product is formed while the first pass loads: template and
+//    data spectra come from HBM, L2 or L1 with coalesced 8-byte loads (a CTA stays
+//    on a data row for many pairs; registers are better spent on a third CTA per SM
+//    than on keeping the row, FlatGeo::MINB).
 //  * Thread t ends holding z[t + T*q], q = 0..15 (T = n/16).  The per-bin
 //    argmax is a warp redux on |z|^2 bit patterns followed by one 64-bit
 //    shared-memory atomicMax per warp and bin on the key
 //    (|z|^2 bits << 32) | ~lag, which makes the lowest lag win exact ties.
 //  * Persistent CTAs walk a contiguous range of pairs, data row outer,
-//    template inner, so the data spectrum is reloaded only when the row
-//    changes and concurrent CTAs on different rows share templates in L2.
+//    template inner, so concurrent CTAs on different rows share templates in L2.
+//  * Runs whose bins and window are whole blocks of n/16 lags at n >= 512 take
+//    flatw_kernel instead (same bits), and so do the gate passes at those lengths.
 //
 // Threshold contract (src/balanced-inl.h:804-886): a bin reports the lag of
 // max |z|^2 iff that |z|^2 > thr^2 (thr <= 0 -> > 0, so zero is never a
@@ -64,7 +65,7 @@ struct FlatArgs {
   // (the hierarchical plan's trigger count) -- one thread, once
   unsigned long long *trig_total;
   // if set (record output, rs == 2): every output record is also stored here,
-  // the caller's pinned host table seen from the device (flat2_kernel only)
+  // the caller's pinned host table seen from the device (flatw_kernel only)
   int4 *host_rec;
 };
 
@@ -80,6 +81,11 @@ struct FlatGeo {
   static constexpr int CTA = T >= 256 ? T : 256;
   static constexpr int G = CTA / T;                      // pairs in flight per CTA
   static constexpr int BUF = N + N / 16;                 // padded float2 per pair
+  // CTAs per SM the registers are held to (80 / 64 / 64 a thread).  Warps in
+  // flight are worth more here than a data row kept in registers (two CTAs of 128
+  // registers): 16 x 1024 pairs at n = 2048 106 -> 90 us, n = 4096 205 -> 174; four
+  // CTAs spill.
+  static constexpr int MINB = CTA <= 256 ? 3 : CTA <= 512 ? 2 : 1;
   // + double-buffered key slots (KEYCAP = 64) + per-warp slot staging
   static constexpr int SMEM = G * BUF * 8 + G * 2 * 64 * 8 + G * (T >= 32 ? T / 32 : 1) * 16 * 4;
 };
@@ -158,6 +164,19 @@ __device__ __forceinline__ void pass_twiddles(cf *v, const float2 *tw, int strid
   v[15] = cmul(v[15], cmul(w12, w3));
 }
 
+// Pass 0 of a thread's 16 values: 16/R butterflies of radix R, the b-th on v[b + (16/R) q].
+template <int R>
+__device__ __forceinline__ void first_pass(cf *v) {
+  if constexpr (R == 16) dftR<16, 0, 1>(v);
+  else if constexpr (R == 8) { dftR<8, 0, 2>(v); dftR<8, 1, 2>(v); }
+  else if constexpr (R == 4) { dftR<4, 0, 4>(v); dftR<4, 1, 4>(v); dftR<4, 2, 4>(v); dftR<4, 3, 4>(v); }
+  else {
+    static_assert(R == 2, "first radix 2, 4, 8 or 16");
+    dft2<0, 8>(v); dft2<1, 8>(v); dft2<2, 8>(v); dft2<3, 8>(v);
+    dft2<4, 8>(v); dft2<5, 8>(v); dft2<6, 8>(v); dft2<7, 8>(v);
+  }
+}
+
 // Unnormalised inverse FFT of the n values x[t + T*s] = v[s] held by the T
 // threads of one pair slot (Stockham autosort: pass 0 radix R0, then radix
 // 16).  On return v[q] = X[t + T*q].  buf is this slot's padded shared buffer;
@@ -168,22 +187,7 @@ __device__ __forceinline__ void inverse_passes(cf *v, float2 *buf, const float2 
   using Geo = FlatGeo<N>;
   constexpr int T = Geo::T, R0 = Geo::R0, PASSES = Geo::PASSES;
   constexpr int B0 = 16 / R0;   // butterflies per thread in pass 0
-#pragma unroll
-  for (int b = 0; b < B0; b++) {
-    if constexpr (R0 == 16) dftR<16, 0, 1>(v);
-    else if constexpr (R0 == 8) { if (b == 0) dftR<8, 0, 2>(v); else dftR<8, 1, 2>(v); }
-    else if constexpr (R0 == 4) {
-      if (b == 0) dftR<4, 0, 4>(v); else if (b == 1) dftR<4, 1, 4>(v);
-      else if (b == 2) dftR<4, 2, 4>(v); else dftR<4, 3, 4>(v);
-    } else {
-      switch (b) {   // R0 == 2: slots b and b + 8
-        case 0: dft2<0, 8>(v); break; case 1: dft2<1, 8>(v); break;
-        case 2: dft2<2, 8>(v); break; case 3: dft2<3, 8>(v); break;
-        case 4: dft2<4, 8>(v); break; case 5: dft2<5, 8>(v); break;
-        case 6: dft2<6, 8>(v); break; default: dft2<7, 8>(v); break;
-      }
-    }
-  }
+  first_pass<R0>(v);
   pass_sync<CTA_SYNC>(T);
   // Pass 0 output j*R0 + q (j = t + T*b, q < R0): R0 divides 16, so the
   // 16-block of t*R0 holds every q, and T*R0 is a multiple of 16.
@@ -539,7 +543,7 @@ __device__ __forceinline__ void flat_range(const FlatArgs &a, long long ibeg, lo
 // n = 4096, CUDA events, L2 flushed), while flat_range's short dynamic ranges
 // in the batched kernel need the entry barrier and the coherent-load switch.
 template <int N, int MODE>
-__global__ void __launch_bounds__(FlatGeo<N>::CTA, FlatGeo<N>::CTA <= 256 ? 2 : 1)
+__global__ void __launch_bounds__(FlatGeo<N>::CTA, FlatGeo<N>::MINB)
 flat_kernel(const FlatArgs a) {
   using Geo = FlatGeo<N>;
   constexpr int T = Geo::T, G = Geo::G;
@@ -556,13 +560,6 @@ flat_kernel(const FlatArgs a) {
   const long long ibeg = blockIdx.x * per + (blockIdx.x < extra ? blockIdx.x : extra);
   const long long iend = ibeg + per + (blockIdx.x < extra ? 1 : 0);
 
-  // The data row stays in registers while consecutive pairs share it; 1024
-  // threads have 64 registers each, too few for it beside the transform (kept, it
-  // spilled: 149 us for 6 x 300 pairs at n = 16384, threshold 4.5, against 126 us
-  // reloaded from L2).
-  constexpr bool CACHE_D = Geo::CTA <= 512;
-  cf dreg[CACHE_D ? 16 : 1];
-  int cur_d = -1;
   const int lane = threadIdx.x & 31;
 
   // Bin bookkeeping, once per launch.
@@ -617,20 +614,9 @@ flat_kernel(const FlatArgs a) {
     if (live) {
       const float2 *dp = a.data + (long long)(a.d0 + d) * a.data_stride;
       const float2 *hp = a.tmpl + (long long)(a.t0 + tt) * a.tmpl_stride;
-      if (CACHE_D && d != cur_d) {
-#pragma unroll
-        for (int s = 0; s < 16; s++) {
-          float2 x = __ldg(dp + t + T * s);
-          dreg[CACHE_D ? s : 0] = {x.x, x.y};
-        }
-        cur_d = d;
-      }
 #pragma unroll
       for (int s = 0; s < 16; s++) {
-        float2 h = __ldg(hp + t + T * s);
-        cf x;
-        if constexpr (CACHE_D) x = dreg[s];
-        else { const float2 y = __ldg(dp + t + T * s); x = {y.x, y.y}; }
+        const float2 x = __ldg(dp + t + T * s), h = __ldg(hp + t + T * s);
         // D * conj(H)
         v[s].x = fmaf(x.x, h.x, x.y * h.y);
         v[s].y = fmaf(x.y, h.x, -x.x * h.y);
@@ -816,13 +802,9 @@ flat_kernel(const FlatArgs a) {
 }
 
 // Listed mode on its own: the output rows of a device row list (the
-// hierarchical refine, mfb_run_rows).  Survivor lists are short and in
-// arbitrary order, so the run is latency bound (a few pairs per CTA, each
-// loading its own data row): without the data-row cache the kernel fits in
-// 80 registers and three 256-thread CTAs per SM, 444 pairs in flight instead
-// of 296 on 148 SMs.
+// hierarchical refine, mfb_run_rows) with bins that flatw_kernel does not take.
 template <int N>
-__global__ void __launch_bounds__(FlatGeo<N>::CTA, FlatGeo<N>::CTA <= 256 ? 3 : 1)
+__global__ void __launch_bounds__(FlatGeo<N>::CTA, FlatGeo<N>::MINB)
 rows_kernel(const FlatArgs a) {
   using Geo = FlatGeo<N>;
   extern __shared__ __align__(16) float2 smem[];
