@@ -25,12 +25,11 @@
 // previous pair -> rows written -> every CTA's keys final); one more before
 // exit keeps every CTA's shared memory alive while the others read from it.
 // Clusters of 8 or 16 CTAs of 256 threads (4096 points each, three CTAs per
-// SM) or of 4 / 8 CTAs of 512 threads (8192 points, one per SM).  Measured
-// on a B200 against the two-pass kernels (the default): 0.35 vs 0.31 us per
-// pair at n = 32768 and 0.82 vs 0.60 at 65536 on dense blocks with binsize
-// n/16 (pass B takes ~45% of a CTA's time, the three barriers ~20%),
-// faster on short row lists at n = 32768, where the two-pass path reads the
-// row count on the host.  The arithmetic (products, FFT passes,
+// SM) or of 4 / 8 CTAs of 512 threads (8192 points, one per SM).  Measured on a
+// B200 against large2_kernel: 1 pair at n = 32768 16 vs 19 us, 51 listed rows of 4096
+// 56 vs 62, but 128 pairs 38 vs 34 and 1024 pairs 258 vs 152 (pass B takes ~45% of a
+// CTA's time, the three barriers ~20%), so short runs at n = 32768 and captured ones
+// (it has no scratch) come here.  The arithmetic (products, FFT passes,
 // twiddles, key order) is that of large_pass_a / large_pass_b, so the outputs
 // equal the two-pass kernels'.  Clusters walk the pairs template-major with a
 // stride of the cluster count, so clusters running at the same time share a

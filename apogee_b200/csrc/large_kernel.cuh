@@ -1,5 +1,5 @@
 // Fused matched filter for transforms larger than one CTA holds
-// (n = 32768 ... 1048576): a two-pass four-step through an L2-sized scratch.
+// (n = 32768 ... 524288): a two-pass four-step through an L2-sized scratch.
 //
 // With n = N1 * N2, f = f1 + N1 f2 and k = N2 k1 + k2 (f1, k1 < N1; f2, k2 < N2):
 //
@@ -15,8 +15,11 @@
 //           correlation series is never written.
 //   finalize  candidate records -> (index, value) outputs and crossing counts.
 //
-// Pairs run in batches whose scratch (batch x n x 8 bytes, <= 64 MiB) stays
-// resident in the 126 MB L2; pairs are ordered template-major so the data rows
+// These per-batch kernels serve mfb_run_large_static, whose fixed scratch of
+// 8 MiB has no room for large2_kernel's ring; plans run that kernel.  What it shares
+// (arguments, pair order, twiddle tables, keys, records) and the forward
+// transform of series blocks are here too.  Pairs run in batches that fit
+// the scratch and are ordered template-major so the data rows
 // of one template share its spectrum in L2.  This is the unshipped "Tier C"
 // two-dispatch four-step of the reference (src/gpu/tierb.slang:1043-1150) and
 // the CPU plan of src/balanced-inl.h:174-386 for n up to 2^20, fused with the

@@ -20,12 +20,13 @@
 #include <cstddef>
 #include "../../include/mfb.h"
 #include "flat_kernel.cuh"
-#include "flat2_kernel.cuh"
+#include "flatw_kernel.cuh"
 #include "series_kernel.cuh"
 #include "hier_kernels.cuh"
 #include "band_kernels.cuh"
 #include "large_kernel.cuh"
 #include "cluster_kernel.cuh"
+#include "packed_passes.cuh"
 #include "large2_kernel.cuh"
 #include "adjoint_kernel.cuh"
 #include "batch_kernel.cuh"
@@ -103,11 +104,12 @@ struct NConst {
   int grid_peaks = 0, grid_gate = 0, grid_fwd = 0;
   int cta = 0, smem = 0, g = 0;
   int grid_rows = 0;
-  // two pairs per thread (flat2_kernel.cuh at n = 4096, the transforms of
-  // large2_kernel.cuh at 128 ... 1024): the tables as (wr, wr, wi, wi) records
+  // n = 128 ... 1024: the tables as (wr, wr, wi, wi) records for two pairs per
+  // thread (the transforms of large2_kernel.cuh)
   float4 *twid2 = nullptr;
-  float4 *twid2w = nullptr;     // flat2w_kernel: pass 2 in its thread order
-  int grid2 = 0, grid2w = 0;    // flat2_kernel, flat2w_kernel
+  // n >= 512: flatw_kernel's tables, in its thread order, and its grid
+  float2 *twidw = nullptr;
+  int gridw = 0, gridw_gate = 0;
 };
 static std::mutex g_const_mu;
 static std::map<std::pair<int, int>, NConst> g_const;
@@ -123,8 +125,9 @@ static int make_const(int device, NConst &c) {
   c.g = Geo::G;
   CUDA_TRY(cudaFuncSetAttribute(flat_kernel<N, MODE_PEAKS>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, Geo::SMEM));
-  CUDA_TRY(cudaFuncSetAttribute(flat_kernel<N, MODE_GATE>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, Geo::SMEM));
+  if constexpr (N < 512)
+    CUDA_TRY(cudaFuncSetAttribute(flat_kernel<N, MODE_GATE>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, Geo::SMEM));
   CUDA_TRY(cudaFuncSetAttribute(series_forward_kernel<N>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, Geo::SMEM));
   CUDA_TRY(cudaFuncSetAttribute(rows_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -133,44 +136,48 @@ static int make_const(int device, NConst &c) {
   CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, flat_kernel<N, MODE_PEAKS>,
                                                          Geo::CTA, Geo::SMEM));
-  CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, flat_kernel<N, MODE_GATE>,
-                                                         Geo::CTA, Geo::SMEM));
+  if constexpr (N < 512)
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, flat_kernel<N, MODE_GATE>,
+                                                           Geo::CTA, Geo::SMEM));
+  else
+    b2 = 1;   // flatw_kernel has the gate
   CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b3, series_forward_kernel<N>,
                                                          Geo::CTA, Geo::SMEM));
   CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b4, rows_kernel<N>, Geo::CTA,
                                                          Geo::SMEM));
   if (b1 < 1 || b2 < 1 || b3 < 1 || b4 < 1)
     return fail(MFB_ERR_CUDA, "kernel for n=%d cannot be resident on this device", N);
-  if constexpr (N == Flat2Geo::N || (N >= 128 && N <= 1024)) {
-    // the scalar tables' values, duplicated for the two lanes
+  if constexpr (N >= 128 && N <= 1024) {
     std::vector<float4> tw2(tw.size());
     for (size_t i = 0; i < tw.size(); i++) tw2[i] = make_float4(tw[i].x, tw[i].x, tw[i].y, tw[i].y);
     CUDA_TRY(cudaMalloc(&c.twid2, tw2.size() * sizeof(float4)));
     CUDA_TRY(cudaMemcpy(c.twid2, tw2.data(), tw2.size() * sizeof(float4), cudaMemcpyHostToDevice));
   }
-  if constexpr (N == Flat2Geo::N) {
-    CUDA_TRY(cudaFuncSetAttribute(flat2_kernel<MODE_PEAKS>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, Flat2Geo::SMEM));
-    int b5 = 0;
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b5, flat2_kernel<MODE_PEAKS>,
-                                                           Flat2Geo::T, Flat2Geo::SMEM));
-    std::vector<float4> tww(Flat2wGeo::TW);
-    for (int i = 0; i < 240; i++) tww[i] = make_float4(tw[i].x, tw[i].x, tw[i].y, tw[i].y);
-    for (int q = 0; q < 15; q++)
-      for (int t = 0; t < 256; t++) {   // thread K1 + 16 K0 takes entry K0 + 16 K1
-        const float2 w = tw[240 + q * 256 + (t >> 4) + 16 * (t & 15)];
-        tww[240 + q * 256 + t] = make_float4(w.x, w.x, w.y, w.y);
+  if constexpr (N >= 512) {
+    using W = FlatWGeo<N>;
+    std::vector<float2> t(W::TW);
+    for (int i = 0; i < 15 * W::R; i++) t[i] = tw[i];
+    for (int q = 0; q < 15; q++) {
+      if (W::PASSES == 4)
+        for (int K0 = 0; K0 < W::R; K0++)
+          for (int K1 = 0; K1 < 16; K1++)
+            t[W::OFF2 + q * 16 * W::R + 16 * K0 + K1] = tw[twiddle_offset<N>(2) + q * 16 * W::R + K0 + W::R * K1];
+      for (int i = 0; i < W::T; i++) {
+        const int k = W::PASSES == 3 ? (i >> 4) + W::R * (i & 15)
+                                     : (i >> 8) + W::R * (((i >> 4) & 15) + 16 * (i & 15));
+        t[W::OFF3 + q * W::T + i] = tw[twiddle_offset<N>(W::PASSES - 1) + q * W::T + k];
       }
-    CUDA_TRY(cudaMalloc(&c.twid2w, tww.size() * sizeof(float4)));
-    CUDA_TRY(cudaMemcpy(c.twid2w, tww.data(), tww.size() * sizeof(float4), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaFuncSetAttribute(flat2w_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  Flat2wGeo::SMEM));
-    int b6 = 0;
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b6, flat2w_kernel, Flat2wGeo::T,
-                                                           Flat2wGeo::SMEM));
-    if (b5 < 1 || b6 < 1) return fail(MFB_ERR_CUDA, "packed kernel for n=%d cannot be resident", N);
-    c.grid2 = b5 * sms;
-    c.grid2w = b6 * sms;
+    }
+    CUDA_TRY(cudaMalloc(&c.twidw, t.size() * sizeof(float2)));
+    CUDA_TRY(cudaMemcpy(c.twidw, t.data(), t.size() * sizeof(float2), cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaFuncSetAttribute(flatw_kernel<N, MODE_PEAKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, W::SMEM));
+    CUDA_TRY(cudaFuncSetAttribute(flatw_kernel<N, MODE_GATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, W::SMEM));
+    int b5 = 0, b6 = 0;
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b5, flatw_kernel<N, MODE_PEAKS>, W::CTA, W::SMEM));
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b6, flatw_kernel<N, MODE_GATE>, W::CTA, W::SMEM));
+    if (b5 < 1 || b6 < 1) return fail(MFB_ERR_CUDA, "block-bins kernel for n=%d cannot be resident", N);
+    c.gridw = b5 * sms;
+    c.gridw_gate = b6 * sms;
   }
   c.grid_rows = b4 * sms;
   c.grid_peaks = b1 * sms;
@@ -203,11 +210,31 @@ static int get_const(int device, int n, NConst **out) {
   return MFB_OK;
 }
 
+// flatw_kernel covers n >= 512 with window and bins in whole blocks of n/16 lags
+// (dense or listed), and every gate pass at those lengths; it gives the same bits
+// as flat_kernel / rows_kernel.
+static bool flatw_applies(int n, const NConst &c, const FlatArgs &a) {
+  const int block = n / 16;
+  return c.twidw && a.ws % block == 0 && a.we % block == 0 && a.binsize % block == 0;
+}
+
 template <int MODE>
-static cudaError_t launch_flat(int n, const NConst &c, const FlatArgs &a, cudaStream_t s) {
-  const int grid = MODE == MODE_PEAKS ? c.grid_peaks : c.grid_gate;
+static cudaError_t launch_flatw(int n, const NConst &c, FlatArgs a, cudaStream_t s) {
+  a.twid = c.twidw;
+  const int grid = MODE == MODE_PEAKS ? c.gridw : c.gridw_gate;
   switch (n) {
-#define MFB_CASE(NN) case NN: flat_kernel<NN, MODE><<<grid, c.cta, c.smem, s>>>(a); break;
+#define MFB_CASE(NN) \
+  case NN: flatw_kernel<NN, MODE><<<grid, FlatWGeo<NN>::CTA, FlatWGeo<NN>::SMEM, s>>>(a); break;
+    MFB_CASE(512) MFB_CASE(1024) MFB_CASE(2048) MFB_CASE(4096) MFB_CASE(8192) MFB_CASE(16384)
+#undef MFB_CASE
+    default: return cudaErrorInvalidValue;
+  }
+  return cudaGetLastError();
+}
+
+static cudaError_t launch_peaks(int n, const NConst &c, const FlatArgs &a, cudaStream_t s) {
+  switch (n) {
+#define MFB_CASE(NN) case NN: flat_kernel<NN, MODE_PEAKS><<<c.grid_peaks, c.cta, c.smem, s>>>(a); break;
     MFB_CASE(64) MFB_CASE(128) MFB_CASE(256) MFB_CASE(512) MFB_CASE(1024)
     MFB_CASE(2048) MFB_CASE(4096) MFB_CASE(8192) MFB_CASE(16384)
 #undef MFB_CASE
@@ -216,25 +243,13 @@ static cudaError_t launch_flat(int n, const NConst &c, const FlatArgs &a, cudaSt
   return cudaGetLastError();
 }
 
-// The two-pairs-per-thread kernel covers n = 4096 peaks over the whole lag
-// window with bins a multiple of 32 lags and at most KEYCAP bins, dense or
-// listed; it gives the same bits as flat_kernel / rows_kernel.
-static bool flat2w_applies(int n, const FlatArgs &a) {
-  return n == Flat2wGeo::N && (a.ws & 255) == 0 && (a.we & 255) == 0 && (a.binsize & 255) == 0;
-}
-static bool flat2_applies(int n, const NConst &c, const FlatArgs &a) {
-  return flat2w_applies(n, a) || (n == Flat2Geo::N && c.twid2 && a.ws == 0 && a.we == n &&
-                                  (a.binsize & 31) == 0 && a.nb <= KEYCAP);
-}
-
-static cudaError_t launch_flat2(const NConst &c, FlatArgs a, cudaStream_t s) {
-  if (flat2w_applies(Flat2wGeo::N, a)) {
-    a.twid = reinterpret_cast<const float2 *>(c.twid2w);
-    flat2w_kernel<<<c.grid2w, Flat2wGeo::T, Flat2wGeo::SMEM, s>>>(a);
-    return cudaGetLastError();
+static cudaError_t launch_gate(int n, const NConst &c, const FlatArgs &a, cudaStream_t s) {
+  switch (n) {
+#define MFB_CASE(NN) case NN: flat_kernel<NN, MODE_GATE><<<c.grid_gate, c.cta, c.smem, s>>>(a); break;
+    MFB_CASE(64) MFB_CASE(128) MFB_CASE(256)
+#undef MFB_CASE
+    default: return launch_flatw<MODE_GATE>(n, c, a, s);
   }
-  a.twid = reinterpret_cast<const float2 *>(c.twid2);
-  flat2_kernel<MODE_PEAKS><<<c.grid2, Flat2Geo::T, Flat2Geo::SMEM, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -575,7 +590,7 @@ struct mfb_plan {
   LargeConst *lc = nullptr;
   LargeScratch ls;
   std::vector<LargeScratch> ls_old;
-  int packed = 1;           // use flat2_kernel where it applies (mfb_set_packed)
+  int packed = 1;           // use flatw_kernel where it applies (mfb_set_packed)
   int cluster = -1;         // mfb_set_cluster's choice; -1: cluster_mode's rule
 };
 
@@ -849,9 +864,10 @@ static int run_large(mfb_plan *p, int d0, int nd, int t0, int nt, const int32_t 
 }
 
 // The dense block of `a` at n <= 16384.
-static cudaError_t launch_peaks(const mfb_plan *p, const FlatArgs &a) {
-  if (p->packed && flat2_applies((int)p->n, *p->c, a)) return launch_flat2(*p->c, a, p->stream);
-  return launch_flat<MODE_PEAKS>((int)p->n, *p->c, a, p->stream);
+static cudaError_t launch_dense(const mfb_plan *p, const FlatArgs &a) {
+  if (p->packed && flatw_applies((int)p->n, *p->c, a))
+    return launch_flatw<MODE_PEAKS>((int)p->n, *p->c, a, p->stream);
+  return launch_peaks((int)p->n, *p->c, a, p->stream);
 }
 
 static int run_impl(mfb_plan *p, int d0, int nd, int t0, int nt, size_t binsize,
@@ -873,7 +889,7 @@ static int run_impl(mfb_plan *p, int d0, int nd, int t0, int nt, size_t binsize,
   if (is_large(p->n))
     return run_large(p, d0, nd, t0, nt, nullptr, nullptr, binsize, threshold, start, end, nb, idx, val,
                      counts, rs);
-  CUDA_TRY(launch_peaks(p, a));
+  CUDA_TRY(launch_dense(p, a));
   return MFB_OK;
 }
 
@@ -931,12 +947,12 @@ static int run_rows_impl(mfb_plan *p, int d0, int nd, int t0, int nt, const int3
     return run_large(p, d0, nd, t0, nt, rows, nrows, binsize, threshold, start, end, nb, idx, val,
                      counts, rs);
   a.trig_total = trig_total;
-  if (p->packed && flat2_applies((int)p->n, *p->c, a)) {
+  if (p->packed && flatw_applies((int)p->n, *p->c, a)) {
     if (host_rec && rs == 2) {
       a.host_rec = host_rec;
       if (host_written) *host_written = true;
     }
-    CUDA_TRY(launch_flat2(*p->c, a, p->stream));
+    CUDA_TRY(launch_flatw<MODE_PEAKS>((int)p->n, *p->c, a, p->stream));
   } else {
     CUDA_TRY(launch_rows((int)p->n, *p->c, a, p->stream));
   }
@@ -1070,7 +1086,7 @@ extern "C" int mfb_run_series(mfb_plan *p, const void *series, size_t nseries,
     a.out_val = (float2 *)val + (size_t)b0 * nt * nb0;
     a.rs = 1;
     a.out_cnt = counts ? counts + (size_t)b0 * nt : nullptr;
-    CUDA_TRY(launch_peaks(p, a));
+    CUDA_TRY(launch_dense(p, a));
     b0 += g;
   }
   return MFB_OK;
@@ -1497,7 +1513,7 @@ static int hier_run_impl(mfb_hplan *h, int d0, int nd, int t0, int nt, size_t bi
     a.fire_list = h->fire_list;
     a.fire_count = h->fire_count;
     a.full_nb = (int)nb;
-    CUDA_TRY(launch_flat<MODE_GATE>((int)h->m, *h->cc, a, s));
+    CUDA_TRY(launch_gate((int)h->m, *h->cc, a, s));
   } else if (h->m == (size_t)BAND_BIG) {
     r = band_big_coarse(h, d0, nd, t0, nt, cs, ce, idx, val, rs, nb, nullptr, s);
     if (r) return r;
@@ -1730,7 +1746,7 @@ extern "C" int mfb_hier_coarse_values(mfb_hplan *h, int d0, int nd, int t0, int 
     a.ws = cs; a.we = ce; a.binsize = ce - cs; a.nb = 1;
     a.t2 = 0.f;
     a.coarse_out = out;
-    CUDA_TRY(launch_flat<MODE_GATE>((int)h->m, *h->cc, a, s));
+    CUDA_TRY(launch_gate((int)h->m, *h->cc, a, s));
     return MFB_OK;
   }
   if (h->m == (size_t)BAND_BIG)
@@ -2023,6 +2039,10 @@ static int get_adj_tables(int device, int n, AdjTables **out) {
   CUDA_TRY(cudaMalloc(&t.lo, lo.size() * sizeof(float2)));
   CUDA_TRY(cudaMemcpy(t.hi, hi.data(), hi.size() * sizeof(float2), cudaMemcpyHostToDevice));
   CUDA_TRY(cudaMemcpy(t.lo, lo.data(), lo.size() * sizeof(float2), cudaMemcpyHostToDevice));
+  // adjoint_kernel's largest shape (88 KB bounds them all: 40 KB of staged twiddles,
+  // 12 of entries, 16 of roots and 16 of list ends)
+  CUDA_TRY(cudaFuncSetAttribute(adjoint_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 88 << 10));
+  CUDA_TRY(cudaFuncSetAttribute(adjoint_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 88 << 10));
   *out = &(g_adj[{device, n}] = t);
   return MFB_OK;
 }
@@ -2070,9 +2090,7 @@ static int adjoint_side(bool grad_data, int n, int nd, int nt, int nb, const flo
   if (a.accumulate) CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)a.own * n * sizeof(float2), st));
   const size_t smem = adjoint_smem(a.fblk, lists * a.slots, tw.hi_count + (1 << tw.lo_bits));
   const dim3 grid((unsigned)tiles, (unsigned)split);
-  // one limit for every shape, so that callers on several threads set the same value
   auto kernel = grad_data ? adjoint_kernel<true> : adjoint_kernel<false>;
-  CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 88 << 10));
   kernel<<<grid, ADJ_THREADS, smem, st>>>(a);
   CUDA_TRY(cudaGetLastError());
   return MFB_OK;

@@ -78,13 +78,13 @@ int mfb_run(mfb_plan *p, int d0, int nd, int t0, int nt, size_t binsize, float t
    device). records: DEVICE [nd*nt*nb] x 16 bytes. */
 int mfb_run_records(mfb_plan *p, int d0, int nd, int t0, int nt, size_t binsize, float threshold,
                     size_t start, size_t end, void *records, int32_t *counts);
-/* Kernel choice for n = 4096 (no counterpart in the reference, whose CPU
-   engine picks its own code path per shape): on (the default), runs whose
-   lag window is [0, n) with bins a multiple of 32 lags and at most 64 bins
-   use the kernel that carries two pairs per thread in packed FP32x2
-   arithmetic; off, they use the one-pair-per-thread kernel.  Both compute
-   the same operations in the same order and give bit-identical results;
-   the switch lets a caller compare or time the two. */
+/* Kernel choice for n = 512 ... 16384 (no counterpart in the reference, whose CPU
+   engine picks its own code path per shape): on (the default), runs whose lag
+   window and bins are whole blocks of n/16 lags use the kernel whose exchanges stay
+   within half-warps where they can (flatw_kernel); off, they use the general
+   kernel, as all other runs do.  Both compute the same operations in the same order
+   and give bit-identical results; the switch lets a caller compare or time the
+   two.  (The name is that of the packed two-pair kernel which once stood here.) */
 int mfb_set_packed(mfb_plan *p, int on);
 /* Kernel choice for n = 32768 and 65536 (no counterpart in the reference,
    whose CPU engine always runs its four-step plan through memory): mode 0

@@ -357,35 +357,83 @@ def test_packed_kernel_matches_one_pair_kernel_and_oracle(nd, nt, binsize, thres
     assert (got_i[untouched] == -7).all()
 
 
-@pytest.mark.parametrize("nd, nt, binsize, win", [
-    (1, 1, 4096, None),                 # one pair: the second lane is dead
-    (3, 5, 256, None),                  # odd pair count, data rows change inside an item
-    (2, 301, 256, (1024, 3072)),        # a window of whole blocks (block-wise series filtering)
-    (5, 7, 768, (256, 4096)),           # bins of three blocks
-    (1, 2, 2048, (0, 256)),             # one block
+@pytest.mark.parametrize("n", [512, 1024, 2048, 4096, 8192, 16384])
+@pytest.mark.parametrize("nd, nt, blocks, win", [
+    (1, 1, 16, None),            # one pair: most pair slots have none
+    (3, 5, 1, None),             # 15 pairs, data rows change between them
+    (2, 301, 1, (4, 12)),        # a window of whole blocks (block-wise series filtering)
+    (5, 7, 3, (1, 16)),          # bins of three blocks
+    (1, 2, 8, (0, 1)),           # one block
 ])
-@pytest.mark.parametrize("thr", [0.0, 350.0, 1e6])
-def test_block_bins_kernel_is_bit_identical(nd, nt, binsize, win, thr):
-    """n = 4096 with bins and window in multiples of 256 lags (the kernel whose
-    second exchange stays within half-warps) against the one-pair kernel:
-    same bits; and against the FP64 oracle.  Thresholds: every bin reports,
-    some do (z has deviation 128 per component), none does."""
+def test_block_bins_kernel_is_bit_identical(n, nd, nt, blocks, win):
+    """Bins and window in whole blocks of n/16 lags (the kernel whose exchanges
+    stay within half-warps where they can) against flat_kernel: same bits,
+    dense and listed; and against the FP64 oracle.  Thresholds: every bin
+    reports, some do (z has deviation 2 sqrt(n) per component), none does."""
+    import torch
     mf = _mf()
     from apogee_b200 import _lib
-    rng = np.random.default_rng(nd * 1000 + nt)
-    D, H = noise(rng, (nd, 4096)), noise(rng, (nt, 4096))
-    f = mf.MatchedFilter(4096, nd, nt)
+    L = _lib.lib()
+    rng = np.random.default_rng(nd * 1000 + nt + n)
+    D, H = noise(rng, (nd, n)), noise(rng, (nt, n))
+    block = n // 16
+    binsize = blocks * block
+    win = None if win is None else (win[0] * block, win[1] * block)
+    lo, hi = win or (0, n)
+    f = mf.MatchedFilter(n, nd, nt)
     f.set_data(D)
     f.set_templates(H)
-    out, cnt = f.run(binsize=binsize, threshold=thr, window=win, counts=True)
-    out, cnt = out.copy(), cnt.copy()
-    _lib.check(_lib.lib().mfb_set_packed(f._plan, 0))
-    ref, rcnt = f.run(binsize=binsize, threshold=thr, window=win, counts=True)
-    np.testing.assert_array_equal(out["index"], ref["index"])
-    np.testing.assert_array_equal(out["value"], ref["value"])
-    np.testing.assert_array_equal(cnt, rcnt)
     z = oracle.correlate(D, H[:8])
-    assert not parity.compare(out["index"][:, :8], out["value"][:, :8], z, binsize, thr, win)
+    for thr in (0.0, 5.5 * np.sqrt(n), 1e3 * n):
+        _lib.check(L.mfb_set_packed(f._plan, 1))
+        out, cnt = f.run(binsize=binsize, threshold=thr, window=win, counts=True)
+        out, cnt = out.copy(), cnt.copy()
+        assert not parity.compare(out["index"][:, :8], out["value"][:, :8], z, binsize, thr, win)
+        rows = torch.from_numpy(rng.permutation(nd * nt)[: nd * nt // 2 + 1].astype(np.int32)).cuda()
+        count = torch.tensor([rows.numel()], dtype=torch.int32, device="cuda")
+        nb = out.shape[2]
+        idx = torch.full((nd * nt, nb), -7, dtype=torch.int64, device="cuda")
+        val = torch.zeros(nd * nt, nb, dtype=torch.complex64, device="cuda")
+        _lib.check(L.mfb_run_rows(f._plan, 0, nd, 0, nt, rows.data_ptr(), count.data_ptr(), rows.numel(),
+                                  binsize, thr, lo, hi, idx.data_ptr(), val.data_ptr(), None))
+        r = rows.long().cpu().numpy()
+        np.testing.assert_array_equal(idx.cpu().numpy()[r], out["index"].reshape(-1, nb)[r])
+        np.testing.assert_array_equal(val.cpu().numpy()[r], out["value"].reshape(-1, nb)[r])
+        _lib.check(L.mfb_set_packed(f._plan, 0))
+        ref, rcnt = f.run(binsize=binsize, threshold=thr, window=win, counts=True)
+        np.testing.assert_array_equal(out["index"], ref["index"])
+        np.testing.assert_array_equal(out["value"], ref["value"])
+        np.testing.assert_array_equal(cnt, rcnt)
+
+
+@pytest.mark.parametrize("n, band", [(2048, 512), (4096, 1024), (8192, 2048), (8192, 4096), (16384, 8192),
+                                     (32768, 16384), (1024, 256)])
+def test_fp32_coarse_values_vs_fp64(n, band):
+    """The FP32 gate pass at every band length, whole and partial windows, odd pair
+    counts: coarse maxima against FP64.  Bound: the transform's FP32 error scales
+    with its output's deviation (log2(band) stages of 2^-23 against a root mean
+    square over the band), and keys drop five mantissa bits of |z|^2 (2^-19 of |z|)."""
+    mf = _mf()
+    rng = np.random.default_rng(band)
+    nd, nt = 3, 7
+    D, H = noise(rng, (nd, n)), noise(rng, (nt, n))
+    P = (np.abs(H) ** 2).mean(0).astype(np.float32)
+    hf = mf.HierarchicalFilter(n, nd, nt, band=band, coarse="fp32")
+    hf.set_reference(P)
+    hf.set_coarse_threshold(1.0)
+    hf.set_data(D)
+    hf.set_templates(H)
+    f = float(np.float32(P[:band].astype(np.float64).sum() / P.astype(np.float64).sum()))
+    R = n // band
+    for window in (None, (n // 3, n // 2), (0, R)):
+        lo, hi = (0, n) if window is None else window
+        cs, ce = max(0, lo // R - 1), min(band, -(-hi // R))
+        for d in range(nd):
+            z = np.fft.ifft(D[d, :band].astype(np.complex128) * np.conj(H[:, :band]), axis=1) * band / np.sqrt(f)
+            want = np.abs(z[:, cs:ce]).max(1)
+            got = hf.coarse_values(window=window)[d]
+            rms = np.sqrt((np.abs(z) ** 2).mean(1))
+            assert (np.abs(got - want) <= 2.0 ** -19 * want + np.log2(band) * 2.0 ** -23 * 4 * rms).all()
 
 
 @pytest.mark.parametrize("n", [64, 256, 1024, 2048, 8192, 16384])
