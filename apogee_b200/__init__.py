@@ -452,18 +452,33 @@ class MatchedFilter:
                                hi.ctypes.data, nblk, t0, nt, binsize, threshold,
                                idx_d.data_ptr(), val_d.data_ptr())
         _lib.check(rc, "run_series failed")
-        idx = idx_d.cpu().numpy().reshape(nblk, nt, nb)
-        val = val_d.cpu().numpy().reshape(nblk, nt, nb)
-        stream.synchronize()
-        if layout.order is not None:
-            ri = np.empty_like(idx)
-            rv = np.empty_like(val)
-            ri[layout.order], rv[layout.order] = idx, val
-            idx, val = ri, rv
         if raw:
+            idx = idx_d.cpu().numpy().reshape(nblk, nt, nb)
+            val = val_d.cpu().numpy().reshape(nblk, nt, nb)
+            stream.synchronize()
+            if layout.order is not None:
+                ri = np.empty_like(idx)
+                rv = np.empty_like(val)
+                ri[layout.order], rv[layout.order] = idx, val
+                idx, val = ri, rv
             return idx, val
-        out = np.empty(idx.shape, PEAK_DTYPE)
-        out["index"], out["value"] = idx, val
+        # PEAK_DTYPE records put together on the device, one copy into pinned memory, one
+        # into the caller's array (two pageable copies and a strided assignment of each
+        # field: 657 us for a whole run of 64 blocks x 128 templates at n = 4096, this 438)
+        words = nblk * nt * nb
+        rec = self._buffer("srec", (words, 2), torch.int64)
+        rec[:, 0] = idx_d
+        rec[:, 1] = val_d.view(torch.int64)
+        rec_h = self._buffer("srec_h", (words, 2), torch.int64, pinned=True)
+        rec_h.copy_(rec, non_blocking=True)
+        stream.synchronize()
+        out = np.empty((nblk, nt, nb), PEAK_DTYPE)
+        flat = out.view(np.int64).reshape(nblk, nt * nb * 2)
+        src = rec_h.numpy().reshape(nblk, nt * nb * 2)
+        if layout.order is None:
+            flat[...] = src
+        else:
+            flat[layout.order] = src
         return out
 
     def _series_call(self, *args):
