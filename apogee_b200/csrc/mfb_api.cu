@@ -1627,6 +1627,14 @@ static uint32_t float_bits(float x) {
   return u;
 }
 
+// Launches the captured run, ordered with the plan's other runs as a direct run is.
+static cudaError_t launch_hier_graph(mfb_hplan *h, cudaGraphExec_t x) {
+  const mfb_plan *p = h->full;
+  cudaError_t e = p->ls.ring ? scratch_begin(p) : cudaSuccess;
+  if (e == cudaSuccess) e = cudaGraphLaunch(x, p->stream);
+  return e == cudaSuccess && p->ls.ring ? scratch_end(p) : e;
+}
+
 extern "C" int mfb_hier_run_host(mfb_hplan *h, int d0, int nd, int t0, int nt, size_t binsize,
                                  float threshold, size_t start, size_t end, const void *data,
                                  void *records, void *table, int64_t *info) {
@@ -1664,6 +1672,8 @@ extern "C" int mfb_hier_run_host(mfb_hplan *h, int d0, int nd, int t0, int nt, s
       graphable = false;
     }
   }
+  const LargeScratch &ls = h->full->ls;
+  if (ls.ring && *(volatile int *)ls.err) graphable = false;   // the direct run reports it
   mfb_hplan::RunKey key;
   memset(&key, 0, sizeof key);
   key.d0 = d0; key.nd = nd; key.t0 = t0; key.nt = nt;
@@ -1674,7 +1684,7 @@ extern "C" int mfb_hier_run_host(mfb_hplan *h, int d0, int nd, int t0, int nt, s
   key.binsize = binsize; key.start = start; key.end = end;
   key.data = data; key.records = records; key.table = dtab; key.info = dinfo;
   if (graphable && h->graph && memcmp(&key, &h->graph_key, sizeof key) == 0) {
-    CUDA_TRY(cudaGraphLaunch(h->graph, h->full->stream));
+    CUDA_TRY(launch_hier_graph(h, h->graph));
     h->pairs += (long long)nd * nt;
     return MFB_OK;
   }
@@ -1704,7 +1714,7 @@ extern "C" int mfb_hier_run_host(mfb_hplan *h, int d0, int nd, int t0, int nt, s
       if (h->graph) cudaGraphExecDestroy(h->graph);
       h->graph = x;
       h->graph_key = key;
-      CUDA_TRY(cudaGraphLaunch(x, user));
+      CUDA_TRY(launch_hier_graph(h, x));
       h->last_valid = true;
       return MFB_OK;   // the captured call already counted its pairs
     }
