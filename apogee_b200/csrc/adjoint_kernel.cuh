@@ -21,12 +21,17 @@
 // min(n/16, 256) values of f0 for 256/F own rows.  Entries are staged in
 // rounds: a warp sorts one (own, other) row's entries by bucket, then the CTA
 // tabulates W^(l k) for the 32 lanes l and conj(g) W^((F x + 32 a) k) for its
-// groups a of 32 lanes (W^m = hi[m >> lo_bits] * lo[m & mask], FP64-built halves),
+// groups a of 32 lanes (W^m = hi[m >> lo_bits] (1 + lo[m & mask]), FP64-built
+// halves; the second is a root less one, so it adds no rounding of its own),
 // so the inner loop is two shared-memory reads (the second a broadcast) and
 // four FMAs per entry.  Rows without a peak are
-// skipped.  The lags are the forward pass's argmax lags; nothing of the
+// skipped.  Where the summed rows split over many CTAs, clusters of ADJ_CLUSTER
+// of them add up their sums through distributed shared memory first: 291 atomic
+// additions in a row to one output (3 x 872 pairs at n = 2048) doubled the
+// gradient's rounding.  The lags are the forward pass's argmax lags; nothing of the
 // correlation series is stored.
 #pragma once
+#include <cooperative_groups.h>
 #include <cstdint>
 #include "fft_radix.cuh"
 
@@ -37,7 +42,8 @@ constexpr int ADJ_R = 16;              // frequencies per thread = buckets
 constexpr int ADJ_CHUNK = 32;          // entries of one (own, other) row sorted at a time
 constexpr int ADJ_TAB = 40960;         // bytes of staged twiddles per round
 constexpr int ADJ_ITEMS = 1024;        // (own, other, chunk) lists per round
-
+constexpr int ADJ_CLUSTER = 8;         // CTAs of one tile that add up before the atomics
+static_assert(ADJ_R * ADJ_THREADS * sizeof(float2) <= ADJ_TAB, "a CTA's sums fit the staged twiddles");
 
 struct AdjArgs {
   const float2 *src;      // other rows [other][n]: templates (grad_D) or data (grad_H)
@@ -55,6 +61,7 @@ struct AdjArgs {
   int other_per_split;    // other rows per blockIdx.y
   int accumulate;         // 1: atomicAdd into a zeroed out (other split over blockIdx.y)
   int lsh, ash;           // log2 of the lane and group values per entry
+  int clusters;           // 1: blockIdx.y in clusters of ADJ_CLUSTER
   const float2 *tw_hi, *tw_lo;
   int lo_bits, hi_count;
 };
@@ -98,7 +105,7 @@ __global__ void __launch_bounds__(ADJ_THREADS, 2) adjoint_kernel(const AdjArgs a
   auto root = [&](unsigned m) {   // W^(m mod n)
     m &= mask_n;
     const float2 h = s_hi[m >> a.lo_bits], w = s_lo[m & lo_mask];
-    return cmul(cf{h.x, h.y}, cf{w.x, w.y});
+    return cf{fmaf(h.x, w.x, fmaf(-h.y, w.y, h.x)), fmaf(h.x, w.y, fmaf(h.y, w.x, h.y))};
   };
 
   cf acc[ADJ_R];
@@ -182,6 +189,7 @@ __global__ void __launch_bounds__(ADJ_THREADS, 2) adjoint_kernel(const AdjArgs a
 #pragma unroll
           for (int q = 0; q < ADJ_R; q++) {
             const int end = (int)((ew[q >> 2] >> (8 * (q & 3))) & 255u);
+#pragma unroll 1   // about one entry a bucket; unrolled: 128 us instead of 88 at n = 16384, 8 x 256
             for (; e < end; e++, p1 += L, p2 += A) {
               const float2 w = *p1, h = *p2;
               S[q].x = fmaf(w.x, h.x, fmaf(-w.y, h.y, S[q].x));
@@ -207,8 +215,34 @@ __global__ void __launch_bounds__(ADJ_THREADS, 2) adjoint_kernel(const AdjArgs a
       }
     }
   }
-  if (!live) return;
   float2 *op = a.out + (long long)own_row * a.n + f0;
+  if (a.clusters) {       // each CTA adds up ADJ_R / ADJ_CLUSTER of the cluster's 16 frequencies
+    const auto cluster = cooperative_groups::this_cluster();
+    __syncthreads();      // the last round's readers are done
+    float2 *sums = lane_tw;
+#pragma unroll
+    for (int j = 0; j < ADJ_R; j++) sums[j * ADJ_THREADS + tid] = make_float2(acc[j].x, acc[j].y);
+    cluster.sync();
+#pragma unroll
+    for (int q = 0; q < ADJ_R / ADJ_CLUSTER; q++) {
+      const int j = (int)cluster.block_rank() * (ADJ_R / ADJ_CLUSTER) + q;
+      float2 v[ADJ_CLUSTER];
+#pragma unroll
+      for (int c = 0; c < ADJ_CLUSTER; c++) v[c] = cluster.map_shared_rank(sums, c)[j * ADJ_THREADS + tid];
+#pragma unroll
+      for (int h = 1; h < ADJ_CLUSTER; h *= 2) {
+#pragma unroll
+        for (int c = 0; c < ADJ_CLUSTER; c += 2 * h) {
+          v[c].x += v[c + h].x;
+          v[c].y += v[c + h].y;
+        }
+      }
+      if (live) atomicAdd(op + j * sixteenth, v[0]);
+    }
+    cluster.sync();       // the other CTAs may still read this one's sums
+    return;
+  }
+  if (!live) return;
 #pragma unroll
   for (int j = 0; j < ADJ_R; j++) {
     const float2 v = make_float2(acc[j].x, acc[j].y);

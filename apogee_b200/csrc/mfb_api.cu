@@ -1574,7 +1574,7 @@ static int hier_run_impl(mfb_hplan *h, int d0, int nd, int t0, int nt, size_t bi
   }
   if (join) CUDA_TRY(cudaStreamWaitEvent(s, h->ev_join, 0));
   // Refine the survivors with the full filter; no host decision in between.
-  // With the host table as it was left by this plan, the packed kernel also
+  // With the host table as it was left by this plan, flatw_kernel also
   // stores the refined rows into it.
   bool counted = false, host_written = false;
   r = run_rows_impl(p, d0, nd, t0, nt, h->fire_list, h->fire_count, nd * nt, binsize, threshold,
@@ -2044,7 +2044,10 @@ static int get_adj_tables(int device, int n, AdjTables **out) {
   t.hi_count = n >> t.lo_bits;
   std::vector<float2> hi(t.hi_count), lo((size_t)1 << t.lo_bits);
   for (int i = 0; i < t.hi_count; i++) hi[i] = unit_root((long long)i << t.lo_bits, n);
-  for (size_t i = 0; i < lo.size(); i++) lo[i] = unit_root((long long)i, n);
+  for (size_t i = 0; i < lo.size(); i++) {   // W^i - 1 = 2 i sin(pi i/n) e^(i pi i/n)
+    const double s = sin(M_PI * (double)i / n), c = cos(M_PI * (double)i / n);
+    lo[i] = make_float2((float)(-2.0 * s * s), (float)(2.0 * s * c));
+  }
   CUDA_TRY(cudaMalloc(&t.hi, hi.size() * sizeof(float2)));
   CUDA_TRY(cudaMalloc(&t.lo, lo.size() * sizeof(float2)));
   CUDA_TRY(cudaMemcpy(t.hi, hi.data(), hi.size() * sizeof(float2), cudaMemcpyHostToDevice));
@@ -2066,8 +2069,16 @@ static size_t adjoint_smem(int fblk, int items, int roots) {
 
 // One side of the adjoint: a CTA covers 256 (own row, f0) and all other rows;
 // when that leaves the device less than ADJ_FILL CTAs per SM, the summed rows
-// split over blockIdx.y with atomic accumulation.
+// split over blockIdx.y with atomic accumulation.  A long chain of atomics rounds
+// like a long chain of rows, and worse than a balanced split of both, so with
+// few tiles (up to ADJ_FEW, where the split is wide) clusters of CTAs add up
+// their sums first, in one wave of CTAs that leaves clusters room to be placed
+// (7/8 of two per SM); otherwise a CTA sums two rows or more.  B200, gradient of
+// 3 rows, 3 x 872 pairs at n = 2048: 291 splits without clusters 33 us and a
+// relative error of 3.3e-7, two waves of clusters 42 us and 1.6e-7, this 31.6 us
+// and 1.4e-7.
 constexpr int ADJ_FILL = 4;
+constexpr int ADJ_FEW = 16;
 static int adjoint_side(bool grad_data, int n, int nd, int nt, int nb, const float2 *src,
                         const int64_t *idx, const float2 *gz, float2 *out, const AdjTables &tw,
                         int sms, cudaStream_t st) {
@@ -2093,15 +2104,31 @@ static int adjoint_side(bool grad_data, int n, int nd, int nt, int nb, const flo
   const long long tiles = (long long)a.fx * ((a.own + a.slots - 1) / a.slots);
   const long long target = (long long)ADJ_FILL * sms;
   long long split = 1;
-  if (tiles < target) split = std::min<long long>(a.other, std::max<long long>(1, target / tiles));
+  if (tiles < target) split = std::min<long long>(a.other, target / tiles);
+  a.clusters = tiles <= ADJ_FEW && split > ADJ_CLUSTER;
+  if (a.clusters)
+    split = std::min<long long>(split, 7LL * sms / 4 / tiles / ADJ_CLUSTER * ADJ_CLUSTER);
+  else if (tiles > ADJ_FEW)
+    split = std::min<long long>(split, std::max(1, a.other / 2));
   a.other_per_split = (int)((a.other + split - 1) / split);
   split = (a.other + a.other_per_split - 1) / a.other_per_split;
   a.accumulate = split > 1;
+  if (a.clusters) split = (split + ADJ_CLUSTER - 1) / ADJ_CLUSTER * ADJ_CLUSTER;   // the last may have no rows
   if (a.accumulate) CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)a.own * n * sizeof(float2), st));
-  const size_t smem = adjoint_smem(a.fblk, lists * a.slots, tw.hi_count + (1 << tw.lo_bits));
-  const dim3 grid((unsigned)tiles, (unsigned)split);
-  auto kernel = grad_data ? adjoint_kernel<true> : adjoint_kernel<false>;
-  kernel<<<grid, ADJ_THREADS, smem, st>>>(a);
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof cfg);
+  cfg.gridDim = dim3((unsigned)tiles, (unsigned)split);
+  cfg.blockDim = dim3(ADJ_THREADS);
+  cfg.dynamicSmemBytes = adjoint_smem(a.fblk, lists * a.slots, tw.hi_count + (1 << tw.lo_bits));
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 1;
+  attr.val.clusterDim.y = a.clusters ? ADJ_CLUSTER : 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  CUDA_TRY(cudaLaunchKernelEx(&cfg, grad_data ? adjoint_kernel<true> : adjoint_kernel<false>, a));
   CUDA_TRY(cudaGetLastError());
   return MFB_OK;
 }
