@@ -24,9 +24,14 @@
 // 32 lags of a block lie in one bin: one redux per block, the winner's value to a
 // small stage.
 //
+// A slot takes every slots-th pair: the rows whose pairs have candidates (a loud data
+// row) are then shared by all SMs, and the slots of an SM are on the same data row.
+// With a contiguous range per slot the SMs were active 93% (n = 4096) and 79% (16384) of
+// the slowest one's time.
+//
 // Measured on a B200 (us, 16 warps' packed two-pair kernel or flat_kernel before ->
-// now): 16 x 1024 pairs at n = 4096, threshold 5.5 204 -> 160, threshold 0 212 -> 198,
-// its 1312 listed rows 21 -> 18.7.
+// contiguous ranges -> now): 16 x 1024 pairs at n = 4096, threshold 5.5
+// 204 -> 166 -> 159; 6 x 300 at n = 16384 149 -> 118 -> 100.
 #pragma once
 #include "flat_kernel.cuh"
 
@@ -70,11 +75,8 @@ __global__ void __launch_bounds__(FlatWGeo<N>::CTA, FlatWGeo<N>::MINB) flatw_ker
   const long long total = a.list ? (long long)(*a.list_count) : (long long)a.nd * a.nt;
   if (a.list && a.trig_total && blockIdx.x == 0 && threadIdx.x == 0)
     *a.trig_total += (unsigned long long)total;
-  // contiguous pairs per slot, the same CTA's slots side by side
+  // every slots-th pair (see above)
   const long long slots = (long long)gridDim.x * G, me = (long long)blockIdx.x * G + g;
-  const long long per = total / slots, extra = total % slots;
-  const long long ibeg = me * per + (me < extra ? me : extra);
-  const long long iend = ibeg + per + (me < extra ? 1 : 0);
   const int nb = a.nb;
   const int q0 = a.ws / T, q1 = a.we / T;                       // window and bins in blocks (MODE_PEAKS)
   const int bsq = MODE == MODE_PEAKS ? a.binsize / T : 1;
@@ -84,7 +86,7 @@ __global__ void __launch_bounds__(FlatWGeo<N>::CTA, FlatWGeo<N>::MINB) flatw_ker
   if (t < 2) gslots[t] = 0u;
   sync();
 
-  int prev = 0;
+  int prev = 0, par = 1;
   // Outputs of pair `prev`, whose keys have parity par (keys are cleared for the pair two on).
   auto outputs = [&](int par) {
     if constexpr (MODE == MODE_PEAKS) {
@@ -126,8 +128,8 @@ __global__ void __launch_bounds__(FlatWGeo<N>::CTA, FlatWGeo<N>::MINB) flatw_ker
     }
   };
 
-  for (long long item = ibeg; item < iend; ++item) {
-    const int par = (int)(item & 1);
+  for (long long item = me; item < total; item += slots) {
+    par ^= 1;
     const int row = a.list ? a.list[item] : (int)item;
     const int d = row / a.nt, tt = row - d * a.nt;
     cf v[16];
@@ -154,7 +156,7 @@ __global__ void __launch_bounds__(FlatWGeo<N>::CTA, FlatWGeo<N>::MINB) flatw_ker
                                    : q * Geo::REGION + ((hi >> 4) + R * b) * 273 + (hi & 15) * 17 + lo;
         buf[at] = make_float2(v[b + B0 * q].x, v[b + B0 * q].y);
       }
-    if (item > ibeg) outputs(par ^ 1);
+    if (item != me) outputs(par ^ 1);
     sync();
     if (MODE == MODE_GATE && t == 0) gslots[par ^ 1] = 0u;   // read above; next written a barrier on
     if constexpr (PASSES == 3) {
@@ -244,9 +246,9 @@ __global__ void __launch_bounds__(FlatWGeo<N>::CTA, FlatWGeo<N>::MINB) flatw_ker
     }
     prev = row;
   }
-  if (ibeg < iend) {
+  if (me < total) {
     sync();
-    outputs((int)((iend - 1) & 1));
+    outputs(par);
   }
 }
 
