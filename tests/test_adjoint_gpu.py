@@ -207,9 +207,10 @@ def _adjoint_direct(n, nd, nt, nb, seed, peaks):
     (4096, 1, 1, 1, 1.0),       # one row, one entry
     (4096, 5, 200, 16, 0.05),   # rows without a peak among the summed ones
     (8192, 2, 3, 300, 1.0),     # a row's lists in several rounds
-    (1024, 2, 64, 4, 1.0),      # 32 splits: atomics alone
-    (1024, 2, 66, 4, 1.0),      # 33: clusters of eight, seven of them without rows
-    (2048, 3, 872, 4, 1.0),     # 291 splits
+    (1024, 2, 8, 4, 1.0),       # 8 splits: atomics alone
+    (1024, 2, 9, 4, 1.0),       # 9: clusters of eight, seven blocks of them without rows
+    (2048, 3, 872, 4, 1.0),     # as many clusters as fit a wave
+    (4096, 17, 5, 4, 1.0),      # one tile too many for clusters
     (16384, 3, 40, 16, 0.0),    # no peak at all
     (1 << 20, 1, 2, 3, 1.0),    # the longest transform
 ])
