@@ -2028,7 +2028,8 @@ extern "C" int mfb_run_large_static(int device, size_t n, const void *data, int 
 // W_n^m twiddles for the adjoint and the batched four-step: hi[m >> lo_bits] * lo[m & mask],
 // built once per (device, n) from FP64 roots.
 struct AdjTables {
-  float2 *hi = nullptr, *lo = nullptr;
+  float2 *hi = nullptr, *lo = nullptr;   // roots (also the batched launch's)
+  float2 *lo_less_one = nullptr;         // lo - 1, the adjoint kernel's
   int lo_bits = 0, hi_count = 0;
 };
 static std::map<std::pair<int, int>, AdjTables> g_adj;
@@ -2044,14 +2045,20 @@ static int get_adj_tables(int device, int n, AdjTables **out) {
   t.hi_count = n >> t.lo_bits;
   std::vector<float2> hi(t.hi_count), lo((size_t)1 << t.lo_bits);
   for (int i = 0; i < t.hi_count; i++) hi[i] = unit_root((long long)i << t.lo_bits, n);
-  for (size_t i = 0; i < lo.size(); i++) {   // W^i - 1 = 2 i sin(pi i/n) e^(i pi i/n)
+  std::vector<float2> less(lo.size());
+  for (size_t i = 0; i < lo.size(); i++) {
+    lo[i] = unit_root((long long)i, n);
+    // W^i - 1 = 2 i sin(pi i/n) e^(i pi i/n)
     const double s = sin(M_PI * (double)i / n), c = cos(M_PI * (double)i / n);
-    lo[i] = make_float2((float)(-2.0 * s * s), (float)(2.0 * s * c));
+    less[i] = make_float2((float)(-2.0 * s * s), (float)(2.0 * s * c));
   }
+  const size_t lo_bytes = lo.size() * sizeof(float2);
   CUDA_TRY(cudaMalloc(&t.hi, hi.size() * sizeof(float2)));
-  CUDA_TRY(cudaMalloc(&t.lo, lo.size() * sizeof(float2)));
+  CUDA_TRY(cudaMalloc(&t.lo, 2 * lo_bytes));
+  t.lo_less_one = t.lo + lo.size();
   CUDA_TRY(cudaMemcpy(t.hi, hi.data(), hi.size() * sizeof(float2), cudaMemcpyHostToDevice));
-  CUDA_TRY(cudaMemcpy(t.lo, lo.data(), lo.size() * sizeof(float2), cudaMemcpyHostToDevice));
+  CUDA_TRY(cudaMemcpy(t.lo, lo.data(), lo_bytes, cudaMemcpyHostToDevice));
+  CUDA_TRY(cudaMemcpy(t.lo_less_one, less.data(), lo_bytes, cudaMemcpyHostToDevice));
   // adjoint_kernel's largest shape (88 KB bounds them all: 40 KB of staged twiddles,
   // 12 of entries, 16 of roots and 16 of list ends)
   CUDA_TRY(cudaFuncSetAttribute(adjoint_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 88 << 10));
@@ -2093,7 +2100,7 @@ static int adjoint_side(bool grad_data, int n, int nd, int nt, int nb, const flo
   a.slots = ADJ_THREADS / a.fblk;
   while ((1 << a.lsh) < a.fblk && a.lsh < 5) a.lsh++;
   while ((32 << a.ash) < a.fblk) a.ash++;
-  a.tw_hi = tw.hi; a.tw_lo = tw.lo; a.lo_bits = tw.lo_bits; a.hi_count = tw.hi_count;
+  a.tw_hi = tw.hi; a.tw_lo = tw.lo_less_one; a.lo_bits = tw.lo_bits; a.hi_count = tw.hi_count;
   a.fx = n / ADJ_R / a.fblk;
   const int cap = ADJ_TAB / adj_entry_bytes(a.fblk);
   a.chunk = std::min(std::min(nb, ADJ_CHUNK), cap / a.slots);
