@@ -39,7 +39,9 @@ def candidates(n):
 
 #: What tune(n) found on a B200 (CUDA events, probe workload of probe_shape):
 #: the kernel configuration and the cost per pair (us) in the persistent launch
-#: and on the job's own launches.  Used when a batch is not tuned.
+#: and on the job's own launches.  Used when a batch is not tuned.  (With flatw_kernel and
+#: large2_kernel tune() finds 0.0031, 0.0064, 0.0132, 0.033, 0.064, 0.177 and 0.350 on own
+#: launches; these older costs keep jobs near the line in the persistent launch.)
 B200 = {
     1024: ({"unit_items": 8}, 0.0046, 0.0037),
     2048: ({"unit_items": 8}, 0.0094, 0.0076),

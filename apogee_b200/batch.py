@@ -13,7 +13,7 @@ from :mod:`apogee_b200.autotune`.
 
 A job can instead run as its own launches, with the kernels specialised for
 its n (the single-CTA filter with 512 or 1024 threads at n = 8192 / 16384,
-the two-pass kernels above), in the same stream and the same graph, writing
+the four-step kernel above), in the same stream and the same graph, writing
 the same records: ``tune={n: {"dedicated": True}}`` forces that, and the
 autotuner measures both forms per n and sends a job to its own launches when
 the time it saves per pair, times its pairs, exceeds the cost of a launch

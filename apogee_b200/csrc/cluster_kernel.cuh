@@ -1,5 +1,5 @@
 // Fused matched filter for n = 32768 and 65536 on a thread-block cluster:
-// the four-step split of the two-pass kernels (large_kernel.cuh) with the
+// the four-step split of large_kernel.cuh with the
 // transpose between the passes carried through distributed shared memory
 // instead of an HBM/L2 scratch.
 //
@@ -31,7 +31,7 @@
 // CTA's time, the three barriers ~20%), so short runs at n = 32768 and captured ones
 // (it has no scratch) come here.  The arithmetic (products, FFT passes,
 // twiddles, key order) is that of large_pass_a / large_pass_b, so the outputs
-// equal the two-pass kernels'.  Clusters walk the pairs template-major with a
+// equal theirs and large2_kernel's.  Clusters walk the pairs template-major with a
 // stride of the cluster count, so clusters running at the same time share a
 // template spectrum in L2.
 #pragma once

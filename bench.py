@@ -46,7 +46,7 @@ FLOPS_PER_PAIR = lambda n: 5 * n * int(np.log2(n)) + 9 * n   # the reference's o
 # multiply-add; the 16-point first stage runs on the CUDA cores.
 TC_FLOPS_PER_PAIR = 12 * 128 * 64 * 16 * 2 / 8
 # DRAM bytes per launch from one ncu capture of the same kernels on this workload
-# (profiles/coarse_tc_ws_band512_16x1024.md, profiles/flat_kernel_n4096_16x1024.md).
+# (profiles/coarse_tc_ws_band512_16x1024.md, profiles/flatw_kernel.md).
 TRAFFIC_COARSE_TC = 4.347e6
 TRAFFIC_FLAT = 34.18e6
 
@@ -1032,8 +1032,7 @@ def large_record(dev, local, seed, steps, warmup, coarse, cpu_sample=True, rank=
             coarse]),
         "value": pairs / (hier_ms * 1e-3), "unit": "pairs/s", "ms_per_step": hier_ms,
         "gate": gate,
-        "timing": "CUDA events per step, %d steps; the refine of the survivors reads their "
-                  "count on the host at this n" % steps,
+        "timing": "CUDA events per step, %d steps" % steps,
         "flat": {"value": pairs / (flat_ms * 1e-3), "unit": "pairs/s", "ms_per_step": flat_ms,
                  "fp64_detections_missed": missed_f},
         "hier": {"value": pairs / (hier_ms * 1e-3), "ms_per_step": hier_ms, "coarse": coarse,

@@ -53,7 +53,7 @@ typedef struct mfb_hplan mfb_hplan;
 /* ---- flat matched filter ------------------------------------------------ */
 
 /* Replaces ap_mf_create (src/matchfilt.c:73-133; matchedfilter.h:53).  n is a
-   power of two, 64 .. 2^20 (above 16384 the two-pass four-step); device is a
+   power of two, 64 .. 2^20 (above 16384 a four-step split); device is a
    CUDA ordinal.  *out = NULL on error. */
 int mfb_create(mfb_plan **out, size_t n, int ndata, int ntmpl, int device);
 /* Replaces ap_mf_destroy (src/matchfilt.c:135-146). */
