@@ -45,7 +45,8 @@
 // n = 65536: one ticket per unit with every wait, fence and decode in line 450 us;
 // those off the critical path 383; four units per ticket and batches of 150 items
 // (450 MB of scratch) 307; per-item dependencies instead of batches (205 MB) 303, with two
-// units per ticket 310 (103 MB), with one 363.  What bounds it now: latency at 16
+// units per ticket 310 (103 MB), with one 363.  One pair per thread was slower: 64 registers
+// and four CTAs per SM 322 (n = 262144: 1803 against 1538), 80 and three 309 (1612).  What bounds it now: latency at 16
 // warps per SM (128 registers) -- FMA pipe ~40%, issue ~37%, warps waiting at the exchange
 // barrier of A and on loads.
 #pragma once
