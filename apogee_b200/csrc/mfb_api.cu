@@ -2086,6 +2086,40 @@ static size_t adjoint_smem(int fblk, int items, int roots) {
 // and 1.4e-7.
 constexpr int ADJ_FILL = 4;
 constexpr int ADJ_FEW = 16;
+struct AdjPlan {
+  int fblk, slots, fx;      // f0 values and own rows per CTA, blocks of f0 values
+  long long tiles, split;   // CTAs of one split, splits of the summed rows
+  int rows;                 // summed rows per split
+  int clusters;
+};
+static AdjPlan adjoint_plan(int n, int own, int other, int sms) {
+  AdjPlan p;
+  p.fblk = std::min(n / ADJ_R, ADJ_THREADS);
+  p.slots = ADJ_THREADS / p.fblk;
+  p.fx = n / ADJ_R / p.fblk;
+  p.tiles = (long long)p.fx * ((own + p.slots - 1LL) / p.slots);
+  const long long target = (long long)ADJ_FILL * sms;
+  p.split = 1;
+  if (p.tiles < target) p.split = std::min<long long>(other, target / p.tiles);
+  // clusters that fit one wave; a device of few SMs (a partition) may have room for none
+  const long long fit = 7LL * sms / 4 / p.tiles / ADJ_CLUSTER * ADJ_CLUSTER;
+  p.clusters = p.tiles <= ADJ_FEW && p.split > ADJ_CLUSTER && fit > 0;
+  if (p.clusters) p.split = std::min(p.split, fit);
+  else if (p.tiles > ADJ_FEW) p.split = std::min<long long>(p.split, std::max(1, other / 2));
+  p.rows = (int)((other + p.split - 1) / p.split);
+  p.split = (other + p.rows - 1LL) / p.rows;
+  if (p.clusters) p.split = (p.split + ADJ_CLUSTER - 1) / ADJ_CLUSTER * ADJ_CLUSTER;   // the last may have no rows
+  return p;
+}
+
+extern "C" int mfb_adjoint_plan(size_t n, int own, int other, int sms, int64_t *out) {
+  if (!mfb_supported(n) || own < 1 || other < 1 || sms < 1 || !out)
+    return fail(MFB_ERR_ARG, "adjoint plan: bad arguments");
+  const AdjPlan p = adjoint_plan((int)n, own, other, sms);
+  out[0] = p.tiles; out[1] = p.split; out[2] = p.rows; out[3] = p.clusters;
+  return MFB_OK;
+}
+
 static int adjoint_side(bool grad_data, int n, int nd, int nt, int nb, const float2 *src,
                         const int64_t *idx, const float2 *gz, float2 *out, const AdjTables &tw,
                         int sms, cudaStream_t st) {
@@ -2096,35 +2130,22 @@ static int adjoint_side(bool grad_data, int n, int nd, int nt, int nb, const flo
   a.own = grad_data ? nd : nt;
   a.other = grad_data ? nt : nd;
   if ((a.own + 7LL) / 8 > 65535) return fail(MFB_ERR_UNSUPPORTED, "adjoint: too many rows (%d)", a.own);
-  a.fblk = std::min(n / ADJ_R, ADJ_THREADS);
-  a.slots = ADJ_THREADS / a.fblk;
+  const AdjPlan p = adjoint_plan(n, a.own, a.other, sms);
+  a.fblk = p.fblk; a.slots = p.slots; a.fx = p.fx;
+  a.other_per_split = p.rows; a.clusters = p.clusters; a.accumulate = p.split > 1;
   while ((1 << a.lsh) < a.fblk && a.lsh < 5) a.lsh++;
   while ((32 << a.ash) < a.fblk) a.ash++;
   a.tw_hi = tw.hi; a.tw_lo = tw.lo_less_one; a.lo_bits = tw.lo_bits; a.hi_count = tw.hi_count;
-  a.fx = n / ADJ_R / a.fblk;
   const int cap = ADJ_TAB / adj_entry_bytes(a.fblk);
   a.chunk = std::min(std::min(nb, ADJ_CHUNK), cap / a.slots);
   a.chunks = (nb + a.chunk - 1) / a.chunk;
   const int lists = std::min(cap / (a.chunk * a.slots), ADJ_ITEMS / a.slots);   // per own row and round
   a.rows_per_round = a.chunks == 1 ? lists : 1;
   a.lists_per_round = a.chunks == 1 ? 1 : std::min(lists, a.chunks);
-  const long long tiles = (long long)a.fx * ((a.own + a.slots - 1) / a.slots);
-  const long long target = (long long)ADJ_FILL * sms;
-  long long split = 1;
-  if (tiles < target) split = std::min<long long>(a.other, target / tiles);
-  a.clusters = tiles <= ADJ_FEW && split > ADJ_CLUSTER;
-  if (a.clusters)
-    split = std::min<long long>(split, 7LL * sms / 4 / tiles / ADJ_CLUSTER * ADJ_CLUSTER);
-  else if (tiles > ADJ_FEW)
-    split = std::min<long long>(split, std::max(1, a.other / 2));
-  a.other_per_split = (int)((a.other + split - 1) / split);
-  split = (a.other + a.other_per_split - 1) / a.other_per_split;
-  a.accumulate = split > 1;
-  if (a.clusters) split = (split + ADJ_CLUSTER - 1) / ADJ_CLUSTER * ADJ_CLUSTER;   // the last may have no rows
   if (a.accumulate) CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)a.own * n * sizeof(float2), st));
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof cfg);
-  cfg.gridDim = dim3((unsigned)tiles, (unsigned)split);
+  cfg.gridDim = dim3((unsigned)p.tiles, (unsigned)p.split);
   cfg.blockDim = dim3(ADJ_THREADS);
   cfg.dynamicSmemBytes = adjoint_smem(a.fblk, lists * a.slots, tw.hi_count + (1 << tw.lo_bits));
   cfg.stream = st;
