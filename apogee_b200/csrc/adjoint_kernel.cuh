@@ -29,7 +29,7 @@
 // of them add up their sums through distributed shared memory first: 291 atomic
 // additions in a row to one output (3 x 872 pairs at n = 2048) doubled the
 // gradient's rounding.  The lags are the forward pass's argmax lags; nothing of the
-// correlation series is stored.
+// correlation series is stored.  Runs with little to sum take adjoint_direct.cuh.
 #pragma once
 #include <cooperative_groups.h>
 #include <cstdint>

@@ -29,6 +29,7 @@
 #include "packed_passes.cuh"
 #include "large2_kernel.cuh"
 #include "adjoint_kernel.cuh"
+#include "adjoint_direct.cuh"
 #include "batch_kernel.cuh"
 #include "gate_kernels.cuh"
 
@@ -2112,11 +2113,101 @@ static AdjPlan adjoint_plan(int n, int own, int other, int sms) {
   return p;
 }
 
-extern "C" int mfb_adjoint_plan(size_t n, int own, int other, int sms, int64_t *out) {
-  if (!mfb_supported(n) || own < 1 || other < 1 || sms < 1 || !out)
+// adjoint_direct_kernel: own rows per CTA (oc) shrink, and then the summed rows split
+// over blockIdx.z, until the grid covers the device about twice; splits past a cluster
+// or two are summed by clusters.
+struct AdjDirectPlan {
+  int oc, fx, chunks, clusters, rows;
+  long long split;
+};
+static AdjDirectPlan adjoint_direct_plan(int n, int own, int other, int sms) {
+  AdjDirectPlan p;
+  p.fx = ((n >> 1) + ADJ_THREADS - 1) / ADJ_THREADS;
+  const long long target = 2LL * sms;
+  p.oc = 8;
+  while (p.oc > 1 && (long long)p.fx * ((own + p.oc - 1) / p.oc) < target) p.oc >>= 1;
+  p.chunks = (own + p.oc - 1) / p.oc;
+  const long long tiles = (long long)p.fx * p.chunks;
+  p.split = tiles < target ? std::min<long long>(other, (target + tiles - 1) / tiles) : 1;
+  p.rows = (int)((other + p.split - 1) / p.split);
+  p.split = (other + p.rows - 1LL) / p.rows;
+  p.clusters = p.oc == 1 && p.split > ADJD_ATOMICS;
+  if (p.clusters) p.split = (p.split + ADJ_CLUSTER - 1) / ADJ_CLUSTER * ADJ_CLUSTER;   // the last may have no rows
+  return p;
+}
+
+// Whether a gradient takes adjoint_direct_kernel: few entries in all (the limit falls with
+// n, whose frequencies the buckets share 16 to a thread), or too few per pair to pay for a
+// pair's 16-point transform; not where a CTA would sum more than ADJD_ROWS rows (the
+// buckets round less), nor at the longest n with few own rows, where the buckets fill the
+// device.  B200, one gradient (own x other rows, bins), us direct against buckets:
+// n = 64, 32 x 32 of 4 6.9 / 15.1; n = 1024, 3 x 32 of 16 8.6 / 11.0; n = 4096, 8 x 8 of 4
+// 8.3 / 9.7, 128 x 8 of 1 11.8 / 18.9; and past the line n = 1024, 32 x 512 of 16
+// 190 / 68, n = 4096, 128 x 8 of 16 48 / 23, n = 262144, 1 x 32 of 1 91 / 24.
+static bool adjoint_direct(int n, int own, int other, int nb, int rows) {
+  if (rows > ADJD_ROWS || (n > 65536 && own < 4)) return false;
+  if (nb == 1 || (n <= 256 && nb <= 4) || (nb == 2 && other <= 2)) return true;
+  const double entries = (double)n * own * other * nb;
+  const int limit = n <= 256 ? 1 << 25 : n <= 2048 || nb == 2 ? 1 << 23 : 1 << 22;
+  return entries <= (other <= 2 ? limit / 2 : limit);
+}
+
+extern "C" int mfb_adjoint_plan(size_t n, int own, int other, size_t nb, int sms, int64_t *out) {
+  if (!mfb_supported(n) || own < 1 || other < 1 || nb < 1 || nb > n || sms < 1 || !out)
     return fail(MFB_ERR_ARG, "adjoint plan: bad arguments");
+  const AdjDirectPlan d = adjoint_direct_plan((int)n, own, other, sms);
+  if (adjoint_direct((int)n, own, other, (int)nb, d.rows)) {
+    out[0] = (long long)d.fx * d.chunks; out[1] = d.split; out[2] = d.rows; out[3] = d.clusters;
+    out[4] = 1;
+    return MFB_OK;
+  }
   const AdjPlan p = adjoint_plan((int)n, own, other, sms);
-  out[0] = p.tiles; out[1] = p.split; out[2] = p.rows; out[3] = p.clusters;
+  out[0] = p.tiles; out[1] = p.split; out[2] = p.rows; out[3] = p.clusters; out[4] = 0;
+  return MFB_OK;
+}
+
+// A launch in clusters of ADJ_CLUSTER along the given grid dimension, or without.
+template <typename Args>
+static cudaError_t launch_adjoint(void (*kernel)(Args), dim3 grid, size_t smem, int cy, int cz,
+                                  const Args &a, cudaStream_t st) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof cfg);
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(ADJ_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 1;
+  attr.val.clusterDim.y = cy;
+  attr.val.clusterDim.z = cz;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a);
+  return e == cudaSuccess ? cudaGetLastError() : e;
+}
+
+template <bool GD>
+static int adjoint_direct_side(int n, int nd, int nt, int nb, const float2 *src, const int64_t *idx,
+                               const float2 *gz, float2 *out, const AdjTables &tw,
+                               const AdjDirectPlan &p, cudaStream_t st) {
+  AdjDirectArgs a;
+  memset(&a, 0, sizeof a);
+  a.src = src; a.idx = idx; a.gz = gz; a.out = out;
+  a.n = n; a.nd = nd; a.nt = nt; a.nb = nb;
+  a.own = GD ? nd : nt;
+  a.other = GD ? nt : nd;
+  a.tw_hi = tw.hi; a.tw_lo = tw.lo; a.lo_bits = tw.lo_bits; a.hi_count = tw.hi_count;
+  a.other_per_split = p.rows; a.accumulate = p.split > 1; a.clusters = p.clusters;
+  a.bins_per_round = std::min(nb, ADJD_CAP / p.oc);
+  a.rows_per_round = a.bins_per_round == nb ? ADJD_CAP / (p.oc * nb) : 1;
+  if (a.accumulate) CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)a.own * n * sizeof(float2), st));
+  const dim3 grid((unsigned)p.fx, (unsigned)p.chunks, (unsigned)p.split);
+  auto kernel = p.oc == 8   ? adjoint_direct_kernel<8, GD>
+                : p.oc == 4 ? adjoint_direct_kernel<4, GD>
+                : p.oc == 2 ? adjoint_direct_kernel<2, GD>
+                            : adjoint_direct_kernel<1, GD>;
+  CUDA_TRY(launch_adjoint(kernel, grid, 0, 1, p.clusters ? ADJ_CLUSTER : 1, a, st));
   return MFB_OK;
 }
 
@@ -2130,6 +2221,10 @@ static int adjoint_side(bool grad_data, int n, int nd, int nt, int nb, const flo
   a.own = grad_data ? nd : nt;
   a.other = grad_data ? nt : nd;
   if ((a.own + 7LL) / 8 > 65535) return fail(MFB_ERR_UNSUPPORTED, "adjoint: too many rows (%d)", a.own);
+  const AdjDirectPlan dp = adjoint_direct_plan(n, a.own, a.other, sms);
+  if (adjoint_direct(n, a.own, a.other, nb, dp.rows))
+    return grad_data ? adjoint_direct_side<true>(n, nd, nt, nb, src, idx, gz, out, tw, dp, st)
+                     : adjoint_direct_side<false>(n, nd, nt, nb, src, idx, gz, out, tw, dp, st);
   const AdjPlan p = adjoint_plan(n, a.own, a.other, sms);
   a.fblk = p.fblk; a.slots = p.slots; a.fx = p.fx;
   a.other_per_split = p.rows; a.clusters = p.clusters; a.accumulate = p.split > 1;
@@ -2143,21 +2238,10 @@ static int adjoint_side(bool grad_data, int n, int nd, int nt, int nb, const flo
   a.rows_per_round = a.chunks == 1 ? lists : 1;
   a.lists_per_round = a.chunks == 1 ? 1 : std::min(lists, a.chunks);
   if (a.accumulate) CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)a.own * n * sizeof(float2), st));
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof cfg);
-  cfg.gridDim = dim3((unsigned)p.tiles, (unsigned)p.split);
-  cfg.blockDim = dim3(ADJ_THREADS);
-  cfg.dynamicSmemBytes = adjoint_smem(a.fblk, lists * a.slots, tw.hi_count + (1 << tw.lo_bits));
-  cfg.stream = st;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = 1;
-  attr.val.clusterDim.y = a.clusters ? ADJ_CLUSTER : 1;
-  attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  CUDA_TRY(cudaLaunchKernelEx(&cfg, grad_data ? adjoint_kernel<true> : adjoint_kernel<false>, a));
-  CUDA_TRY(cudaGetLastError());
+  const dim3 grid((unsigned)p.tiles, (unsigned)p.split);
+  const size_t smem = adjoint_smem(a.fblk, lists * a.slots, tw.hi_count + (1 << tw.lo_bits));
+  CUDA_TRY(launch_adjoint(grad_data ? adjoint_kernel<true> : adjoint_kernel<false>, grid, smem,
+                          a.clusters ? ADJ_CLUSTER : 1, 1, a, st));
   return MFB_OK;
 }
 

@@ -292,12 +292,13 @@ int mfb_batch_destroy(mfb_batch *b);
 int mfb_adjoint(int device, size_t n, const void *data, int nd, const void *templates, int nt,
                 size_t nb, const int64_t *idx, const void *gz, void *grad_data, void *grad_tmpl,
                 void *stream);
-/* How mfb_adjoint divides one gradient of `own` rows, a sum over `other` rows, on a
-   device of `sms` SMs (host arithmetic only): out[0] CTAs per split, out[1] splits of
-   the summed rows, out[2] summed rows per split, out[3] 1 where clusters of eight
-   splits add up before the atomics (out[1] is then a multiple of eight, and the
-   last splits may have no rows). */
-int mfb_adjoint_plan(size_t n, int own, int other, int sms, int64_t *out);
+/* How mfb_adjoint divides one gradient of `own` rows, a sum over `other` rows with nb
+   bins per pair, on a device of `sms` SMs (host arithmetic only): out[0] CTAs per split,
+   out[1] splits of the summed rows, out[2] summed rows per split, out[3] 1 where
+   clusters of eight splits add up before the atomics (out[1] is then a multiple of
+   eight, and the last splits may have no rows), out[4] 1 for the kernel that evaluates
+   every entry at every frequency, 0 for the one that sums entries into buckets first. */
+int mfb_adjoint_plan(size_t n, int own, int other, size_t nb, int sms, int64_t *out);
 
 /* ---- large transforms with no allocation --------------------------------- */
 

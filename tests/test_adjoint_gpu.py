@@ -224,3 +224,61 @@ def test_adjoint_kernel_edges(n, nd, nt, nb, peaks):
         bound = (24 + nb + max(nd, nt)) * 2.0 ** -24 * scale
         err = (got.to(want.dtype) - want).abs()
         assert bool((err <= bound + 1e-30).all()), (n, nd, nt, nb, float((err / scale.clamp(min=1e-30)).max()))
+
+
+@pytest.mark.parametrize("direct, n, nd, nt, nb, peaks", [
+    (1, 64, 1, 600, 1, 1.0),        # half a warp of frequencies, splits summed by clusters
+    (1, 64, 3, 9, 64, 0.7),         # nine splits: two clusters, most without rows
+    (1, 512, 5, 8, 33, 1.0),        # eight splits: atomics alone
+    (1, 1024, 2, 100, 4, 0.01),     # rows without a peak
+    (1, 4096, 7, 1, 20, 1.0),       # one summed row
+    (1, 16384, 19, 3, 1, 1.0),      # two own rows per thread, the last CTA's second one missing
+    (1, 16384, 38, 3, 1, 0.5),      # four
+    (1, 16384, 77, 16, 1, 1.0),     # eight, as many summed rows as the rule allows
+    (1, 1 << 18, 4, 2, 2, 1.0),
+    (0, 64, 65, 140, 64, 0.5),      # 64 own rows per CTA, a second block of one row
+    (0, 256, 70, 60, 33, 1.0),      # one entry more than a list
+    (0, 512, 40, 20, 32, 0.9),      # lists exactly full
+    (0, 1024, 9, 12, 100, 0.7),     # four own rows per CTA, several lists per row
+    (0, 16384, 2, 8, 20, 1.0),      # 8 splits: atomics alone
+    (0, 16384, 2, 9, 20, 1.0),      # 9: clusters of eight
+    (0, 4096, 17, 5, 16, 1.0),      # one tile too many for clusters
+])
+def test_both_adjoint_kernels_at_their_edges(direct, n, nd, nt, nb, peaks):
+    """As test_adjoint_kernel_edges (its bound holds for both: the direct form has two
+    twiddles and their product, three products and as many additions), each shape on the
+    kernel that the rule gives its data gradient."""
+    import ctypes
+    import torch
+    from apogee_b200 import _lib
+    out = (ctypes.c_int64 * 5)()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    _lib.check(_lib.lib().mfb_adjoint_plan(n, nd, nt, nb, sms, out))
+    if sms == 148:
+        assert out[4] == direct
+    for got, want, scale in _adjoint_direct(n, nd, nt, nb, n + nb, peaks):
+        bound = (24 + nb + max(nd, nt)) * 2.0 ** -24 * scale
+        err = (got.to(want.dtype) - want).abs()
+        assert bool((err <= bound + 1e-30).all()), (n, nd, nt, nb, float((err / scale.clamp(min=1e-30)).max()))
+
+
+@pytest.mark.parametrize("n, nb", [(1024, 4), (16384, 64)])
+def test_row_without_a_peak_adds_nothing(n, nb):
+    """A NaN row that no pair reports a peak for leaves the gradients finite, on both
+    kernels."""
+    import torch
+    from apogee_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(n)
+    nd, nt = 4, 12
+    D = torch.randn(nd, n, dtype=torch.complex64, device="cuda", generator=g)
+    H = torch.randn(nt, n, dtype=torch.complex64, device="cuda", generator=g)
+    H[5] = float("nan")
+    idx = torch.randint(0, n, (nd, nt, nb), device="cuda", generator=g)
+    idx[:, 5] = -1
+    gz = torch.randn(nd, nt, nb, dtype=torch.complex64, device="cuda", generator=g)
+    gd, gh = torch.full_like(D, float("nan")), torch.full_like(H, float("nan"))
+    _lib.check(_lib.lib().mfb_adjoint(0, n, D.data_ptr(), nd, H.data_ptr(), nt, nb, idx.data_ptr(),
+                                      gz.data_ptr(), gd.data_ptr(), gh.data_ptr(),
+                                      torch.cuda.current_stream().cuda_stream))
+    assert torch.isfinite(torch.view_as_real(gd)).all()
+    assert (gh[5] == 0).all() and torch.isfinite(torch.view_as_real(gh)).all()

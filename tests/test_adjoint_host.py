@@ -91,21 +91,26 @@ def test_closed_form_matches_dense_gradient_and_fd():
 
 @pytest.mark.parametrize("sms", [1, 2, 8, 16, 36, 70, 72, 73, 74, 132, 148, 160])
 def test_split_covers_the_summed_rows(sms):
-    """The rule on splits and clusters, over SM counts (a partitioned device has few):
-    every summed row in one split, no split empty but to fill the last cluster."""
+    """The rule on splits and clusters of both kernels, over SM counts (a partitioned
+    device has few): every summed row in one split, no split empty but to fill the
+    last cluster, and a grid the hardware takes."""
     if not os.path.exists(_lib.LIB_PATH):
         pytest.skip("libmfb.so not built")
     L = _lib.lib()
-    out = (ctypes.c_int64 * 4)()
+    out = (ctypes.c_int64 * 5)()
+    kinds = set()
     for n in (64, 512, 4096, 16384, 65536, 1 << 20):
         for own in (1, 2, 3, 8, 16, 17, 64, 300, 5000):
             for other in (1, 2, 7, 8, 9, 16, 63, 300, 5000):
-                _lib.check(L.mfb_adjoint_plan(n, own, other, sms, out))
-                tiles, split, rows, clusters = list(out)
-                assert tiles >= 1 and 1 <= split <= 65535 and rows >= 1
-                assert split * rows >= other
-                empty = split - -(-other // rows)
-                assert empty < (8 if clusters else 1)
-                if clusters:
-                    assert split % 8 == 0 and tiles * split <= max(8 * tiles, 2 * sms + 7 * tiles)
-    assert L.mfb_adjoint_plan(100, 1, 1, sms, out) == _lib.MFB_ERR_ARG
+                for nb in (1, 2, 8, 64):
+                    _lib.check(L.mfb_adjoint_plan(n, own, other, nb, sms, out))
+                    tiles, split, rows, clusters, direct = list(out)
+                    kinds.add((clusters, direct))
+                    assert tiles >= 1 and 1 <= split <= 65535 and rows >= 1
+                    assert split * rows >= other
+                    empty = split - -(-other // rows)
+                    assert empty < (8 if clusters else 1)
+                    if clusters:
+                        assert split % 8 == 0
+    assert {(0, 0), (0, 1)} <= kinds and (sms < 74 or (1, 0) in kinds)
+    assert L.mfb_adjoint_plan(100, 1, 1, 1, sms, out) == _lib.MFB_ERR_ARG
