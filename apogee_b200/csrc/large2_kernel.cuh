@@ -27,10 +27,11 @@
 // is being worked on and never waits -- whatever CTAs are resident.  D and the ring
 // put at least two tickets per CTA between an item's last A ticket and its first B
 // ticket, and again until its slot is wanted, so in steady state nothing waits,
-// and both kinds of unit run side by side.  Waits are bounded (LARGE2_SPIN); a wait
+// and both kinds of unit run side by side.  Waits are bounded (LARGE2_SPIN looks); a wait
 // that runs out sets the plan's error word and every CTA stops taking tickets.
-// The last CTA to leave resets the counters; a finalized item leaves its records
-// zero.
+// The last CTA to leave resets the counters, and the records of a launch that gave up; a
+// finalized item leaves its records zero.  So no launch spoils a later one as long as
+// launches on the same counters follow one another (see run_large, mfb_api.cu).
 //
 // What a unit costs beside its arithmetic is latency: a ticket is drawn one ahead;
 // thread 0 decodes it and looks at its dependency while the current ticket's
@@ -59,12 +60,12 @@ constexpr int LARGE2_GROUP = 4;                // units per ticket, at most
 constexpr unsigned LARGE2_SPIN = 1u << 22;
 constexpr int LARGE2_BUF = 4096 + 4096 / 16;   // float4 records of the exchange buffer
 
-// Counters of one plan, zero between launches; the three arrays of one entry
-// per ring slot follow: tickets of kind A and B finished and items finalized in
-// the slot, all cumulative over the launch.
+// Counters, zero between launches; the three arrays of one entry per ring slot
+// follow: tickets of kind A and B finished and items finalized in the slot, all
+// cumulative over the launch.
 struct Large2Ctl {
   unsigned long long ticket;
-  unsigned exits;
+  unsigned exits;           // CTAs that left, and in the high half those that gave up
   int err;                  // a wait ran out in this launch
 };
 
@@ -77,6 +78,8 @@ struct Large2Args {
   Large2Ctl *ctl;
   int *err;                 // mapped host word, set when a wait ran out
   int ring;                 // slots
+  unsigned spin;            // LARGE2_SPIN
+  int hold;                 // tests: added to the count of A tickets that B waits for
 };
 
 enum { L2_A = 0, L2_B = 1, L2_END = 2 };
@@ -168,7 +171,7 @@ __global__ void __launch_bounds__(256, 2) large2_kernel(const Large2Args g) {
   auto depends = [&](const Large2Ticket &k, unsigned &need) {
     unsigned slot;
     const unsigned round = (unsigned)div((unsigned long long)k.item, (unsigned)ring, slot);
-    need = k.kind == L2_A ? round : (round + 1) * gA;
+    need = k.kind == L2_A ? round : (round + 1) * gA + g.hold;
     return (k.kind == L2_A ? f_done : a_done) + slot;
   };
   // thread 0: ticket x into s_tk[i].
@@ -205,7 +208,7 @@ __global__ void __launch_bounds__(256, 2) large2_kernel(const Large2Args g) {
     unsigned need, spins = 0;
     const unsigned *ctr = depends(s_tk[i], need);
     while (ld_acquire32(ctr) < need) {
-      if (++spins > LARGE2_SPIN || *(volatile int *)&g.ctl->err) {
+      if (++spins > g.spin || *(volatile int *)&g.ctl->err) {
         *(volatile int *)&g.ctl->err = 1;
         *(volatile int *)g.err = 1;
         __threadfence_system();
@@ -256,6 +259,7 @@ __global__ void __launch_bounds__(256, 2) large2_kernel(const Large2Args g) {
     next = atomicAdd(&g.ctl->ticket, 1ull);
   }
   __syncthreads();
+  bool gave_up = false;
   for (int par = 0;; par ^= 1) {
     const Large2Ticket tk = s_tk[par];
     if (tk.fin >= 0) finalize(tk.fin);
@@ -267,7 +271,7 @@ __global__ void __launch_bounds__(256, 2) large2_kernel(const Large2Args g) {
       if (tk.kind == L2_END) break;
       if (tid == 0) s_ok = wait(par);
       __syncthreads();
-      if (!s_ok) break;
+      if (!s_ok) { gave_up = true; break; }
     }
     const int slot = (int)(tk.item % ring);
     if (tk.kind == L2_A) {
@@ -432,12 +436,20 @@ __global__ void __launch_bounds__(256, 2) large2_kernel(const Large2Args g) {
   }
   __syncthreads();
   if (tid == 0) {
+    // low half: CTAs that left; high half: those that gave up
+    const unsigned mine = gave_up ? 0x10001u : 1u;
     __threadfence();
-    s_ok = atomicAdd(&g.ctl->exits, 1u) == gridDim.x - 1;
+    const unsigned sum = atomicAdd(&g.ctl->exits, mine) + mine;
+    s_ok = (sum & 0xffffu) != gridDim.x ? 0 : (sum >> 16) ? 2 : 1;
   }
   __syncthreads();
   if (s_ok) {                 // every other CTA has left
     for (int i = tid; i < 3 * ring; i += 256) a_done[i] = 0u;
+    if (s_ok == 2) {
+      __threadfence();
+      for (long long i = tid; i < (long long)ring * nb2; i += 256) g.rec[i] = make_uint4(0u, 0u, 0u, 0u);
+      g.ctl->err = 0;
+    }
     if (tid == 0) {
       g.ctl->ticket = 0ull;
       g.ctl->exits = 0u;

@@ -539,11 +539,13 @@ extern "C" size_t mfb_nbins(size_t n, size_t binsize, size_t start, size_t end) 
 
 // ---------------------------------------------------------------- flat plan
 // large2_kernel's scratch: rows, candidate records and counters (both zero
-// between launches) of `ring` items, and the mapped error word.
+// between launches) of `ring` items, and the mapped error word.  Counters and records
+// are there twice, [0] for runs that follow one another and [1] for runs captured by
+// a caller, whose order nobody here knows.
 struct LargeScratch {
-  float4 *Y = nullptr;      // one allocation: Y, then rec, then ctl
-  uint4 *rec = nullptr;
-  Large2Ctl *ctl = nullptr;
+  float4 *Y = nullptr;      // one allocation: Y, then ctl[0], rec[0], ctl[1], rec[1]
+  Large2Ctl *ctl[2] = {nullptr, nullptr};
+  uint4 *rec[2] = {nullptr, nullptr};
   int *err = nullptr;       // from g_err_words
   cudaEvent_t used = nullptr;   // after the last use outside a capture
   int ring = 0;
@@ -593,6 +595,8 @@ struct mfb_plan {
   std::vector<LargeScratch> ls_old;
   int packed = 1;           // use flatw_kernel where it applies (mfb_set_packed)
   int cluster = -1;         // mfb_set_cluster's choice; -1: cluster_mode's rule
+  int hold = 0;             // mfb_test_wait_limit
+  bool own_capture = false; // a capture whose graph this library launches
 };
 
 struct DeviceGuard {
@@ -735,7 +739,9 @@ static bool capturing(cudaStream_t s) {
 // with more items (run_series over many blocks) gets a larger ring; the smaller
 // one is kept until the plan goes, because captured graphs may hold it.
 static size_t large_rec_bytes(int ring) { return (size_t)ring * 2 * LARGE_MAX_BINS * sizeof(uint4); }
-static size_t large_ctl_bytes(int ring) { return sizeof(Large2Ctl) + (size_t)ring * 3 * sizeof(unsigned); }
+static size_t large_ctl_bytes(int ring) {
+  return (sizeof(Large2Ctl) + (size_t)ring * 3 * sizeof(unsigned) + 15) & ~(size_t)15;
+}
 
 static void large_free(LargeScratch &s) {
   cudaFree(s.Y);
@@ -745,10 +751,7 @@ static void large_free(LargeScratch &s) {
 }
 static int large_scratch(mfb_plan *p, long long pairs) {
   LargeScratch &cur = p->ls;
-  if (cur.ring && *(volatile int *)cur.err) {   // an earlier launch gave up half-way: start afresh
-    CUDA_TRY(cudaDeviceSynchronize());
-    CUDA_TRY(cudaMemset(cur.rec, 0, large_rec_bytes(cur.ring) + large_ctl_bytes(cur.ring)));
-    CUDA_TRY(cudaDeviceSynchronize());
+  if (cur.ring && *(volatile int *)cur.err) {   // an earlier launch gave up half-way
     *cur.err = 0;
     return fail(MFB_ERR_CUDA, "an earlier run at n=%zu timed out on a dependency; its outputs are invalid", p->n);
   }
@@ -760,11 +763,13 @@ static int large_scratch(mfb_plan *p, long long pairs) {
   LargeScratch s;
   s.ring = ring;
   const size_t rows = (size_t)ring * p->n * sizeof(float4), rest = large_rec_bytes(ring) + large_ctl_bytes(ring);
-  cudaError_t e = cudaMalloc(&s.Y, rows + rest);
+  cudaError_t e = cudaMalloc(&s.Y, rows + 2 * rest);
   if (e == cudaSuccess) {
-    s.rec = reinterpret_cast<uint4 *>(reinterpret_cast<char *>(s.Y) + rows);
-    s.ctl = reinterpret_cast<Large2Ctl *>(reinterpret_cast<char *>(s.rec) + large_rec_bytes(ring));
-    e = cudaMemset(s.rec, 0, rest);
+    for (int i = 0; i < 2; i++) {
+      s.ctl[i] = reinterpret_cast<Large2Ctl *>(reinterpret_cast<char *>(s.Y) + rows + i * rest);
+      s.rec[i] = reinterpret_cast<uint4 *>(reinterpret_cast<char *>(s.ctl[i]) + large_ctl_bytes(ring));
+    }
+    e = cudaMemset(s.ctl[0], 0, rest);
   }
   if (e == cudaSuccess) e = take_err_word(&s.err);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s.used, cudaEventDisableTiming);
@@ -778,7 +783,10 @@ static int large_scratch(mfb_plan *p, long long pairs) {
   return MFB_OK;
 }
 // Runs of one plan enqueued on different streams share its scratch: each waits
-// for the one before.  (A captured run is ordered by whoever launches its graph.)
+// for the one before.  A captured run is ordered by whoever launches its graph: by
+// launch_hier_graph for the plan's own, else by the caller, who must not let it overlap
+// another run of the plan.  If it does, both runs' outputs are wrong, but no later
+// run's: a caller's captures have counters of their own, zeroed in front of each launch.
 static cudaError_t scratch_begin(const mfb_plan *p) {
   return capturing(p->stream) ? cudaSuccess : cudaStreamWaitEvent(p->stream, p->ls.used, 0);
 }
@@ -852,13 +860,18 @@ static int run_large(mfb_plan *p, int d0, int nd, int t0, int nt, const int32_t 
   g.tw2 = c.c2->twid2;
   g.anchors = c.anchors;
   g.Y = p->ls.Y;
-  g.rec = p->ls.rec;
-  g.ctl = p->ls.ctl;
+  const int foreign = capturing(p->stream) && !p->own_capture;
+  g.rec = p->ls.rec[foreign];
+  g.ctl = p->ls.ctl[foreign];
   CUDA_TRY(cudaHostGetDevicePointer((void **)&g.err, p->ls.err, 0));
   g.ring = p->ls.ring;
+  g.spin = p->hold ? 1u << 14 : LARGE2_SPIN;
+  g.hold = p->hold;
   const long long items = (a.total + 1) / 2;
+  const size_t records = (size_t)(list ? g.ring : std::min<long long>(items, g.ring)) * 2 * nb * sizeof(uint4);
   const int grid = (int)std::min<long long>(c.grid2, std::max<long long>(1, items * c.units_a));
   CUDA_TRY(scratch_begin(p));
+  if (foreign) CUDA_TRY(cudaMemsetAsync(g.ctl, 0, large_ctl_bytes(g.ring) + records, p->stream));
   CUDA_TRY(launch_large2(c, g, grid, p->stream));
   CUDA_TRY(scratch_end(p));
   return MFB_OK;
@@ -894,6 +907,13 @@ static int run_impl(mfb_plan *p, int d0, int nd, int t0, int nt, size_t binsize,
   return MFB_OK;
 }
 
+extern "C" int mfb_test_wait_limit(mfb_plan *p, int delta) {
+  if (!p) return fail(MFB_ERR_ARG, "null plan");
+  if (!is_large(p->n)) return fail(MFB_ERR_STATE, "n=%zu has no pass to hold back", p->n);
+  if (delta != 1 && delta != -1) return fail(MFB_ERR_ARG, "delta must be +1 or -1");
+  p->hold += delta;
+  return MFB_OK;
+}
 extern "C" int mfb_set_cluster(mfb_plan *p, int mode) {
   if (!p) return fail(MFB_ERR_ARG, "null plan");
   if (mode < 0 || mode > 2) return fail(MFB_ERR_ARG, "cluster mode must be 0, 1 or 2");
@@ -1133,7 +1153,7 @@ struct mfb_hplan {
     int d0, nd, t0, nt, same;
     uint32_t thr_bits, gate_bits;
     size_t binsize, start, end;
-    const void *data, *records, *table, *info;
+    const void *data, *records, *table, *info, *scratch;
   };
   RunKey last_key, graph_key;
   bool last_valid = false;
@@ -1684,6 +1704,7 @@ extern "C" int mfb_hier_run_host(mfb_hplan *h, int d0, int nd, int t0, int nt, s
   key.gate_bits = float_bits(h->cal_thr);
   key.binsize = binsize; key.start = start; key.end = end;
   key.data = data; key.records = records; key.table = dtab; key.info = dinfo;
+  key.scratch = ls.Y;   // a graph goes with the scratch it was captured on
   if (graphable && h->graph && memcmp(&key, &h->graph_key, sizeof key) == 0) {
     CUDA_TRY(launch_hier_graph(h, h->graph));
     h->pairs += (long long)nd * nt;
@@ -1704,8 +1725,10 @@ extern "C" int mfb_hier_run_host(mfb_hplan *h, int d0, int nd, int t0, int nt, s
     int rc = MFB_OK;
     cudaError_t e = cudaStreamBeginCapture(h->cap, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
+      h->full->own_capture = true;
       rc = hier_run_impl(h, d0, nd, t0, nt, binsize, threshold, start, end, (int64_t *)records,
                          (char *)records + 8, nullptr, 2, 0, dtab, (long long *)dinfo, data);
+      h->full->own_capture = false;
       e = cudaStreamEndCapture(h->cap, &g);
     }
     h->full->stream = user;

@@ -98,6 +98,12 @@ int mfb_set_packed(mfb_plan *p, int on);
    of up to 64 pairs and captured runs, mode 0 for larger blocks (1.7x faster
    at 1024 pairs); at 65536 mode 0. */
 int mfb_set_cluster(mfb_plan *p, int mode);
+/* Failure-detection test hook, as mfb_batch_test_wait_limit: adds delta (+1 or -1) to
+   the count of first-pass tickets that the second pass of later runs in the persistent
+   four-step kernel waits for.  With +1 the count is never reached; the wait gives up
+   after a short limit and the launch returns with its outputs unfinished.  -1 restores
+   the plan.  MFB_ERR_STATE where n <= 16384. */
+int mfb_test_wait_limit(mfb_plan *p, int delta);
 /* Replaces ap_mf_run_sel (src/matchfilt.c:492-503) in list form: run only the
    output rows rows[0..*nrows) of the block [d0,d0+nd) x [t0,t0+nt), where a row
    is (d-d0)*nt + (t-t0) and the row count lives in DEVICE memory (nrows), so a

@@ -252,3 +252,44 @@ def test_series_ring_grows_beyond_the_plan():
         z = oracle.correlate(D[None], H)
         assert not parity.compare(out["index"][b][None], out["value"][b][None], z, n // 8, 0.0,
                                   (n // 4, 3 * n // 4))
+
+
+def test_run_that_gave_up_spoils_no_later_one():
+    """A dependency wait that runs out (a count that is never reached; no GPU fault) leaves
+    counters and records half-way.  The next runs start from zero all the same: a replay
+    of a graph captured before, which no host call precedes, and a direct run."""
+    import torch
+    mf = _mf()
+    from apogee_b200 import _lib
+    L = _lib.lib()
+    n, nd, nt = 65536, 3, 25
+    g = torch.Generator(device="cuda").manual_seed(4)
+    f = mf.MatchedFilter(n, nd, nt)
+    f.set_data(torch.randn(nd, n, dtype=torch.complex64, device="cuda", generator=g))
+    f.set_templates(torch.randn(nt, n, dtype=torch.complex64, device="cuda", generator=g))
+    nb = 16
+    idx = torch.empty(nd, nt, nb, dtype=torch.int64, device="cuda")
+    val = torch.empty(nd, nt, nb, dtype=torch.complex64, device="cuda")
+    other_i, other_v = torch.empty_like(idx), torch.empty_like(val)
+
+    def run(i, v):
+        f._bind_stream()
+        return L.mfb_run(f._plan, 0, nd, 0, nt, n // nb, 0.0, 0, n, i.data_ptr(), v.data_ptr(), None)
+    _lib.check(run(idx, val))
+    torch.cuda.synchronize()
+    ref_i, ref_v = idx.clone(), val.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        _lib.check(run(idx, val))
+    _lib.check(L.mfb_test_wait_limit(f._plan, 1))
+    _lib.check(run(other_i, other_v))
+    torch.cuda.synchronize()
+    _lib.check(L.mfb_test_wait_limit(f._plan, -1))
+    for _ in range(2):
+        idx.fill_(-7)
+        graph.replay()
+        assert torch.equal(idx, ref_i) and torch.equal(val, ref_v)
+    assert run(idx, val) < 0                     # reports the run that gave up
+    idx.fill_(-7)
+    _lib.check(run(idx, val))
+    assert torch.equal(idx, ref_i) and torch.equal(val, ref_v)
