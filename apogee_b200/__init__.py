@@ -38,6 +38,9 @@ PEAK_DTYPE = np.dtype([("index", "<i8"), ("value", "<c8")])
 #: Transform lengths the device kernels cover.
 SIZES = frozenset(1 << k for k in range(6, 21))
 
+#: Largest n of the kernels whose thread blocks do not wait on one another.
+_SINGLE_CTA = 16384
+
 __all__ = ["MatchedFilter", "HierarchicalFilter", "PEAK_DTYPE", "devices", "Device",
            "UnsupportedSize", "backend", "targets", "set_target", "__version__"]
 
@@ -347,7 +350,7 @@ class MatchedFilter:
             cnt_h = self._buffer("cnt_h", (rows,), torch.int32, pinned=True)
             cnt_h.copy_(cnt_d, non_blocking=True)
         self._after_launch()
-        stream.synchronize()
+        self._finish(stream)
         if raw:
             out = (idx_h.numpy().reshape(nd, nt, nb), val_h.numpy().reshape(nd, nt, nb))
         else:
@@ -358,6 +361,12 @@ class MatchedFilter:
 
     def _after_launch(self):
         pass
+
+    def _finish(self, stream):
+        """Wait for the run; raise if a dependency wait inside it ran out."""
+        stream.synchronize()
+        if self.n > _SINGLE_CTA:
+            _lib.check(_lib.lib().mfb_status(self._plan), "matched filter failed")
 
     def run_device(self, binsize=None, threshold=0.0, window=None, data=None, templates=None):
         """run() without leaving the device: returns torch CUDA tensors
@@ -455,7 +464,7 @@ class MatchedFilter:
         if raw:
             idx = idx_d.cpu().numpy().reshape(nblk, nt, nb)
             val = val_d.cpu().numpy().reshape(nblk, nt, nb)
-            stream.synchronize()
+            self._finish(stream)
             if layout.order is not None:
                 ri = np.empty_like(idx)
                 rv = np.empty_like(val)
@@ -471,7 +480,7 @@ class MatchedFilter:
         rec[:, 1] = val_d.view(torch.int64)
         rec_h = self._buffer("srec_h", (words, 2), torch.int64, pinned=True)
         rec_h.copy_(rec, non_blocking=True)
-        stream.synchronize()
+        self._finish(stream)
         out = np.empty((nblk, nt, nb), PEAK_DTYPE)
         flat = out.view(np.int64).reshape(nblk, nt * nb * 2)
         src = rec_h.numpy().reshape(nblk, nt * nb * 2)
@@ -907,6 +916,11 @@ class HierarchicalFilter(MatchedFilter):
         self._tdirty = True
         self._thr_applied = False
 
+    def _finish(self, stream):
+        stream.synchronize()
+        if self.n > _SINGLE_CTA:
+            _lib.check(_lib.lib().mfb_hier_status(self._hplan), "hierarchical filter failed")
+
     # ---- run ----------------------------------------------------------------
     def _launch(self, records, raw_idx, raw_val, counts, d0, nd, t0, nt, binsize, thr, start, end):
         L = _lib.lib()
@@ -967,7 +981,7 @@ class HierarchicalFilter(MatchedFilter):
         host = self._hostdata.ctypes.data if self._ddirty else None
         fn, args, tail, _ = rep[2]
         _lib.check(fn(self._hplan, *args, host, *tail), "hierarchical filter failed")
-        stream.synchronize()
+        self._finish(stream)
         if host is not None:
             self._ddirty = False
         out, info = self._outview[1], self._outview[2]
@@ -988,7 +1002,7 @@ class HierarchicalFilter(MatchedFilter):
         tail = (rec_d.data_ptr(), tab.data_ptr(), info.data_ptr())
         self._last_args = (fn, args, tail, (rec_d, tab, info))   # the tensors stay alive
         _lib.check(fn(self._hplan, *args, host, *tail), "hierarchical filter failed")
-        stream.synchronize()
+        self._finish(stream)
         if host is not None:
             self._ddirty = False
         key = (tab.data_ptr(), info.data_ptr(), nd, nt, nb)

@@ -71,6 +71,7 @@ SIGNATURES = {
     "mfb_set_stream": (_I, [_P, _P]),
     "mfb_set_packed": (_I, [_P, _I]),
     "mfb_set_cluster": (_I, [_P, _I]),
+    "mfb_status": (_I, [_P]),
     "mfb_test_wait_limit": (_I, [_P, _I]),
     "mfb_set_data": (_I, [_P, _I, _I, _P]),
     "mfb_set_templates": (_I, [_P, _I, _I, _P]),
@@ -95,6 +96,8 @@ SIGNATURES = {
     "mfb_hier_run_records": (_I, [_P, _I, _I, _I, _I, _SZ, _F, _SZ, _SZ, _P, _P]),
     "mfb_hier_run_host": (_I, [_P, _I, _I, _I, _I, _SZ, _F, _SZ, _SZ, _P, _P, _P, _P]),
     "mfb_hier_run_phase": (_I, [_P, _I, _I, _I, _I, _I, _SZ, _F, _SZ, _SZ, _P, _P, _P]),
+    "mfb_hier_status": (_I, [_P]),
+    "mfb_hier_test_wait_limit": (_I, [_P, _I]),
     "mfb_hier_last_triggers": (_I, [_P, _I64P]),
     "mfb_hier_stats": (_I, [_P, _I64P, _I64P]),
     "mfb_hier_config": (_I, [_P, _SZP, _IP]),

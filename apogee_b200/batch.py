@@ -269,11 +269,15 @@ class BatchedFilter:
 
     def wait(self):
         """Synchronise and raise if a dependency wait of the last run ran out."""
+        L = _lib.lib()
+        codes = []
         if self._plan is not None:
-            _lib.check(_lib.lib().mfb_batch_status(self._plan, self._stream()),
-                       "batch run failed")
+            codes.append(L.mfb_batch_status(self._plan, self._stream()))
         else:
             _torch().cuda.current_stream(self._dev).synchronize()
+        # every plan's word is read, so that none is left for the next wait()
+        codes += [L.mfb_status(own["plan"]) for own in self._own]
+        _lib.check(min(codes, default=0), "batch run failed")
 
     def capture(self):
         """Record run() in a CUDA graph (replay() re-launches it)."""

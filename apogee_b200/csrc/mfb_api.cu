@@ -546,7 +546,6 @@ struct LargeScratch {
   float4 *Y = nullptr;      // one allocation: Y, then ctl[0], rec[0], ctl[1], rec[1]
   Large2Ctl *ctl[2] = {nullptr, nullptr};
   uint4 *rec[2] = {nullptr, nullptr};
-  int *err = nullptr;       // from g_err_words
   cudaEvent_t used = nullptr;   // after the last use outside a capture
   int ring = 0;
 };
@@ -597,6 +596,7 @@ struct mfb_plan {
   int cluster = -1;         // mfb_set_cluster's choice; -1: cluster_mode's rule
   int hold = 0;             // mfb_test_wait_limit
   bool own_capture = false; // a capture whose graph this library launches
+  int *err = nullptr;       // mapped host word (g_err_words), set by a run that gave up
 };
 
 struct DeviceGuard {
@@ -662,6 +662,7 @@ extern "C" int mfb_destroy(mfb_plan *p) {
   cudaFree(p->sspec);
   large_free(p->ls);
   for (LargeScratch &s : p->ls_old) large_free(s);
+  give_err_word(p->err);
   delete p;
   return MFB_OK;
 }
@@ -746,15 +747,17 @@ static size_t large_ctl_bytes(int ring) {
 static void large_free(LargeScratch &s) {
   cudaFree(s.Y);
   if (s.used) cudaEventDestroy(s.used);
-  give_err_word(s.err);
   s = LargeScratch();
+}
+// Whether a run of the plan gave up since the last look.
+static int large_status(const mfb_plan *p) {
+  if (!p->err || !*(volatile int *)p->err) return MFB_OK;
+  *(volatile int *)p->err = 0;
+  return fail(MFB_ERR_CUDA, "a run at n=%zu timed out on a dependency; its outputs are invalid", p->n);
 }
 static int large_scratch(mfb_plan *p, long long pairs) {
   LargeScratch &cur = p->ls;
-  if (cur.ring && *(volatile int *)cur.err) {   // an earlier launch gave up half-way
-    *cur.err = 0;
-    return fail(MFB_ERR_CUDA, "an earlier run at n=%zu timed out on a dependency; its outputs are invalid", p->n);
-  }
+  if (int r = large_status(p)) return r;   // an earlier run gave up
   pairs = std::max(pairs, (long long)p->nd * p->nt);
   const int per = (p->lc->units_a + p->lc->units_b) / LARGE2_GROUP;
   const long long most = large2_delay(p->lc->grid2, per) * 5 / 2;
@@ -771,7 +774,7 @@ static int large_scratch(mfb_plan *p, long long pairs) {
     }
     e = cudaMemset(s.ctl[0], 0, rest);
   }
-  if (e == cudaSuccess) e = take_err_word(&s.err);
+  if (e == cudaSuccess && !p->err) e = take_err_word(&p->err);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s.used, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();   // before any stream uses them
   if (e != cudaSuccess) {
@@ -863,7 +866,7 @@ static int run_large(mfb_plan *p, int d0, int nd, int t0, int nt, const int32_t 
   const int foreign = capturing(p->stream) && !p->own_capture;
   g.rec = p->ls.rec[foreign];
   g.ctl = p->ls.ctl[foreign];
-  CUDA_TRY(cudaHostGetDevicePointer((void **)&g.err, p->ls.err, 0));
+  CUDA_TRY(cudaHostGetDevicePointer((void **)&g.err, p->err, 0));
   g.ring = p->ls.ring;
   g.spin = p->hold ? 1u << 14 : LARGE2_SPIN;
   g.hold = p->hold;
@@ -907,6 +910,10 @@ static int run_impl(mfb_plan *p, int d0, int nd, int t0, int nt, size_t binsize,
   return MFB_OK;
 }
 
+extern "C" int mfb_status(mfb_plan *p) {
+  if (!p) return fail(MFB_ERR_ARG, "null plan");
+  return large_status(p);
+}
 extern "C" int mfb_test_wait_limit(mfb_plan *p, int delta) {
   if (!p) return fail(MFB_ERR_ARG, "null plan");
   if (!is_large(p->n)) return fail(MFB_ERR_STATE, "n=%zu has no pass to hold back", p->n);
@@ -1694,7 +1701,8 @@ extern "C" int mfb_hier_run_host(mfb_hplan *h, int d0, int nd, int t0, int nt, s
     }
   }
   const LargeScratch &ls = h->full->ls;
-  if (ls.ring && *(volatile int *)ls.err) graphable = false;   // the direct run reports it
+  r = large_status(h->full);   // an earlier run gave up
+  if (r) return r;
   mfb_hplan::RunKey key;
   memset(&key, 0, sizeof key);
   key.d0 = d0; key.nd = nd; key.t0 = t0; key.nt = nt;
@@ -1798,13 +1806,29 @@ extern "C" int mfb_hier_coarse_values(mfb_hplan *h, int d0, int nd, int t0, int 
   return MFB_OK;
 }
 
+// After a synchronisation: whether a coarse pass or a refine gave up.
+static int hier_status(mfb_hplan *h) {
+  if (tc_coarse_check(h->tc)) return fail(MFB_ERR_CUDA, "%s", tc_coarse_error());
+  return large_status(h->full);
+}
+
+extern "C" int mfb_hier_status(mfb_hplan *h) {
+  if (!h) return fail(MFB_ERR_ARG, "null plan");
+  return large_status(h->full);
+}
+extern "C" int mfb_hier_test_wait_limit(mfb_hplan *h, int delta) {
+  if (!h) return fail(MFB_ERR_ARG, "null plan");
+  hier_drop_graph(h);
+  return mfb_test_wait_limit(h->full, delta);
+}
+
 extern "C" int mfb_hier_last_triggers(mfb_hplan *h, int64_t *triggers) {
   if (!h || !triggers) return fail(MFB_ERR_ARG, "null argument");
   DeviceGuard dg(h->device);
   int32_t c = 0;
   CUDA_TRY(cudaMemcpyAsync(&c, h->fire_count, sizeof c, cudaMemcpyDeviceToHost, h->full->stream));
   CUDA_TRY(cudaStreamSynchronize(h->full->stream));
-  if (tc_coarse_check(h->tc)) return fail(MFB_ERR_CUDA, "%s", tc_coarse_error());
+  if (int r = hier_status(h)) return r;
   *triggers = c;
   return MFB_OK;
 }
@@ -1815,7 +1839,7 @@ extern "C" int mfb_hier_stats(mfb_hplan *h, int64_t *pairs, int64_t *triggers) {
   unsigned long long tot = 0;
   CUDA_TRY(cudaMemcpyAsync(&tot, h->trig_total, sizeof tot, cudaMemcpyDeviceToHost, h->full->stream));
   CUDA_TRY(cudaStreamSynchronize(h->full->stream));
-  if (tc_coarse_check(h->tc)) return fail(MFB_ERR_CUDA, "%s", tc_coarse_error());
+  if (int r = hier_status(h)) return r;
   if (pairs) *pairs = h->pairs;
   if (triggers) *triggers = (int64_t)tot;
   return MFB_OK;

@@ -98,6 +98,11 @@ int mfb_set_packed(mfb_plan *p, int on);
    of up to 64 pairs and captured runs, mode 0 for larger blocks (1.7x faster
    at 1024 pairs); at 65536 mode 0. */
 int mfb_set_cluster(mfb_plan *p, int mode);
+/* MFB_ERR_CUDA, once, if a dependency wait inside a run of this plan ran out (the
+   outputs of that run are then not valid).  Reads a host word: call it after
+   synchronising with the run, also after replays of a graph it was captured in.  The
+   plan's next call that uses the persistent four-step kernel reports it otherwise. */
+int mfb_status(mfb_plan *p);
 /* Failure-detection test hook, as mfb_batch_test_wait_limit: adds delta (+1 or -1) to
    the count of first-pass tickets that the second pass of later runs in the persistent
    four-step kernel waits for.  With +1 the count is never reached; the wait gives up
@@ -199,6 +204,11 @@ int mfb_hier_run_host(mfb_hplan *p, int d0, int nd, int t0, int nt, size_t binsi
 int mfb_hier_run_phase(mfb_hplan *p, int phase, int d0, int nd, int t0, int nt, size_t binsize,
                        float threshold, size_t start, size_t end, int64_t *idx, void *val,
                        int32_t *counts);
+/* mfb_status for the plan's refine; mfb_hier_last_triggers and mfb_hier_stats look
+   at it, and at the coarse pass, by themselves. */
+int mfb_hier_status(mfb_hplan *p);
+/* mfb_test_wait_limit for the plan's refine. */
+int mfb_hier_test_wait_limit(mfb_hplan *p, int delta);
 /* Survivors of the last mfb_hier_run (synchronises the plan's stream). */
 int mfb_hier_last_triggers(mfb_hplan *p, int64_t *triggers);
 /* Replaces ap_hmf_run_series (src/hmf.c:158-220): runs of blocks with equal

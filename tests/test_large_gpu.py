@@ -293,3 +293,58 @@ def test_run_that_gave_up_spoils_no_later_one():
     idx.fill_(-7)
     _lib.check(run(idx, val))
     assert torch.equal(idx, ref_i) and torch.equal(val, ref_v)
+
+
+def test_run_that_gave_up_is_reported():
+    """run(), run_series(), a hierarchical run (direct, then its replayed graph) and a
+    batch's wait() raise for the very run whose dependency wait ran out, and the next
+    run is right."""
+    mf = _mf()
+    from apogee_b200 import _lib
+    from apogee_b200.batch import BatchedFilter, Job
+    L = _lib.lib()
+    n, nd, nt = 65536, 2, 9
+    rng = np.random.default_rng(8)
+    D, H = noise(rng, (nd, n)), noise(rng, (nt, n))
+    x = noise(rng, 2 * n)
+
+    f = mf.MatchedFilter(n, nd, nt)
+    f.set_data(D)
+    f.set_templates(H)
+    st, lo, hi = np.array([0, n // 2]), np.zeros(2, int), np.full(2, n)
+    def series():
+        return f.run_series(x, st, lo, hi, binsize=n // 4)
+    def flat():
+        f.set_data(D)
+        return f.run(binsize=n // 16).copy()
+    h = mf.HierarchicalFilter(n, nd, nt, band=8192, coarse="fp32")
+    h.set_coarse_threshold(0.0)
+    h.set_data(D)
+    h.set_templates(H)
+    def hier():
+        return h.run(binsize=n // 16).copy()
+    for call, plan, hook in ((flat, f._plan, L.mfb_test_wait_limit), (series, f._plan, L.mfb_test_wait_limit),
+                             (hier, None, L.mfb_hier_test_wait_limit)):
+        ref = call()
+        p = plan if plan is not None else h._hplan
+        _lib.check(hook(p, 1))
+        for _ in range(3):                       # hier: direct, captured, replayed
+            with pytest.raises(RuntimeError, match="timed out on a dependency"):
+                call()
+        _lib.check(hook(p, -1))
+        for _ in range(3):
+            np.testing.assert_array_equal(call(), ref)
+
+    bf = BatchedFilter([Job(H, data=D, binsize=n // 16)], tune={n: {"dedicated": True}})
+    bf.run()
+    bf.wait()
+    ref = bf.result(0).copy()
+    _lib.check(L.mfb_test_wait_limit(bf._own[0]["plan"], 1))
+    bf.run()
+    with pytest.raises(RuntimeError, match="timed out on a dependency"):
+        bf.wait()
+    _lib.check(L.mfb_test_wait_limit(bf._own[0]["plan"], -1))
+    bf.run()
+    bf.wait()
+    np.testing.assert_array_equal(bf.result(0), ref)
+    bf.close()
