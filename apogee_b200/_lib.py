@@ -67,6 +67,7 @@ SIGNATURES = {
     "mfb_batch_info": (_I, [_P, _I64P, _IP, _IP, _IP, _SZP]),
     "mfb_batch_destroy": (_I, [_P]),
     "mfb_create": (_I, [_PP, _SZ, _I, _I, _I]),
+    "mfb_create_sharing": (_I, [_PP, _SZ, _I, _I, _P]),
     "mfb_destroy": (_I, [_P]),
     "mfb_set_stream": (_I, [_P, _P]),
     "mfb_set_packed": (_I, [_P, _I]),

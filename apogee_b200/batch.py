@@ -214,8 +214,13 @@ class BatchedFilter:
         torch = _torch()
         L = _lib.lib()
         plan = ctypes.c_void_p()
-        _lib.check(L.mfb_create(ctypes.byref(plan), j.n, j.nd, j.nt, self.device.index),
-                   "batch job plan failed")
+        # the own launches follow one another: one scratch serves those of large n
+        first = next((o["plan"] for o in self._own if self.jobs[o["index"]].n > 16384), None)
+        if j.n > 16384 and first is not None:
+            rc = L.mfb_create_sharing(ctypes.byref(plan), j.n, j.nd, j.nt, first)
+        else:
+            rc = L.mfb_create(ctypes.byref(plan), j.n, j.nd, j.nt, self.device.index)
+        _lib.check(rc, "batch job plan failed")
         own = {"index": i, "plan": plan, "keep": []}
         try:
             _lib.check(L.mfb_set_stream(plan, self._stream()))

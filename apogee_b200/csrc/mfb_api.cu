@@ -538,16 +538,21 @@ extern "C" size_t mfb_nbins(size_t n, size_t binsize, size_t start, size_t end) 
 }
 
 // ---------------------------------------------------------------- flat plan
-// large2_kernel's scratch: rows, candidate records and counters (both zero
-// between launches) of `ring` items, and the mapped error word.  Counters and records
-// are there twice, [0] for runs that follow one another and [1] for runs captured by
-// a caller, whose order nobody here knows.
+// large2_kernel's scratch, of one plan or shared (mfb_share_scratch): rows, and counters
+// and candidate records.  The latter are zero between launches, whatever the plan
+// and its layout of them, and are there twice: [0] for runs that follow one another and
+// [1] for runs captured by a caller, whose order nobody here knows.
 struct LargeScratch {
-  float4 *Y = nullptr;      // one allocation: Y, then ctl[0], rec[0], ctl[1], rec[1]
-  Large2Ctl *ctl[2] = {nullptr, nullptr};
-  uint4 *rec[2] = {nullptr, nullptr};
-  cudaEvent_t used = nullptr;   // after the last use outside a capture
-  int ring = 0;
+  int device;
+  char *rows = nullptr, *state[2] = {nullptr, nullptr};   // state: one allocation
+  size_t rows_bytes = 0, state_bytes = 0;                 // state_bytes: each
+  size_t refused = SIZE_MAX;                              // rows the device had no room for
+  cudaEvent_t used = nullptr;         // after the last use outside a capture
+  unsigned generation = 0;            // counts reallocations
+  bool captured = false;              // a caller's graph may hold the present addresses
+  std::vector<char *> kept;           // ... or these, outgrown since
+  explicit LargeScratch(int dev) : device(dev) {}
+  ~LargeScratch();
 };
 
 // Mapped host words for the error flags of large2_kernel launches, a page at a
@@ -588,10 +593,9 @@ struct mfb_plan {
   int starts_cap = 0;
   float2 *sspec = nullptr;
   int sspec_rows = 0;
-  // large-n state: constants and scratch (with rings outgrown by later runs)
+  // large-n state: constants and scratch (empty until the first run that uses it)
   LargeConst *lc = nullptr;
-  LargeScratch ls;
-  std::vector<LargeScratch> ls_old;
+  std::shared_ptr<LargeScratch> ls;
   int packed = 1;           // use flatw_kernel where it applies (mfb_set_packed)
   int cluster = -1;         // mfb_set_cluster's choice; -1: cluster_mode's rule
   int hold = 0;             // mfb_test_wait_limit
@@ -608,10 +612,22 @@ struct DeviceGuard {
   ~DeviceGuard() { if (prev >= 0 && prev != dev_) cudaSetDevice(prev); }
 };
 
-static int large_scratch(mfb_plan *p, long long pairs);
-extern "C" int mfb_destroy(mfb_plan *p);
+LargeScratch::~LargeScratch() {
+  DeviceGuard dg(device);
+  cudaFree(rows);
+  cudaFree(state[0]);
+  for (char *k : kept) cudaFree(k);
+  if (used) cudaEventDestroy(used);
+}
 
-extern "C" int mfb_create(mfb_plan **out, size_t n, int ndata, int ntmpl, int device) {
+static int large_scratch(mfb_plan *p, long long pairs, size_t nb);
+extern "C" int mfb_destroy(mfb_plan *p);
+constexpr long long CLUSTER_PAIRS = 64;   // see cluster_mode
+
+// scratch: the large-n scratch to use, or nullptr for the plan's own; eager: allocate
+// what a run without an allocation needs.
+static int create_plan(mfb_plan **out, size_t n, int ndata, int ntmpl, int device,
+                       const std::shared_ptr<LargeScratch> &scratch, bool eager) {
   if (!out) return fail(MFB_ERR_ARG, "null output handle");
   *out = nullptr;
   if (ndata < 1 || ntmpl < 1) return fail(MFB_ERR_ARG, "ndata and ntemplates must be >= 1");
@@ -641,16 +657,24 @@ extern "C" int mfb_create(mfb_plan **out, size_t n, int ndata, int ntmpl, int de
   cudaMemset(p->data, 0, (size_t)ndata * n * sizeof(float2));
   cudaMemset(p->tmpl, 0, (size_t)ntmpl * n * sizeof(float2));
   CUDA_TRY(cudaDeviceSynchronize());
-  if (n == 32768) {
-    // runs at this length never allocate (they may be captured at the first call)
-    r = large_scratch(p, (long long)ndata * ntmpl);
+  if (is_large(n)) p->ls = scratch ? scratch : std::make_shared<LargeScratch>(device);
+  if (eager && n == 32768 && (long long)ndata * ntmpl > CLUSTER_PAIRS) {
+    // runs at this length do not allocate (smaller blocks, lists and captured runs take
+    // the cluster kernel, which has no scratch)
+    r = large_scratch(p, (long long)ndata * ntmpl, 1);
     if (r != MFB_OK) { mfb_destroy(p); return r; }
   }
   *out = p;
   return MFB_OK;
 }
 
-static void large_free(LargeScratch &s);
+extern "C" int mfb_create(mfb_plan **out, size_t n, int ndata, int ntmpl, int device) {
+  return create_plan(out, n, ndata, ntmpl, device, nullptr, true);
+}
+extern "C" int mfb_create_sharing(mfb_plan **out, size_t n, int ndata, int ntmpl, mfb_plan *owner) {
+  if (!owner) return fail(MFB_ERR_ARG, "null plan");
+  return create_plan(out, n, ndata, ntmpl, owner->device, owner->ls, true);
+}
 
 extern "C" int mfb_destroy(mfb_plan *p) {
   if (!p) return MFB_OK;
@@ -660,8 +684,7 @@ extern "C" int mfb_destroy(mfb_plan *p) {
   cudaFree(p->tmpl);
   cudaFree(p->starts_dev);
   cudaFree(p->sspec);
-  large_free(p->ls);
-  for (LargeScratch &s : p->ls_old) large_free(s);
+  p->ls.reset();
   give_err_word(p->err);
   delete p;
   return MFB_OK;
@@ -734,55 +757,86 @@ static bool capturing(cudaStream_t s) {
   }
   return cs != cudaStreamCaptureStatusNone;
 }
-// Scratch of the large-n kernel, allocated on first use: a ring of item slots
-// (two pairs each), two and a half times the kernel's delay between an item's two
-// passes, or as many as the run has items if those are fewer (two at least).  A run
-// with more items (run_series over many blocks) gets a larger ring; the smaller
-// one is kept until the plan goes, because captured graphs may hold it.
-static size_t large_rec_bytes(int ring) { return (size_t)ring * 2 * LARGE_MAX_BINS * sizeof(uint4); }
+// Scratch of the large-n kernel, allocated on first use: a ring of item slots (two
+// pairs each), two and a half times the kernel's delay between an item's two passes, or as
+// many as the run has items if those are fewer (two at least), and records for the run's
+// bins.  A run that needs more (run_series over many blocks, more bins) gets more; what it
+// outgrows is freed, unless a caller's graph may hold it.  Under capture nothing is
+// allocated: any ring of two slots or more will do.
 static size_t large_ctl_bytes(int ring) {
   return (sizeof(Large2Ctl) + (size_t)ring * 3 * sizeof(unsigned) + 15) & ~(size_t)15;
 }
-
-static void large_free(LargeScratch &s) {
-  cudaFree(s.Y);
-  if (s.used) cudaEventDestroy(s.used);
-  s = LargeScratch();
+static size_t large_state_bytes(int ring, size_t nb) {
+  return large_ctl_bytes(ring) + (size_t)ring * 2 * nb * sizeof(uint4);
 }
+static int large_want(const mfb_plan *p, long long pairs) {
+  const int per = (p->lc->units_a + p->lc->units_b) / LARGE2_GROUP;
+  const long long most = large2_delay(p->lc->grid2, per) * 5 / 2;
+  return (int)std::max<long long>(2, std::min((pairs + 1) / 2, most));
+}
+// Item slots of a run: what it wants, as far as the scratch has room.
+static int large_ring(const mfb_plan *p, long long pairs, size_t nb) {
+  const LargeScratch &s = *p->ls;
+  int ring = (int)std::min<size_t>(large_want(p, pairs), s.rows_bytes / (p->n * sizeof(float4)));
+  if (large_state_bytes(ring, nb) > s.state_bytes)
+    ring = (int)((s.state_bytes - sizeof(Large2Ctl) - 16) / (3 * sizeof(unsigned) + 2 * nb * sizeof(uint4)));
+  return ring;
+}
+
 // Whether a run of the plan gave up since the last look.
 static int large_status(const mfb_plan *p) {
   if (!p->err || !*(volatile int *)p->err) return MFB_OK;
   *(volatile int *)p->err = 0;
   return fail(MFB_ERR_CUDA, "a run at n=%zu timed out on a dependency; its outputs are invalid", p->n);
 }
-static int large_scratch(mfb_plan *p, long long pairs) {
-  LargeScratch &cur = p->ls;
+// Keeps or frees an outgrown allocation.
+static void large_drop(LargeScratch &s, char *block) {
+  if (s.captured && block) { s.kept.push_back(block); return; }
+  cudaDeviceSynchronize();
+  cudaFree(block);
+}
+static int large_scratch(mfb_plan *p, long long pairs, size_t nb) {
   if (int r = large_status(p)) return r;   // an earlier run gave up
-  pairs = std::max(pairs, (long long)p->nd * p->nt);
-  const int per = (p->lc->units_a + p->lc->units_b) / LARGE2_GROUP;
-  const long long most = large2_delay(p->lc->grid2, per) * 5 / 2;
-  const int ring = (int)std::max<long long>(2, std::min((pairs + 1) / 2, most));
-  if (cur.ring >= ring) return MFB_OK;
-  LargeScratch s;
-  s.ring = ring;
-  const size_t rows = (size_t)ring * p->n * sizeof(float4), rest = large_rec_bytes(ring) + large_ctl_bytes(ring);
-  cudaError_t e = cudaMalloc(&s.Y, rows + 2 * rest);
-  if (e == cudaSuccess) {
-    for (int i = 0; i < 2; i++) {
-      s.ctl[i] = reinterpret_cast<Large2Ctl *>(reinterpret_cast<char *>(s.Y) + rows + i * rest);
-      s.rec[i] = reinterpret_cast<uint4 *>(reinterpret_cast<char *>(s.ctl[i]) + large_ctl_bytes(ring));
-    }
-    e = cudaMemset(s.ctl[0], 0, rest);
-  }
+  LargeScratch &s = *p->ls;
+  const size_t slot = p->n * sizeof(float4);
+  if (capturing(p->stream) && s.rows_bytes >= 2 * slot && s.state_bytes) return MFB_OK;
+  const int ring = large_want(p, std::max(pairs, (long long)p->nd * p->nt));
+  size_t rows = ring * slot;
+  while (rows >= s.refused && rows > 2 * slot) rows = std::max(2 * slot, rows / 2);
+  cudaError_t e = cudaSuccess;
+  if (!s.used) e = cudaEventCreateWithFlags(&s.used, cudaEventDisableTiming);
   if (e == cudaSuccess && !p->err) e = take_err_word(&p->err);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s.used, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaDeviceSynchronize();   // before any stream uses them
+  if (e == cudaSuccess && s.rows_bytes < rows) {
+    large_drop(s, s.rows);
+    s.rows = nullptr;
+    s.rows_bytes = 0;
+    s.generation++;
+    while ((e = cudaMalloc(&s.rows, rows)) == cudaErrorMemoryAllocation && rows > 2 * slot) {
+      cudaGetLastError();             // a shorter ring is slower, no more
+      s.refused = rows;
+      rows = std::max(2 * slot, rows / 2);
+    }
+    if (e == cudaSuccess) s.rows_bytes = rows;
+  }
+  // records: as many as the bins ask for, two slots of LARGE_MAX_BINS at least
+  const size_t state = std::max(large_state_bytes(ring, nb), large_state_bytes(2, LARGE_MAX_BINS));
+  if (e == cudaSuccess && s.state_bytes < state) {
+    large_drop(s, s.state[0]);
+    s.state[0] = s.state[1] = nullptr;
+    s.state_bytes = 0;
+    s.generation++;
+    e = cudaMalloc(&s.state[0], 2 * state);
+    if (e == cudaSuccess) {
+      s.state[1] = s.state[0] + state;
+      s.state_bytes = state;
+      e = cudaMemset(s.state[0], 0, 2 * state);
+      if (e == cudaSuccess) e = cudaDeviceSynchronize();   // before any stream uses it
+    }
+  }
   if (e != cudaSuccess) {
-    large_free(s);
+    cudaGetLastError();
     return fail(MFB_ERR_CUDA, "large-n scratch for n=%zu: %s", p->n, cudaGetErrorString(e));
   }
-  if (cur.ring) p->ls_old.push_back(cur);
-  cur = s;
   return MFB_OK;
 }
 // Runs of one plan enqueued on different streams share its scratch: each waits
@@ -791,13 +845,13 @@ static int large_scratch(mfb_plan *p, long long pairs) {
 // another run of the plan.  If it does, both runs' outputs are wrong, but no later
 // run's: a caller's captures have counters of their own, zeroed in front of each launch.
 static cudaError_t scratch_begin(const mfb_plan *p) {
-  return capturing(p->stream) ? cudaSuccess : cudaStreamWaitEvent(p->stream, p->ls.used, 0);
+  return capturing(p->stream) ? cudaSuccess : cudaStreamWaitEvent(p->stream, p->ls->used, 0);
 }
 static cudaError_t scratch_end(const mfb_plan *p) {
-  return capturing(p->stream) ? cudaSuccess : cudaEventRecord(p->ls.used, p->stream);
+  return capturing(p->stream) ? cudaSuccess : cudaEventRecord(p->ls->used, p->stream);
 }
 // Series blocks that fit the scratch.
-static int large_rows(const mfb_plan *p) { return p->ls.ring * 2; }
+static int large_rows(const mfb_plan *p) { return (int)(p->ls->rows_bytes / (p->n * sizeof(float2))); }
 
 // The cluster kernel's geometry for a run (1 or 2), or 0 for large2_kernel.  At
 // n = 32768, unless mfb_set_cluster says otherwise, lists and dense runs of up to
@@ -807,7 +861,6 @@ static int large_rows(const mfb_plan *p) { return p->ls.ring * 2; }
 // 38 us, 1024 pairs 152 against 258).  A captured run at that length keeps to the
 // cluster kernel, which has no scratch: its graph may run beside other runs of the
 // plan.
-constexpr long long CLUSTER_PAIRS = 64;
 static int cluster_mode(const mfb_plan *p, bool listed, long long pairs) {
   int mode = p->cluster;
   if (mode < 0)
@@ -826,7 +879,7 @@ static int run_large(mfb_plan *p, int d0, int nd, int t0, int nt, const int32_t 
   const LargeConst &c = *p->lc;
   const int cl = cluster_mode(p, list != nullptr, (long long)nd * nt);
   if (!cl) {
-    int sr = large_scratch(p, (long long)nd * nt);
+    int sr = large_scratch(p, (long long)nd * nt, nb);
     if (sr) return sr;
   }
   if (end > p->n) end = p->n;
@@ -858,23 +911,24 @@ static int run_large(mfb_plan *p, int d0, int nd, int t0, int nt, const int32_t 
     return MFB_OK;
   }
   Large2Args g;
+  memset(&g, 0, sizeof g);
   g.a = a;
   g.tw1 = c.c1->twid2;
   g.tw2 = c.c2->twid2;
   g.anchors = c.anchors;
-  g.Y = p->ls.Y;
+  g.Y = reinterpret_cast<float4 *>(p->ls->rows);
   const int foreign = capturing(p->stream) && !p->own_capture;
-  g.rec = p->ls.rec[foreign];
-  g.ctl = p->ls.ctl[foreign];
+  if (foreign) p->ls->captured = true;
+  g.ring = large_ring(p, list ? LLONG_MAX - 1 : a.total, nb);
+  g.ctl = reinterpret_cast<Large2Ctl *>(p->ls->state[foreign]);
+  g.rec = reinterpret_cast<uint4 *>(p->ls->state[foreign] + large_ctl_bytes(g.ring));
   CUDA_TRY(cudaHostGetDevicePointer((void **)&g.err, p->err, 0));
-  g.ring = p->ls.ring;
   g.spin = p->hold ? 1u << 14 : LARGE2_SPIN;
   g.hold = p->hold;
   const long long items = (a.total + 1) / 2;
-  const size_t records = (size_t)(list ? g.ring : std::min<long long>(items, g.ring)) * 2 * nb * sizeof(uint4);
   const int grid = (int)std::min<long long>(c.grid2, std::max<long long>(1, items * c.units_a));
   CUDA_TRY(scratch_begin(p));
-  if (foreign) CUDA_TRY(cudaMemsetAsync(g.ctl, 0, large_ctl_bytes(g.ring) + records, p->stream));
+  if (foreign) CUDA_TRY(cudaMemsetAsync(g.ctl, 0, large_state_bytes(g.ring, nb), p->stream));
   CUDA_TRY(launch_large2(c, g, grid, p->stream));
   CUDA_TRY(scratch_end(p));
   return MFB_OK;
@@ -1010,14 +1064,14 @@ extern "C" int mfb_forward(mfb_plan *p, const void *series, size_t nseries,
     return fail(MFB_ERR_ARG, "invalid forward-transform arguments");
   DeviceGuard dg(p->device);
   if (is_large(p->n)) {
-    int sr = large_scratch(p, std::max<long long>(nblocks, (long long)p->nd * p->nt));
+    int sr = large_scratch(p, nblocks, 1);
     if (sr) return sr;
     const LargeConst &c = *p->lc;
     LargeArgs a;
     memset(&a, 0, sizeof a);
     a.n = (int)p->n; a.N1 = c.N1; a.N2 = c.N2;
     a.total = nblocks;
-    a.Y = reinterpret_cast<float2 *>(p->ls.Y);
+    a.Y = reinterpret_cast<float2 *>(p->ls->rows);
     a.tw1 = c.c1->twid; a.tw2 = c.c2->twid;
     a.tw_hi = c.tw_hi; a.tw_lo = c.tw_lo; a.lo_bits = c.lo_bits;
     LargeFwd f;
@@ -1091,6 +1145,10 @@ extern "C" int mfb_run_series(mfb_plan *p, const void *series, size_t nseries,
     CUDA_TRY(cudaMalloc(&p->sspec, (size_t)cap * row_bytes));
     p->sspec_rows = cap;
   }
+  if (is_large(p->n)) {   // the largest group's scratch at once
+    int r = large_scratch(p, (long long)cap * nt, std::min<size_t>(nb0, LARGE_MAX_BINS));
+    if (r) return r;
+  }
   // Groups of consecutive equal windows, at most `cap` blocks each.
   for (int b0 = 0; b0 < nblocks;) {
     int g = 1;
@@ -1160,7 +1218,8 @@ struct mfb_hplan {
     int d0, nd, t0, nt, same;
     uint32_t thr_bits, gate_bits;
     size_t binsize, start, end;
-    const void *data, *records, *table, *info, *scratch;
+    const void *data, *records, *table, *info;
+    unsigned scratch, pad;
   };
   RunKey last_key, graph_key;
   bool last_valid = false;
@@ -1184,7 +1243,7 @@ extern "C" int mfb_hier_create(mfb_hplan **out, size_t n, int ndata, int ntmpl, 
       coarse_kind != MFB_COARSE_FP16X3)
     return fail(MFB_ERR_ARG, "unknown coarse kind %d", coarse_kind);
   mfb_plan *full = nullptr;
-  int r = mfb_create(&full, n, ndata, ntmpl, device);
+  int r = create_plan(&full, n, ndata, ntmpl, device, nullptr, false);   // lists only
   if (r) return r;
   DeviceGuard dg(device);
   mfb_hplan *h = new mfb_hplan;
@@ -1658,9 +1717,10 @@ static uint32_t float_bits(float x) {
 // Launches the captured run, ordered with the plan's other runs as a direct run is.
 static cudaError_t launch_hier_graph(mfb_hplan *h, cudaGraphExec_t x) {
   const mfb_plan *p = h->full;
-  cudaError_t e = p->ls.ring ? scratch_begin(p) : cudaSuccess;
+  const bool ordered = p->ls && p->ls->used;
+  cudaError_t e = ordered ? scratch_begin(p) : cudaSuccess;
   if (e == cudaSuccess) e = cudaGraphLaunch(x, p->stream);
-  return e == cudaSuccess && p->ls.ring ? scratch_end(p) : e;
+  return e == cudaSuccess && ordered ? scratch_end(p) : e;
 }
 
 extern "C" int mfb_hier_run_host(mfb_hplan *h, int d0, int nd, int t0, int nt, size_t binsize,
@@ -1700,7 +1760,6 @@ extern "C" int mfb_hier_run_host(mfb_hplan *h, int d0, int nd, int t0, int nt, s
       graphable = false;
     }
   }
-  const LargeScratch &ls = h->full->ls;
   r = large_status(h->full);   // an earlier run gave up
   if (r) return r;
   mfb_hplan::RunKey key;
@@ -1712,7 +1771,7 @@ extern "C" int mfb_hier_run_host(mfb_hplan *h, int d0, int nd, int t0, int nt, s
   key.gate_bits = float_bits(h->cal_thr);
   key.binsize = binsize; key.start = start; key.end = end;
   key.data = data; key.records = records; key.table = dtab; key.info = dinfo;
-  key.scratch = ls.Y;   // a graph goes with the scratch it was captured on
+  if (h->full->ls) key.scratch = h->full->ls->generation;   // a graph goes with its scratch
   if (graphable && h->graph && memcmp(&key, &h->graph_key, sizeof key) == 0) {
     CUDA_TRY(launch_hier_graph(h, h->graph));
     h->pairs += (long long)nd * nt;

@@ -56,6 +56,16 @@ typedef struct mfb_hplan mfb_hplan;
    power of two, 64 .. 2^20 (above 16384 a four-step split); device is a
    CUDA ordinal.  *out = NULL on error. */
 int mfb_create(mfb_plan **out, size_t n, int ndata, int ntmpl, int device);
+/* mfb_create on owner's device, for plans whose runs follow one another: the new plan
+   uses owner's scratch for large n instead of one of its own.  Runs on different streams
+   are ordered; the two plans must not be used from two threads at once.
+   That scratch (of the persistent four-step kernel: n >= 65536, and n = 32768 in dense
+   blocks of more than 64 pairs) is allocated by mfb_create at n = 32768 and by a plan's
+   first run above, and grown by a run that needs more: rows of the pairs in flight, at
+   most 205 MiB (240 MiB at n = 2^20), and 64 bytes per bin of those pairs (0.4 MB at 16
+   bins and n = 65536, 27 MB at 1024).  A device with less room gets less, at some cost
+   in speed. */
+int mfb_create_sharing(mfb_plan **out, size_t n, int ndata, int ntmpl, mfb_plan *owner);
 /* Replaces ap_mf_destroy (src/matchfilt.c:135-146). */
 int mfb_destroy(mfb_plan *p);
 /* Stream for every later enqueue on this plan (a cudaStream_t, NULL = legacy). */

@@ -348,3 +348,165 @@ def test_run_that_gave_up_is_reported():
     bf.wait()
     np.testing.assert_array_equal(bf.result(0), ref)
     bf.close()
+
+
+def _held(make):
+    """Device bytes that `make` leaves allocated, and what it returns."""
+    import torch
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    out = make()
+    torch.cuda.synchronize()
+    return free - torch.cuda.mem_get_info()[0], out
+
+
+def _plan(n, nd, nt, owner=None):
+    import ctypes
+    from apogee_b200 import _lib
+    h = ctypes.c_void_p()
+    if owner is None:
+        _lib.check(_lib.lib().mfb_create(ctypes.byref(h), n, nd, nt, 0))
+    else:
+        _lib.check(_lib.lib().mfb_create_sharing(ctypes.byref(h), n, nd, nt, owner))
+    return h
+
+
+def _run_plan(p, n, nd, nt, nb):
+    """One dense run on zeroed rows; its (idx, val)."""
+    import torch
+    from apogee_b200 import _lib
+    L = _lib.lib()
+    idx = torch.empty(nd * nt * nb, dtype=torch.int64, device="cuda")
+    val = torch.empty(nd * nt * nb, dtype=torch.complex64, device="cuda")
+    _lib.check(L.mfb_set_stream(p, torch.cuda.current_stream().cuda_stream))
+    _lib.check(L.mfb_run(p, 0, nd, 0, nt, n // nb, 0.0, 0, n, idx.data_ptr(), val.data_ptr(), None))
+    return idx, val
+
+
+def test_scratch_is_what_the_runs_need():
+    """Nothing is held for lists and small blocks at n = 32768; records follow the bins; a
+    scratch that is outgrown is given back; a plan made to share holds none."""
+    import torch
+    from apogee_b200 import _lib
+    import apogee_b200 as mf
+    L = _lib.lib()
+    MB = 1 << 20
+    n = 32768
+    rows = lambda nd, nt: (nd + nt) * n * 8
+    _run_plan(_plan(n, 1, 1), n, 1, 1, 16)                       # constants of this length
+    held, p = _held(lambda: _plan(n, 2, 32))
+    assert held <= rows(2, 32) + 4 * MB
+    L.mfb_destroy(p)
+    held, h = _held(lambda: mf.HierarchicalFilter(n, 2, 300, band=16384, coarse="fp32"))
+    held_p, p = _held(lambda: _plan(n, 2, 300))
+    assert held_p <= rows(2, 300) + 213 * MB                     # 203.5 MiB of rows and few records
+    L.mfb_destroy(p)
+    del h
+
+    n = 65536
+    nd, nt = 2, 300
+    def first():
+        p = _plan(n, nd, nt)
+        _run_plan(p, n, nd, nt, 16)
+        return p
+    first()                                                      # constants of this length
+    base = (nd + nt) * n * 8
+    held, p = _held(first)
+    assert held <= base + 213 * MB
+    grown, _ = _held(lambda: _run_plan(p, n, nd, nt, 4096)[0].sum().item())
+    assert grown <= 60 * MB + 2 * nd * nt * 4096 * 16            # 2 x 27 MB of records, and the outputs
+    held, q = _held(lambda: _plan(n, nd, nt, owner=p))
+    assert held <= base + 4 * MB
+    L.mfb_destroy(p)                                             # q keeps the scratch
+    _run_plan(q, n, nd, nt, 16)
+    L.mfb_destroy(q)
+
+
+def test_plans_that_share_scratch():
+    """Plans of different lengths on one scratch, interleaved on two streams and replayed
+    from one graph, give what plans of their own give."""
+    import torch
+    from apogee_b200 import _lib
+    L = _lib.lib()
+    g = torch.Generator(device="cuda").manual_seed(2)
+    shapes = [(131072, 2, 3, 16), (32768, 5, 41, 64), (65536, 3, 50, 256), (262144, 1, 5, 16)]
+    plans, alone, want = [], [], []
+    for n, nd, nt, nb in shapes:
+        D = torch.randn(nd, n, dtype=torch.complex64, device="cuda", generator=g)
+        H = torch.randn(nt, n, dtype=torch.complex64, device="cuda", generator=g)
+        pair = []
+        for owner in (None, plans[0] if plans else None):
+            p = _plan(n, nd, nt, owner)
+            _lib.check(L.mfb_set_stream(p, torch.cuda.current_stream().cuda_stream))
+            if n == 32768:
+                _lib.check(L.mfb_set_cluster(p, 0))
+            _lib.check(L.mfb_set_data(p, 0, nd, D.data_ptr()))
+            _lib.check(L.mfb_set_templates(p, 0, nt, H.data_ptr()))
+            pair.append(p)
+        torch.cuda.synchronize()
+        alone.append(pair[0])
+        plans.append(pair[1])
+        want.append(_run_plan(pair[0], n, nd, nt, nb))
+    def all_runs():
+        return [_run_plan(p, *s) for p, s in zip(plans, shapes)]
+    def check(got):
+        torch.cuda.synchronize()
+        for (i, v), (wi, wv) in zip(got, want):
+            assert torch.equal(i, wi) and torch.equal(v, wv)
+    check(all_runs())
+    check(all_runs()[::-1][::-1])
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    got = []
+    for r in range(8):
+        s = streams[r & 1]
+        s.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(s):
+            got.append(_run_plan(plans[r % 4], *shapes[r % 4]))
+    torch.cuda.synchronize()
+    check(got[:4])
+    check(got[4:])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = all_runs()
+    for _ in range(2):
+        for i, _v in got:
+            i.fill_(-7)
+        graph.replay()
+        check(got)
+    check(all_runs())
+    for p in alone + plans:
+        L.mfb_destroy(p)
+
+
+def test_outgrown_scratch_of_a_captured_run_stays():
+    """A graph captured before the scratch grew replays on what it was captured with."""
+    import torch
+    from apogee_b200 import _lib
+    L = _lib.lib()
+    n, nd, nt, nb = 65536, 1, 8, 16
+    g = torch.Generator(device="cuda").manual_seed(6)
+    x = torch.randn(60 * n, dtype=torch.complex64, device="cuda", generator=g)
+    H = torch.randn(nt, n, dtype=torch.complex64, device="cuda", generator=g)
+    p = _plan(n, nd, nt)
+    _lib.check(L.mfb_set_stream(p, torch.cuda.current_stream().cuda_stream))
+    _lib.check(L.mfb_set_data(p, 0, nd, x.data_ptr()))
+    _lib.check(L.mfb_set_templates(p, 0, nt, H.data_ptr()))
+    want = _run_plan(p, n, nd, nt, nb)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = _run_plan(p, n, nd, nt, nb)
+    st = np.arange(60, dtype=np.uint64) * n                      # 480 pairs of 1024 bins: everything grows
+    lo, hi = np.zeros(60, np.uint64), np.full(60, n, np.uint64)
+    idx = torch.empty(60 * nt * 1024, dtype=torch.int64, device="cuda")
+    val = torch.empty(60 * nt * 1024, dtype=torch.complex64, device="cuda")
+    _lib.check(L.mfb_set_stream(p, torch.cuda.current_stream().cuda_stream))
+    _lib.check(L.mfb_run_series(p, x.data_ptr(), x.numel(), st.ctypes.data, lo.ctypes.data, hi.ctypes.data,
+                                60, 0, nt, n // 1024, 0.0, idx.data_ptr(), val.data_ptr(), None))
+    for _ in range(2):
+        got[0].fill_(-7)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    L.mfb_destroy(p)
