@@ -74,6 +74,7 @@ struct Large2Args {
   const float4 *tw1, *tw2;  // passes of the N1- and N2-point transforms, (wr, wr, wi, wi)
   const float2 *anchors;    // [N1/C][5][256]: pass A's twiddle at q = 0, 4, 8, 12, and its step
   float4 *Y;                // [ring][n]
+  int nkeys, kmod;          // bin keys per pair; kmod > 0: keys by (k1, bin mod kmod), else by bin
   uint4 *rec;               // [ring][2][nb] {re, im, ~lag, |z|^2 bits}, zero between launches
   Large2Ctl *ctl;
   int *err;                 // mapped host word, set when a wait ran out
@@ -83,6 +84,19 @@ struct Large2Args {
 };
 
 enum { L2_A = 0, L2_B = 1, L2_END = 2 };
+
+// Keys of a unit of kind B, where bins are not shared by whole warps: a unit sees G
+// neighbouring lags of every k1 (aligned to G), so of narrow bins it sees a few per k1
+// (`kmod`, a power of two; one where bins and window are multiples of G) and needs
+// N1 * kmod keys instead of one per bin.  4096 keys for each of two pairs left one CTA per
+// SM and were scanned whole by every unit: 4096 bins, threshold 0, n = 65536, 4 x 128 pairs
+// 1557 -> 385 us (the per-batch launches before: 861), n = 262144, 4 x 64 2344 -> 778 (1611).
+__host__ __device__ inline void large2_keys(int N1, int G, int bs, int ws, int nb, int &nkeys, int &kmod) {
+  int S = bs % G == 0 && ws % G == 0 ? 1 : 2;
+  while (S > 1 && S < (G + bs - 2) / bs + 1) S *= 2;
+  kmod = (long long)N1 * S < nb ? S : 0;
+  nkeys = kmod ? N1 * S : nb;
+}
 
 // Items between an item's A and B tickets, for `per` tickets per item and a
 // grid of `grid` CTAs: two tickets per CTA and a tenth.
@@ -135,7 +149,7 @@ __global__ void __launch_bounds__(256, 2) large2_kernel(const Large2Args g) {
   static_assert(C * T2 == 256 && G * T1 == 256 && G * ROW <= LARGE2_BUF && N2 * C <= LARGE2_BUF, "");
   extern __shared__ __align__(16) float4 large2_smem[];
   float4 *buf = large2_smem;
-  unsigned long long *keys = reinterpret_cast<unsigned long long *>(buf + LARGE2_BUF);   // [2][nb]
+  unsigned long long *keys = reinterpret_cast<unsigned long long *>(buf + LARGE2_BUF);   // [2][nkeys]
   __shared__ Large2Ticket s_tk[2];
   __shared__ int s_ok;
   __shared__ long long s_fin;
@@ -145,7 +159,7 @@ __global__ void __launch_bounds__(256, 2) large2_kernel(const Large2Args g) {
   const long long total = a.list_count ? (long long)*a.list_count : a.total;
   const long long N = (total + 1) / 2;                   // items
   if (N == 0) return;
-  const int nb = a.nb, nb2 = 2 * nb, ring = g.ring;
+  const int nb = a.nb, nb2 = 2 * nb, nk = g.nkeys, ring = g.ring;
   unsigned *a_done = reinterpret_cast<unsigned *>(g.ctl + 1), *b_done = a_done + ring, *f_done = b_done + ring;
   // units per ticket: keep at least four tickets of kind A per CTA
   int grp = LARGE2_GROUP;
@@ -159,7 +173,7 @@ __global__ void __launch_bounds__(256, 2) large2_kernel(const Large2Args g) {
   unsigned smask = 0u, srank = 0u;
   if (a.seg > 0) bin_segment(T1, a.seg, smask, srank);
   else
-    for (int b = tid; b < nb2; b += 256) keys[b] = 0ull;
+    for (int b = tid; b < 2 * nk; b += 256) keys[b] = 0ull;
 
   // x / d and its remainder, in 32 bits when x allows.
   auto div = [](unsigned long long x, unsigned d, unsigned &r) {
@@ -402,22 +416,30 @@ __global__ void __launch_bounds__(256, 2) large2_kernel(const Large2Args g) {
                 const int k1 = t + T1 * s, lag = N2 * k1 + k2, at = 2 * pad16(k1);
                 const float2 m2 = p2::fma(X[s], X[s], p2::mul(Y[s], Y[s]));
                 const bool in = lag >= a.ws && lag < a.we;
-                pass_b_key(keys, park + at, cf{X[s].x, Y[s].x}, m2.x, lag, in && m2.x > a.t2, 0, 0u, 0u,
-                           a.ws, bs, inv_bs);
-                pass_b_key(keys + nb, park + at + 1, cf{X[s].y, Y[s].y}, m2.y, lag,
-                           in && live_b && m2.y > a.t2, 0, 0u, 0u, a.ws, bs, inv_bs);
+                const bool ca = in && m2.x > a.t2, cb = in && live_b && m2.y > a.t2;
+                if (!(ca || cb)) continue;
+                const int bin = bin_of(lag - a.ws, bs, inv_bs);
+                unsigned long long *key = keys + (g.kmod ? k1 * g.kmod + (bin & (g.kmod - 1)) : bin);
+                if (ca) {
+                  park[at] = make_float2(X[s].x, Y[s].x);
+                  atomicMax(key, ((unsigned long long)(__float_as_uint(m2.x) & ~31u) << 32) | (unsigned)~lag);
+                }
+                if (cb) {
+                  park[at + 1] = make_float2(X[s].y, Y[s].y);
+                  atomicMax(key + nk, ((unsigned long long)(__float_as_uint(m2.y) & ~31u) << 32) | (unsigned)~lag);
+                }
               }
             }
             __syncthreads();
-            for (int b = tid; b < nb2; b += 256) {
+            for (int b = tid; b < 2 * nk; b += 256) {
               const unsigned long long kk = keys[b];
               if (kk == 0ull) continue;
               keys[b] = 0ull;
-              const int sel = b >= nb;
+              const int sel = b >= nk;
               const int lag = (int)(~(unsigned)kk), gw = (lag & (N2 - 1)) - k2base, k1w = lag / N2;
               const float2 v = reinterpret_cast<const float2 *>(buf + gw * ROW)[2 * pad16(k1w) + sel];
-              rec_max(rec + b, make_uint4(__float_as_uint(v.x), __float_as_uint(v.y), (unsigned)kk,
-                                          (unsigned)(kk >> 32)));
+              rec_max(rec + sel * nb + bin_of(lag - a.ws, bs, inv_bs),
+                      make_uint4(__float_as_uint(v.x), __float_as_uint(v.y), (unsigned)kk, (unsigned)(kk >> 32)));
             }
             __syncthreads();          // the next unit's rows go where the values were parked
           }

@@ -306,7 +306,7 @@ static std::map<std::pair<int, int>, LargeConst> g_large;
 // large2_kernel at every supported split.
 #define LARGE2_SPLITS(X) X(128, 256) X(256, 256) X(256, 512) X(512, 512) X(512, 1024) X(1024, 1024)
 
-constexpr int large2_smem(int nb) { return LARGE2_BUF * 16 + 2 * nb * 8; }
+constexpr int large2_smem(int nkeys) { return LARGE2_BUF * 16 + 2 * nkeys * 8; }
 
 template <int N1, int N2>
 static int large2_attr(LargeConst &c, int sms) {
@@ -318,7 +318,7 @@ static int large2_attr(LargeConst &c, int sms) {
   if (b < 1) return fail(MFB_ERR_CUDA, "large kernel (%d x %d) cannot be resident", N1, N2);
   c.units_a = N1 / large2_cols<N2>();
   c.units_b = N2 / (256 / (N1 / 16));
-  c.grid2 = 2 * sms;      // two CTAs per SM (registers and shared memory at up to ~2700 bins)
+  c.grid2 = 2 * sms;      // two CTAs per SM (registers, and shared memory at any number of bins)
   LargeArgs a;
   memset(&a, 0, sizeof a);
   a.n = N1 * N2;
@@ -505,7 +505,11 @@ static cudaError_t launch_large(const LargeConst &c, const LargeArgs &a, cudaStr
 }
 
 static cudaError_t launch_large2(const LargeConst &c, const Large2Args &g, int grid, cudaStream_t s) {
-  const int smem = large2_smem(g.a.nb);
+  int smem = large2_smem(g.nkeys);
+  // At N2 = 1024 a unit of kind A reads 32 bytes of every 128-byte line and finds the rest
+  // in L1 later; two CTAs with this many keys would leave L1 20 KB (n = 2^20, 2 x 32 pairs,
+  // 3000 bins: 831 us, one CTA per SM 624).
+  if (c.N2 == 1024 && smem > 96 << 10) smem = std::max(smem, 116 << 10);
 #define L2_CASE(A, B) if (c.N1 == A && c.N2 == B) large2_kernel<A, B><<<grid, 256, smem, s>>>(g);
   LARGE2_SPLITS(L2_CASE)
 #undef L2_CASE
@@ -923,6 +927,7 @@ static int run_large(mfb_plan *p, int d0, int nd, int t0, int nt, const int32_t 
   g.ctl = reinterpret_cast<Large2Ctl *>(p->ls->state[foreign]);
   g.rec = reinterpret_cast<uint4 *>(p->ls->state[foreign] + large_ctl_bytes(g.ring));
   CUDA_TRY(cudaHostGetDevicePointer((void **)&g.err, p->err, 0));
+  large2_keys(c.N1, 256 / (c.N1 / 16), a.binsize, a.ws, (int)nb, g.nkeys, g.kmod);
   g.spin = p->hold ? 1u << 14 : LARGE2_SPIN;
   g.hold = p->hold;
   const long long items = (a.total + 1) / 2;

@@ -510,3 +510,42 @@ def test_outgrown_scratch_of_a_captured_run_stays():
         torch.cuda.synchronize()
         assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
     L.mfb_destroy(p)
+
+
+@pytest.mark.parametrize("n", [32768, 65536, 131072, 262144, 524288])
+@pytest.mark.parametrize("binsize, win", [
+    ("n/4096", (0, 1)),          # whole groups of a unit's neighbouring lags: one key per k1
+    ("n/1024 + 1", (0, 1)),      # groups that straddle two bins
+    ("n/3000", (0.013, 0.97)),   # and a window on no boundary
+    ("3", (0.4, 0.4)),           # bins narrower than a group, in a short window
+])
+def test_many_bins(n, binsize, win):
+    """Up to 4096 bins per pair, an odd pair count, at threshold 0 (every lag a candidate) and
+    above: the persistent kernel's keys by k1 against the two-pass kernels' keys by bin."""
+    import torch
+    mf = _mf()
+    from apogee_b200 import _lib
+    L = _lib.lib()
+    binsize = eval(binsize.replace("/", "//"), {"n": n})
+    lo, hi = int(win[0] * n), int(win[1] * n)
+    if lo == hi:
+        lo, hi = lo + 5, lo + 5 + 3 * 4000 - 1
+    nd, nt = 1, 3
+    g = torch.Generator(device="cuda").manual_seed(n)
+    D = torch.randn(nd, n, dtype=torch.complex64, device="cuda", generator=g)
+    H = torch.randn(nt, n, dtype=torch.complex64, device="cuda", generator=g)
+    f = mf.MatchedFilter(n, nd, nt)
+    _lib.check(L.mfb_set_cluster(f._plan, 0))
+    f.set_data(D)
+    f.set_templates(H)
+    nb = L.mfb_nbins(n, binsize, lo, hi)
+    assert 900 < nb <= 4096
+    for thr in (0.0, 3.3 * np.sqrt(n)):
+        idx = torch.full((nd, nt, nb), -7, dtype=torch.int64, device="cuda")
+        val = torch.zeros(nd, nt, nb, dtype=torch.complex64, device="cuda")
+        rc = L.mfb_run_large_static(0, n, D.data_ptr(), nd, H.data_ptr(), nt, binsize, thr, lo, hi,
+                                    idx.data_ptr(), val.data_ptr(), None, torch.cuda.current_stream().cuda_stream)
+        _lib.check(rc)
+        for _ in range(2):
+            i2, v2 = f.run_device(binsize=binsize, threshold=thr, window=(lo, hi))
+            assert torch.equal(i2, idx) and torch.equal(v2, val)
