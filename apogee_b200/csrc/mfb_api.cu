@@ -872,6 +872,39 @@ static int cluster_mode(const mfb_plan *p, bool listed, long long pairs) {
   return mode > 0 && p->lc && p->lc->cl[mode - 1].C > 0 ? mode : 0;
 }
 
+// Short dense runs that take the launches per batch (pass A, pass B, finalize) instead of
+// large2_kernel, whose ring neither fills nor overlaps the two passes on so few items:
+// where bins are not whole multiples of N2 lags, either at threshold 0 (every lag a
+// candidate) or with so many bins that writing them out counts; and a pair or two of the
+// longest transform.  Up to SHORT_POINTS lags in all, where the two meet.  B200, us here
+// against large2_kernel, 1 x pairs: 50 ragged bins at threshold 0, n = 65536, 16 pairs 30 / 38,
+// 128 92 / 98, 256 157 / 175 (one launch of 205 MB; in 64 MB batches 183); n = 524288, 4 pairs
+// 39 / 48; 4096 bins above it, n = 65536, 8 pairs 22 / 35; n = 2^20, one pair 28 / 34.  Above
+// a threshold with few bins large2_kernel wins from two pairs on (n = 65536, 16 pairs 24 / 19).
+constexpr long long SHORT_POINTS = 1ll << 23;
+static bool short_run(const LargeArgs &a) {
+  if (a.list || a.n == 32768) return false;   // cluster_mode has that length's rule
+  if (a.n == 1 << 20 && a.total <= 2) return true;
+  return a.seg == 0 && a.total * a.n <= SHORT_POINTS && (a.t2 > 0.f ? a.nb > 1024 : a.nb <= 1024);
+}
+// The launches per batch, in the scratch's rows, with the records of captured runs
+// (zeroed here first).
+static int run_batches(mfb_plan *p, LargeArgs a) {
+  const LargeScratch &s = *p->ls;
+  a.Y = reinterpret_cast<float2 *>(s.rows);
+  a.rec = reinterpret_cast<uint4 *>(s.state[1]);
+  if (capturing(p->stream) && !p->own_capture) p->ls->captured = true;
+  const int most = (int)std::min<size_t>(large_rows(p), s.state_bytes / ((size_t)a.nb * sizeof(uint4)));
+  CUDA_TRY(scratch_begin(p));
+  for (a.pair0 = 0; a.pair0 < a.total; a.pair0 += most) {
+    a.batch = (int)std::min<long long>(most, a.total - a.pair0);
+    CUDA_TRY(cudaMemsetAsync(a.rec, 0, (size_t)a.batch * a.nb * sizeof(uint4), p->stream));
+    CUDA_TRY(launch_large(*p->lc, a, p->stream));
+  }
+  CUDA_TRY(scratch_end(p));
+  return MFB_OK;
+}
+
 // list: listed rows; list_count: how many, on the device.  data: the rows to
 // filter (default the plan's data rows).
 static int run_large(mfb_plan *p, int d0, int nd, int t0, int nt, const int32_t *list,
@@ -914,6 +947,7 @@ static int run_large(mfb_plan *p, int d0, int nd, int t0, int nt, const int32_t 
     CUDA_TRY(launch_cluster(c, cl, a, list ? 0 : a.total, p->stream));
     return MFB_OK;
   }
+  if (short_run(a)) return run_batches(p, a);
   Large2Args g;
   memset(&g, 0, sizeof g);
   g.a = a;
@@ -1013,7 +1047,8 @@ static int run_rows_impl(mfb_plan *p, int d0, int nd, int t0, int nt, const int3
                          const int32_t *nrows, int max_rows, size_t binsize, float threshold,
                          size_t start, size_t end, int64_t *idx, void *val, int32_t *counts,
                          int rs, unsigned long long *trig_total = nullptr, bool *added = nullptr,
-                         int4 *host_rec = nullptr, bool *host_written = nullptr) {
+                         int4 *host_rec = nullptr, bool *host_written = nullptr,
+                         bool empty = false) {
   if (added) *added = false;
   if (host_written) *host_written = false;
   if (!p) return fail(MFB_ERR_ARG, "null plan");
@@ -1030,6 +1065,7 @@ static int run_rows_impl(mfb_plan *p, int d0, int nd, int t0, int nt, const int3
   a.out_val = (float2 *)val;
   a.rs = rs;
   a.out_cnt = counts;   // rows not listed keep whatever the caller put there
+  if (is_large(p->n) && empty && nb <= (size_t)LARGE_MAX_BINS) return large_status(p);
   if (is_large(p->n))
     return run_large(p, d0, nd, t0, nt, rows, nrows, binsize, threshold, start, end, nb, idx, val,
                      counts, rs);
@@ -1050,6 +1086,7 @@ static int run_rows_impl(mfb_plan *p, int d0, int nd, int t0, int nt, const int3
 extern "C" int mfb_run_rows(mfb_plan *p, int d0, int nd, int t0, int nt, const int32_t *rows,
                             const int32_t *nrows, int max_rows, size_t binsize, float threshold,
                             size_t start, size_t end, int64_t *idx, void *val, int32_t *counts) {
+  bool empty = false;
   if (p && is_large(p->n) && !cluster_mode(p, true, 0) && rows && nrows && max_rows >= 0) {
     // this length checks the list's length against max_rows: read it on the host
     DeviceGuard dg(p->device);
@@ -1057,9 +1094,10 @@ extern "C" int mfb_run_rows(mfb_plan *p, int d0, int nd, int t0, int nt, const i
     CUDA_TRY(cudaMemcpyAsync(&cnt, nrows, sizeof cnt, cudaMemcpyDeviceToHost, p->stream));
     CUDA_TRY(cudaStreamSynchronize(p->stream));
     if (cnt > max_rows) return fail(MFB_ERR_ARG, "row count %d exceeds max_rows %d", cnt, max_rows);
+    empty = cnt == 0;
   }
   return run_rows_impl(p, d0, nd, t0, nt, rows, nrows, max_rows, binsize, threshold, start, end,
-                       idx, val, counts, 1);
+                       idx, val, counts, 1, nullptr, nullptr, nullptr, nullptr, empty);
 }
 
 extern "C" int mfb_forward(mfb_plan *p, const void *series, size_t nseries,

@@ -546,6 +546,75 @@ def test_many_bins(n, binsize, win):
         rc = L.mfb_run_large_static(0, n, D.data_ptr(), nd, H.data_ptr(), nt, binsize, thr, lo, hi,
                                     idx.data_ptr(), val.data_ptr(), None, torch.cuda.current_stream().cuda_stream)
         _lib.check(rc)
+        rows = torch.arange(nd * nt, dtype=torch.int32, device="cuda")   # lists take no other kernel
+        count = torch.tensor([nd * nt], dtype=torch.int32, device="cuda")
         for _ in range(2):
+            i2, v2 = torch.full_like(idx, -7), torch.zeros_like(val)
+            f._bind_stream()
+            _lib.check(L.mfb_run_rows(f._plan, 0, nd, 0, nt, rows.data_ptr(), count.data_ptr(), nd * nt, binsize,
+                                      thr, lo, hi, i2.data_ptr(), v2.data_ptr(), None))
+            assert torch.equal(i2, idx) and torch.equal(v2, val)
             i2, v2 = f.run_device(binsize=binsize, threshold=thr, window=(lo, hi))
             assert torch.equal(i2, idx) and torch.equal(v2, val)
+
+
+@pytest.mark.parametrize("n, nd, nt, nb, thr", [
+    (65536, 1, 1, 50, 0.0),
+    (65536, 2, 64, 50, 0.0),         # 2^23 lags: the last on the launches per batch
+    (65536, 3, 43, 50, 0.0),         # the first in the persistent kernel
+    (65536, 1, 1, 4090, 900.0),
+    (131072, 5, 7, 1024, 0.0),       # the edge on bins, either side and threshold
+    (131072, 5, 7, 1025, 0.0),
+    (131072, 5, 7, 1024, 1200.0),
+    (131072, 5, 7, 1025, 1200.0),
+    (262144, 1, 3, 300, 0.0),
+    (524288, 2, 2, 16, 0.0),
+    (1 << 20, 1, 1, 16, 0.0),        # any bins
+    (1 << 20, 1, 2, 16, 3000.0),
+    (1 << 20, 1, 3, 16, 0.0),
+    (1 << 20, 1, 2, 1000, 0.0),
+])
+def test_short_runs(n, nd, nt, nb, thr):
+    """Dense runs around the rule on short runs give the bits of the same rows listed (which
+    always take the persistent kernel), direct, with counts and captured."""
+    import torch
+    mf = _mf()
+    from apogee_b200 import _lib
+    L = _lib.lib()
+    g = torch.Generator(device="cuda").manual_seed(n + nb)
+    f = mf.MatchedFilter(n, nd, nt)
+    f.set_data(torch.randn(nd, n, dtype=torch.complex64, device="cuda", generator=g))
+    f.set_templates(torch.randn(nt, n, dtype=torch.complex64, device="cuda", generator=g))
+    lo, hi = (0, n) if nb == 16 else (7, n - 30)
+    binsize = n // 16 if nb == 16 else -(-(hi - lo) // nb)
+    nb = L.mfb_nbins(n, binsize, lo, hi)
+    shape = (nd, nt, nb)
+    rows = torch.arange(nd * nt, dtype=torch.int32, device="cuda")
+    count = torch.tensor([nd * nt], dtype=torch.int32, device="cuda")
+    idx = torch.full(shape, -7, dtype=torch.int64, device="cuda")
+    val = torch.zeros(shape, dtype=torch.complex64, device="cuda")
+    f._bind_stream()
+    _lib.check(L.mfb_run_rows(f._plan, 0, nd, 0, nt, rows.data_ptr(), count.data_ptr(), nd * nt, binsize, thr,
+                              lo, hi, idx.data_ptr(), val.data_ptr(), None))
+    kw = dict(binsize=binsize, threshold=thr, window=(lo, hi))
+    for _ in range(2):
+        i, v = f.run_device(**kw)
+        assert torch.equal(i, idx) and torch.equal(v, val)
+    out, cnt = f.run(counts=True, **kw)
+    np.testing.assert_array_equal(out["index"], idx.cpu().numpy())
+    np.testing.assert_array_equal(cnt, (idx >= 0).sum(-1).cpu().numpy())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        i, v = f.run_device(**kw)
+    for _ in range(2):
+        i.fill_(-7)
+        graph.replay()
+        assert torch.equal(i, idx) and torch.equal(v, val)
+    count.zero_()                                # an empty list writes nothing
+    idx.fill_(-7)
+    f._bind_stream()
+    _lib.check(L.mfb_run_rows(f._plan, 0, nd, 0, nt, rows.data_ptr(), count.data_ptr(), nd * nt, binsize, thr,
+                              lo, hi, idx.data_ptr(), val.data_ptr(), None))
+    assert (idx == -7).all()
+    i, v = f.run_device(**kw)
+    assert not (i == -7).any()
