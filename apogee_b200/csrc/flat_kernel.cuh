@@ -65,7 +65,7 @@ struct FlatArgs {
   // (the hierarchical plan's trigger count) -- one thread, once
   unsigned long long *trig_total;
   // if set (record output, rs == 2): every output record is also stored here,
-  // the caller's pinned host table seen from the device (flatw_kernel only)
+  // the caller's pinned host table seen from the device (listed runs, nb <= KEYCAP)
   int4 *host_rec;
 };
 
@@ -248,6 +248,13 @@ __device__ __forceinline__ bool any_candidate(const cf *v, float t2, bool live, 
 #pragma unroll
   for (int q = 0; q < 16; q++) mx = fmaxf(mx, fmaf(v[q].x, v[q].x, v[q].y * v[q].y));
   return __any_sync(gmask, live && mx > t2);
+}
+
+// Output o of a run with a host table (FlatArgs::host_rec): a 16-byte store over the
+// host link.
+__device__ __forceinline__ void store_host(int4 *host_rec, long long o, long long ix, float2 val) {
+  host_rec[o] = make_int4((int)(unsigned)(unsigned long long)ix, (int)(unsigned)((unsigned long long)ix >> 32),
+                          __float_as_int(val.x), __float_as_int(val.y));
 }
 
 // Items [ibeg, iend) of one launch's pairs (item i = pairs i*G .. i*G+G-1 of
@@ -478,6 +485,7 @@ __device__ __forceinline__ void flat_range(const FlatArgs &a, long long ibeg, lo
             }
             a.out_idx[(obase + b) * a.rs] = ix;
             a.out_val[(obase + b) * a.rs] = val;
+            if (a.host_rec) store_host(a.host_rec, obase + b, ix, val);
           }
           if (a.out_cnt) {
             const int c = __reduce_add_sync(gmask, cnt);

@@ -105,10 +105,7 @@ __global__ void __launch_bounds__(FlatWGeo<N>::CTA, FlatWGeo<N>::MINB) flatw_ker
         const long long o = (long long)prev * nb + t;
         a.out_idx[o * a.rs] = ix;
         a.out_val[o * a.rs] = val;
-        if (a.host_rec)   // 16-byte store over the host link into the host table
-          a.host_rec[o] = make_int4((int)(unsigned)(unsigned long long)ix,
-                                    (int)(unsigned)((unsigned long long)ix >> 32),
-                                    __float_as_int(val.x), __float_as_int(val.y));
+        if (a.host_rec) store_host(a.host_rec, o, ix, val);
         if (a.out_cnt && kk != 0ull) atomicAdd(a.out_cnt + prev, 1);
       }
     } else {

@@ -415,3 +415,27 @@ def test_repeated_run_skips_set_up_but_follows_every_change():
     hf.set_data(bank)
     check(binsize=512, threshold=20.0)
     check(binsize=512, threshold=20.0, window=(0, n))    # a tuple window: same result
+
+
+@pytest.mark.parametrize("n, band", [(128, 64), (512, 64), (4096, 512), (8192, 1024), (16384, 1024)])
+@pytest.mark.parametrize("bins", ["n/64", "ragged", "n/128"])
+def test_general_bins_are_stored_into_the_host_table(n, band, bins):
+    """Bins that are no whole blocks of n/16 lags: the listed kernel stores refined rows
+    of up to 64 bins into the host table itself, a copy kernel those of more."""
+    nd, nt = 3, 29
+    rng = np.random.default_rng(n)
+    H = noise(rng, (nt, n))
+    hf = _filter(n, nd, nt, band, "fp32", 0.0)
+    hf.set_templates(H)
+    hf.set_data(noise(rng, (nd, n)))
+    hf.set_coarse_threshold(float(np.quantile(hf.coarse_values(), 0.7)))
+    kw = {"n/64": dict(binsize=n // 64), "n/128": dict(binsize=n // 128),
+          "ragged": dict(binsize=n // 10 + 1, window=(3, n - 5))}[bins]
+    for k in range(5):
+        D = noise(rng, (nd, n))
+        hf.set_data(D)
+        out = hf.run(threshold=2.0 * np.sqrt(n), **kw)
+        idx, val = _dense(hf, threshold=2.0 * np.sqrt(n), **kw)
+        np.testing.assert_array_equal(out["index"], idx)
+        np.testing.assert_array_equal(out["value"], val)
+        assert (idx >= 0).any()
