@@ -550,8 +550,13 @@ __device__ __forceinline__ void flat_range(const FlatArgs &a, long long ibeg, lo
 // measured 6% slower on the B200 (246 vs 232 us for 16 x 1024 pairs at
 // n = 4096, CUDA events, L2 flushed), while flat_range's short dynamic ranges
 // in the batched kernel need the entry barrier and the coherent-load switch.
-template <int N, int MODE>
-__global__ void __launch_bounds__(FlatGeo<N>::CTA, FlatGeo<N>::MINB)
+//
+// MINB: CTAs per SM.  A run with no more items than two CTAs per SM take at once has no
+// use for a third and takes the form with 128 registers, which has all 32 loads of a
+// pair in flight: us at threshold 0, three CTAs / two, n = 128, 4 x 100 pairs 12.5 / 10.6;
+// n = 256, 2 x 37 pairs of 64 bins 12.7 / 10.9; n = 1024, 1 x 16 of 64 14.5 / 12.7.
+template <int N, int MODE, int MINB = FlatGeo<N>::MINB>
+__global__ void __launch_bounds__(FlatGeo<N>::CTA, MINB)
 flat_kernel(const FlatArgs a) {
   using Geo = FlatGeo<N>;
   constexpr int T = Geo::T, G = Geo::G;

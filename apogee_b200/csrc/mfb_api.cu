@@ -105,6 +105,7 @@ struct NConst {
   int grid_peaks = 0, grid_gate = 0, grid_fwd = 0;
   int cta = 0, smem = 0, g = 0;
   int grid_rows = 0;
+  int grid_few = 0;             // items up to which flat_kernel runs two CTAs per SM
   // n = 128 ... 1024: the tables as (wr, wr, wi, wi) records for two pairs per
   // thread (the transforms of large2_kernel.cuh)
   float4 *twid2 = nullptr;
@@ -180,6 +181,11 @@ static int make_const(int device, NConst &c) {
     c.gridw = b5 * sms;
     c.gridw_gate = b6 * sms;
   }
+  if constexpr (Geo::MINB == 3) {
+    CUDA_TRY(cudaFuncSetAttribute(flat_kernel<N, MODE_PEAKS, 2>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, Geo::SMEM));
+    c.grid_few = 2 * sms;
+  }
   c.grid_rows = b4 * sms;
   c.grid_peaks = b1 * sms;
   c.grid_gate = b2 * sms;
@@ -233,9 +239,22 @@ static cudaError_t launch_flatw(int n, const NConst &c, FlatArgs a, cudaStream_t
   return cudaGetLastError();
 }
 
+template <int N>
+static void launch_peaks_n(const NConst &c, const FlatArgs &a, cudaStream_t s) {
+  using Geo = FlatGeo<N>;
+  if constexpr (Geo::MINB == 3) {
+    const long long items = ((long long)a.nd * a.nt + Geo::G - 1) / Geo::G;
+    if (items <= c.grid_few) {
+      flat_kernel<N, MODE_PEAKS, 2><<<(int)items, Geo::CTA, Geo::SMEM, s>>>(a);
+      return;
+    }
+  }
+  flat_kernel<N, MODE_PEAKS><<<c.grid_peaks, Geo::CTA, Geo::SMEM, s>>>(a);
+}
+
 static cudaError_t launch_peaks(int n, const NConst &c, const FlatArgs &a, cudaStream_t s) {
   switch (n) {
-#define MFB_CASE(NN) case NN: flat_kernel<NN, MODE_PEAKS><<<c.grid_peaks, c.cta, c.smem, s>>>(a); break;
+#define MFB_CASE(NN) case NN: launch_peaks_n<NN>(c, a, s); break;
     MFB_CASE(64) MFB_CASE(128) MFB_CASE(256) MFB_CASE(512) MFB_CASE(1024)
     MFB_CASE(2048) MFB_CASE(4096) MFB_CASE(8192) MFB_CASE(16384)
 #undef MFB_CASE

@@ -455,3 +455,30 @@ def test_threshold_skips_only_pairs_without_candidates(n, win):
         out = check(f, D, H, binsize, thr, w)
         assert (out["index"][1, 4] >= 0).any()
         assert (out["index"] >= 0).any(-1).sum() < 27
+
+
+@pytest.mark.parametrize("n", [64, 128, 256, 1024, 4096])
+@pytest.mark.parametrize("thr", [0.0, 4.0])
+def test_few_items_give_the_same_bits(n, thr):
+    """Runs of up to two CTAs per SM take flat_kernel's form with more registers: at the
+    line, one pair past it and in pieces, general bins, against each other."""
+    import torch
+    mf = _mf()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    line = 2 * sms * max(1, 4096 // n)                 # pairs that fill two CTAs per SM
+    g = torch.Generator(device="cuda").manual_seed(n)
+    nt = line + 1
+    D = torch.randn(1, n, dtype=torch.complex64, device="cuda", generator=g)
+    H = torch.randn(nt, n, dtype=torch.complex64, device="cuda", generator=g)
+    f = mf.MatchedFilter(n, 1, nt)
+    f.set_data(D)
+    f.set_templates(H)
+    kw = dict(binsize=n // 5 + 1, threshold=thr * np.sqrt(n), window=(1, n - 2))
+    whole = f.run_device(**kw)
+    for parts in ((0, line), (line, 1), (5, 33)):
+        i, v = f.run_device(templates=parts, **kw)
+        t = slice(parts[0], parts[0] + parts[1])
+        assert torch.equal(i, whole[0][:, t]) and torch.equal(v, whole[1][:, t])
+    i, v = whole[0].cpu().numpy(), whole[1].cpu().numpy()
+    z = oracle.correlate(D.cpu().numpy(), H[:8].cpu().numpy())
+    assert not parity.compare(i[:, :8], v[:, :8], z, n // 5 + 1, thr * np.sqrt(n), (1, n - 2))
