@@ -80,6 +80,8 @@ SIGNATURES = {
     "mfb_run_records": (_I, [_P, _I, _I, _I, _I, _SZ, _F, _SZ, _SZ, _P, _P]),
     "mfb_run_rows": (_I, [_P, _I, _I, _I, _I, _P, _P, _I, _SZ, _F, _SZ, _SZ, _P, _P, _P]),
     "mfb_run_series": (_I, [_P, _P, _SZ, _P, _P, _P, _I, _I, _I, _SZ, _F, _P, _P, _P]),
+    "mfb_run_series_records": (_I, [_P, _P, _SZ, _P, _P, _P, _I, _I, _I, _SZ, _F, _P, _P]),
+    "mfb_hier_run_series_records": (_I, [_P, _P, _SZ, _P, _P, _P, _I, _I, _I, _SZ, _F, _P, _P]),
     "mfb_forward": (_I, [_P, _P, _SZ, _P, _I, _P]),
     "mfb_nbins": (_SZ, [_SZ, _SZ, _SZ, _SZ]),
     "mfb_last_error": (ctypes.c_char_p, []),

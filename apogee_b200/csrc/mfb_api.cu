@@ -1166,11 +1166,11 @@ extern "C" int mfb_forward(mfb_plan *p, const void *series, size_t nseries,
   return MFB_OK;
 }
 
-extern "C" int mfb_run_series(mfb_plan *p, const void *series, size_t nseries,
-                              const uint64_t *starts, const uint64_t *win_start,
-                              const uint64_t *win_end, int nblocks, int t0, int nt,
-                              size_t binsize, float threshold, int64_t *idx, void *val,
-                              int32_t *counts) {
+// rs: stride of idx (int64) and val (complex64) between results, as FlatArgs has it.
+static int run_series_impl(mfb_plan *p, const void *series, size_t nseries, const uint64_t *starts,
+                           const uint64_t *win_start, const uint64_t *win_end, int nblocks, int t0,
+                           int nt, size_t binsize, float threshold, int64_t *idx, void *val,
+                           int32_t *counts, int rs) {
   if (!p) return fail(MFB_ERR_ARG, "null plan");
   if (!series || !starts || !win_start || !win_end || nblocks < 1 || !idx || !val)
     return fail(MFB_ERR_ARG, "invalid run_series arguments");
@@ -1224,22 +1224,39 @@ extern "C" int mfb_run_series(mfb_plan *p, const void *series, size_t nseries,
     size_t lo = win_start[b0], hi = win_end[b0];
     if (is_large(p->n)) {
       r = run_large(p, 0, g, t0, nt, nullptr, nullptr, binsize, threshold, lo, hi, nb0,
-                    idx + (size_t)b0 * nt * nb0, (float2 *)val + (size_t)b0 * nt * nb0,
-                    counts ? counts + (size_t)b0 * nt : nullptr, 1, p->sspec);
+                    idx + (size_t)b0 * nt * nb0 * rs, (float2 *)val + (size_t)b0 * nt * nb0 * rs,
+                    counts ? counts + (size_t)b0 * nt : nullptr, rs, p->sspec);
       if (r) return r;
       b0 += g;
       continue;
     }
     FlatArgs a = base_args(p, 0, g, t0, nt, binsize, threshold, lo, hi, nb0);
     a.data = p->sspec;
-    a.out_idx = (long long *)idx + (size_t)b0 * nt * nb0;
-    a.out_val = (float2 *)val + (size_t)b0 * nt * nb0;
-    a.rs = 1;
+    a.out_idx = (long long *)idx + (size_t)b0 * nt * nb0 * rs;
+    a.out_val = (float2 *)val + (size_t)b0 * nt * nb0 * rs;
+    a.rs = rs;
     a.out_cnt = counts ? counts + (size_t)b0 * nt : nullptr;
     CUDA_TRY(launch_dense(p, a));
     b0 += g;
   }
   return MFB_OK;
+}
+extern "C" int mfb_run_series(mfb_plan *p, const void *series, size_t nseries,
+                              const uint64_t *starts, const uint64_t *win_start,
+                              const uint64_t *win_end, int nblocks, int t0, int nt,
+                              size_t binsize, float threshold, int64_t *idx, void *val,
+                              int32_t *counts) {
+  return run_series_impl(p, series, nseries, starts, win_start, win_end, nblocks, t0, nt, binsize,
+                         threshold, idx, val, counts, 1);
+}
+extern "C" int mfb_run_series_records(mfb_plan *p, const void *series, size_t nseries,
+                                      const uint64_t *starts, const uint64_t *win_start,
+                                      const uint64_t *win_end, int nblocks, int t0, int nt,
+                                      size_t binsize, float threshold, void *records,
+                                      int32_t *counts) {
+  if (!records) return fail(MFB_ERR_ARG, "null pointer argument");
+  return run_series_impl(p, series, nseries, starts, win_start, win_end, nblocks, t0, nt, binsize,
+                         threshold, (int64_t *)records, (char *)records + 8, counts, 2);
 }
 
 // ---------------------------------------------------------- hierarchical plan
@@ -2773,11 +2790,11 @@ extern "C" int mfb_batch_info(mfb_batch *b, int64_t *tickets, int *grid, int *se
 }
 
 // ------------------------------------------------- hierarchical run_series
-extern "C" int mfb_hier_run_series(mfb_hplan *h, const void *series, size_t nseries,
-                                   const uint64_t *starts, const uint64_t *win_start,
-                                   const uint64_t *win_end, int nblocks, int t0, int nt,
-                                   size_t binsize, float threshold, int64_t *idx, void *val,
-                                   int32_t *counts) {
+static int hier_run_series_impl(mfb_hplan *h, const void *series, size_t nseries,
+                                const uint64_t *starts, const uint64_t *win_start,
+                                const uint64_t *win_end, int nblocks, int t0, int nt,
+                                size_t binsize, float threshold, int64_t *idx, void *val,
+                                int32_t *counts, int rs) {
   if (!h) return fail(MFB_ERR_ARG, "null plan");
   mfb_plan *p = h->full;
   if (!series || !starts || !win_start || !win_end || nblocks < 1 || !idx || !val)
@@ -2813,12 +2830,29 @@ extern "C" int mfb_hier_run_series(mfb_hplan *h, const void *series, size_t nser
     int r = mfb_forward(p, series, nseries, p->starts_dev + b0, g, p->data);
     if (r) return r;
     r = hier_run_impl(h, 0, g, t0, nt, binsize, threshold, win_start[b0], win_end[b0],
-                      idx + (size_t)b0 * nt * nb0, (float2 *)val + (size_t)b0 * nt * nb0,
-                      counts ? counts + (size_t)b0 * nt : nullptr, 1);
+                      idx + (size_t)b0 * nt * nb0 * rs, (float2 *)val + (size_t)b0 * nt * nb0 * rs,
+                      counts ? counts + (size_t)b0 * nt : nullptr, rs);
     if (r) return r;
     b0 += g;
   }
   return MFB_OK;
+}
+extern "C" int mfb_hier_run_series(mfb_hplan *h, const void *series, size_t nseries,
+                                   const uint64_t *starts, const uint64_t *win_start,
+                                   const uint64_t *win_end, int nblocks, int t0, int nt,
+                                   size_t binsize, float threshold, int64_t *idx, void *val,
+                                   int32_t *counts) {
+  return hier_run_series_impl(h, series, nseries, starts, win_start, win_end, nblocks, t0, nt, binsize,
+                              threshold, idx, val, counts, 1);
+}
+extern "C" int mfb_hier_run_series_records(mfb_hplan *h, const void *series, size_t nseries,
+                                           const uint64_t *starts, const uint64_t *win_start,
+                                           const uint64_t *win_end, int nblocks, int t0, int nt,
+                                           size_t binsize, float threshold, void *records,
+                                           int32_t *counts) {
+  if (!records) return fail(MFB_ERR_ARG, "null pointer argument");
+  return hier_run_series_impl(h, series, nseries, starts, win_start, win_end, nblocks, t0, nt, binsize,
+                              threshold, (int64_t *)records, (char *)records + 8, counts, 2);
 }
 
 // --------------------------------------------------------- gate model (device)

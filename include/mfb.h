@@ -141,6 +141,11 @@ int mfb_run_series(mfb_plan *p, const void *series, size_t nseries, const uint64
                    const uint64_t *win_start, const uint64_t *win_end, int nblocks,
                    int t0, int nt, size_t binsize, float threshold,
                    int64_t *idx, void *val, int32_t *counts);
+/* mfb_run_series with PEAK_DTYPE record output, as mfb_run_records. */
+int mfb_run_series_records(mfb_plan *p, const void *series, size_t nseries, const uint64_t *starts,
+                           const uint64_t *win_start, const uint64_t *win_end, int nblocks,
+                           int t0, int nt, size_t binsize, float threshold, void *records,
+                           int32_t *counts);
 /* Forward spectra of blocks, FFT(series[start..start+n)/n) zero-padded past
    nseries, into spectra [nblocks][n] (DEVICE).  Replaces the GPU forward
    stage Context.forward (python/matchedfilter/_vkcompute.py:855-906). */
@@ -230,6 +235,11 @@ int mfb_hier_run_series(mfb_hplan *p, const void *series, size_t nseries, const 
                         const uint64_t *win_start, const uint64_t *win_end, int nblocks,
                         int t0, int nt, size_t binsize, float threshold,
                         int64_t *idx, void *val, int32_t *counts);
+/* mfb_hier_run_series with PEAK_DTYPE record output. */
+int mfb_hier_run_series_records(mfb_hplan *p, const void *series, size_t nseries,
+                                const uint64_t *starts, const uint64_t *win_start,
+                                const uint64_t *win_end, int nblocks, int t0, int nt,
+                                size_t binsize, float threshold, void *records, int32_t *counts);
 /* Replaces ap_hmf_stats (src/hmf.c:84-103): pairs and triggers since creation
    (synchronises the plan's stream).  Triggers are summed on the device, so
    runs need no host round trip and can be captured in a CUDA graph. */

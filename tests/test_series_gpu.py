@@ -91,3 +91,35 @@ def test_series_equals_block_by_block():
     spec = oracle.series_spectra(series, starts, n)
     z = oracle.correlate(spec, H)
     assert not parity.compare(idx, val, z, 512)
+
+
+@pytest.mark.parametrize("kind", ["flat", "hier"])
+@pytest.mark.parametrize("n", [512, 4096, 65536])
+def test_records_equal_separate_arrays(kind, n):
+    """The structured result (records written by the kernels, one copy) against raw=True (two
+    arrays), over windows that are grouped out of the caller's order, one bin and many, and a
+    result larger than the one before."""
+    import apogee_b200 as mf
+    rng = np.random.default_rng(n)
+    nt, blocks = 3, 7
+    H = noise(rng, (nt, n))
+    x = noise(rng, n * 5)
+    if kind == "flat":
+        f = mf.MatchedFilter(n, 2, nt)
+    else:
+        f = mf.HierarchicalFilter(n, 2, nt, band=n // 8, coarse="fp32")
+        f.set_coarse_threshold(0.0)
+    f.set_templates(H)
+    st = np.arange(blocks) * (n // 2)
+    lo = np.where(np.arange(blocks) % 3 == 1, n // 8, n // 4)
+    for binsize in (n // 2, n // 16, n // 512 + 1):
+        kw = dict(binsize=binsize, threshold=np.sqrt(2.0) * 1.5)
+        out = f.run_series(x, st, lo, lo + n // 2, **kw)
+        idx, val = f.run_series(x, st, lo, lo + n // 2, raw=True, **kw)
+        assert out.dtype == mf.PEAK_DTYPE and out.shape == (blocks, nt, -(-(n // 2) // binsize))
+        np.testing.assert_array_equal(out["index"], idx)
+        np.testing.assert_array_equal(out["value"], val)
+        assert (idx >= 0).any()
+        again = f.run_series(x, st, lo, lo + n // 2, **kw)
+        assert not np.shares_memory(again, out)
+        np.testing.assert_array_equal(again, out)
