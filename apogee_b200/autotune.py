@@ -39,17 +39,15 @@ def candidates(n):
 
 #: What tune(n) found on a B200 (CUDA events, probe workload of probe_shape):
 #: the kernel configuration and the cost per pair (us) in the persistent launch
-#: and on the job's own launches.  Used when a batch is not tuned.  (With flatw_kernel and
-#: large2_kernel tune() finds 0.0031, 0.0064, 0.0132, 0.033, 0.064, 0.177 and 0.350 on own
-#: launches; these older costs keep jobs near the line in the persistent launch.)
+#: and on the job's own launches.  Used when a batch is not tuned.
 B200 = {
-    1024: ({"unit_items": 8}, 0.0046, 0.0037),
-    2048: ({"unit_items": 8}, 0.0094, 0.0076),
-    4096: ({"unit_items": 8}, 0.0198, 0.0148),
-    8192: ({"split": 64}, 0.131, 0.038),
-    16384: ({"split": 64}, 0.235, 0.086),
-    32768: ({"split": 128}, 0.477, 0.335),
-    65536: ({"split": 256}, 0.940, 0.661),
+    1024: ({"unit_items": 8}, 0.0043, 0.0030),
+    2048: ({"unit_items": 8}, 0.0090, 0.0062),
+    4096: ({"unit_items": 8}, 0.0185, 0.0127),
+    8192: ({"split": 64}, 0.129, 0.0320),
+    16384: ({"split": 64}, 0.233, 0.0605),
+    32768: ({"split": 64}, 0.457, 0.173),
+    65536: ({"split": 128}, 0.906, 0.341),
 }
 
 

@@ -140,3 +140,17 @@ def test_repeat_key_accepts_only_immutable_arguments():
     assert _repeat_key(np.int64(256), 5.5, None, None, None) is None
     assert _repeat_key(256, np.float32(5.5), None, None, None) is None
     assert _repeat_key(256, 5.5, (0, 4096.0), None, None) is None
+
+
+def test_default_batch_costs_are_usable():
+    """The untuned costs: configurations the kernel takes, own launches never dearer, and the
+    line from them (DEDICATED_LAUNCH_US over the saving per pair)."""
+    from types import SimpleNamespace
+    from apogee_b200 import autotune, batch
+    for n, (cfg, pp, dp) in autotune.B200.items():
+        assert cfg in autotune.candidates(n) and 0 < dp < pp
+        line = batch.DEDICATED_LAUNCH_US / (pp - dp)
+        d = autotune.default(n)
+        assert batch.dedicated(SimpleNamespace(pairs=int(line) + 1), d)
+        assert not batch.dedicated(SimpleNamespace(pairs=int(line)), d)
+    assert 17 <= batch.DEDICATED_LAUNCH_US / (autotune.B200[65536][1] - autotune.B200[65536][2]) < 19
