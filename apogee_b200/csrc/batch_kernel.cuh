@@ -178,7 +178,7 @@ __device__ __forceinline__ void small_unit(int jid, int u, float2 *smem) {
   const long long items = ((long long)j.nd * j.nt + G - 1) / G;
   const long long ibeg = (long long)u * j.unit_items;
   const long long iend = min(items, ibeg + j.unit_items);
-  flat_range<N, MODE_PEAKS, false>(f, ibeg, iend, smem);
+  flat_range<N>(f, ibeg, iend, smem);
 }
 
 template <int N>

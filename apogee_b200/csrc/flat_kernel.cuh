@@ -11,15 +11,15 @@
 //    butterfly per thread per pass.  A thread keeps 16 complex values in
 //    registers; passes exchange through padded shared memory.
 //  * The conjugate product is formed while the first pass loads: template and
-//    data spectra come from HBM, L2 or L1 with coalesced 8-byte loads (a CTA stays
-//    on a data row for many pairs; registers are better spent on a third CTA per SM
-//    than on keeping the row, FlatGeo::MINB).
+//    data spectra come from HBM, L2 or L1 with coalesced 8-byte loads (neighbouring
+//    items share a data row; registers are better spent on a third CTA per SM than on
+//    keeping it, FlatGeo::MINB).
 //  * Thread t ends holding z[t + T*q], q = 0..15 (T = n/16).  The per-bin
 //    argmax is a warp redux on |z|^2 bit patterns followed by one 64-bit
 //    shared-memory atomicMax per warp and bin on the key
 //    (|z|^2 bits << 32) | ~lag, which makes the lowest lag win exact ties.
-//  * Persistent CTAs walk a contiguous range of pairs, data row outer,
-//    template inner, so concurrent CTAs on different rows share templates in L2.
+//  * Persistent CTAs take every gridDim.x-th item, data row outer, template inner,
+//    so that a loud data row's pairs are shared by all SMs.
 //  * Runs whose bins and window are whole blocks of n/16 lags at n >= 512 take
 //    flatw_kernel instead (same bits), and so do the gate passes at those lengths.
 //
@@ -259,12 +259,10 @@ __device__ __forceinline__ void store_host(int4 *host_rec, long long o, long lon
 
 // Items [ibeg, iend) of one launch's pairs (item i = pairs i*G .. i*G+G-1 of
 // the dense block or the list), processed by one CTA of FlatGeo<N>::CTA
-// threads with `smem` its dynamic shared memory.  CACHE_D keeps a data row
-// in registers while consecutive pairs share it (long static ranges); without
-// it the data spectrum is loaded beside each template (short dynamic ranges,
-// 32 registers fewer).  Used by the batched kernel (ranges handed out at run
-// time); synchronises the CTA on entry, so smem may still be in use then.
-template <int N, int MODE, bool CACHE_D = true>
+// threads with `smem` its dynamic shared memory.  Used by the batched kernel
+// (ranges handed out at run time) and rows_kernel; synchronises the CTA on entry,
+// so smem may still be in use then.
+template <int N>
 __device__ __forceinline__ void flat_range(const FlatArgs &a, long long ibeg, long long iend,
                                            float2 *smem) {
   using Geo = FlatGeo<N>;
@@ -275,13 +273,11 @@ __device__ __forceinline__ void flat_range(const FlatArgs &a, long long ibeg, lo
   const long long total = a.list ? (long long)(*a.list_count) : (long long)a.nd * a.nt;
   __syncthreads();
 
-  cf dreg[CACHE_D ? 16 : 1];   // the data row, kept while consecutive pairs share it
-  int cur_d = -1;
   const int lane = threadIdx.x & 31;
 
   // Bin bookkeeping, once per launch.
   const int W = a.we - a.ws;
-  const int bs = (MODE == MODE_GATE) ? W : a.binsize;
+  const int bs = a.binsize;
   const float inv_bs = 1.0f / (float)bs;
   const int Tdiv = T / bs, Tmod = T - Tdiv * bs;
   const unsigned gmask = (T >= 32) ? 0xffffffffu : (((1u << T) - 1u) << (lane & ~(T - 1)));
@@ -304,7 +300,7 @@ __device__ __forceinline__ void flat_range(const FlatArgs &a, long long ibeg, lo
       if (rlo >= bs) { rlo -= bs; blo++; }
     }
   }
-  const int nbins = (MODE == MODE_GATE) ? 1 : a.nb;
+  const int nbins = a.nb;
   const bool small_keys = nbins <= KEYCAP;
   unsigned long long *kslots = reinterpret_cast<unsigned long long *>(smem + G * Geo::BUF);
   // Per-warp staging of the 16 slot winners (fast layout only).
@@ -331,38 +327,13 @@ __device__ __forceinline__ void flat_range(const FlatArgs &a, long long ibeg, lo
     if (live) {
       const float2 *hp = a.tmpl + (long long)(a.t0 + tt) * a.tmpl_stride;
       const float2 *dp = a.data + (long long)(a.d0 + d) * a.data_stride;
-      if constexpr (CACHE_D) {
-        if (d != cur_d) {
-          if (a.data_cg) {   // data written earlier in the same launch
 #pragma unroll
-            for (int s = 0; s < 16; s++) {
-              float2 x = __ldcg(dp + t + T * s);
-              dreg[s] = {x.x, x.y};
-            }
-          } else {
-#pragma unroll
-            for (int s = 0; s < 16; s++) {
-              float2 x = __ldg(dp + t + T * s);
-              dreg[s] = {x.x, x.y};
-            }
-          }
-          cur_d = d;
-        }
-#pragma unroll
-        for (int s = 0; s < 16; s++) {
-          float2 h = __ldg(hp + t + T * s);
-          // D * conj(H)
-          v[s].x = fmaf(dreg[s].x, h.x, dreg[s].y * h.y);
-          v[s].y = fmaf(dreg[s].y, h.x, -dreg[s].x * h.y);
-        }
-      } else {
-#pragma unroll
-        for (int s = 0; s < 16; s++) {
-          const float2 x = a.data_cg ? __ldcg(dp + t + T * s) : __ldg(dp + t + T * s);
-          const float2 h = __ldg(hp + t + T * s);
-          v[s].x = fmaf(x.x, h.x, x.y * h.y);
-          v[s].y = fmaf(x.y, h.x, -x.x * h.y);
-        }
+      for (int s = 0; s < 16; s++) {
+        // data_cg: data written earlier in the same launch
+        const float2 x = a.data_cg ? __ldcg(dp + t + T * s) : __ldg(dp + t + T * s);
+        const float2 h = __ldg(hp + t + T * s);
+        v[s].x = fmaf(x.x, h.x, x.y * h.y);
+        v[s].y = fmaf(x.y, h.x, -x.x * h.y);
       }
     } else {
 #pragma unroll
@@ -371,7 +342,7 @@ __device__ __forceinline__ void flat_range(const FlatArgs &a, long long ibeg, lo
     inverse_passes<N>(v, buf, a.twid, t);
     // Thread t now holds z[t + T*q] in v[q].
     // Keys: a double-buffered slot array when the bins fit, else buf itself.
-    const int nb = (MODE == MODE_GATE) ? 1 : a.nb;
+    const int nb = a.nb;
     unsigned long long *keys;
     if (small_keys) {
       keys = kslots + ((g * 2 + (int)(item & 1)) * KEYCAP);
@@ -469,70 +440,53 @@ __device__ __forceinline__ void flat_range(const FlatArgs &a, long long ibeg, lo
     }
     group_sync(T);
     if (live) {
-      if constexpr (MODE == MODE_PEAKS) {
-        const long long obase = (long long)row * nb;
-        if (small_keys) {
-          int cnt = 0;
-          for (int b = t; b < nb; b += T) {
-            const unsigned long long kk = keys[b];
-            long long ix = -1;
-            float2 val = make_float2(0.f, 0.f);
-            if (kk != 0ull) {
-              const int k = (int)(~(unsigned)kk);
-              ix = k;
-              val = buf[pad16(k)];
-              cnt++;
-            }
-            a.out_idx[(obase + b) * a.rs] = ix;
-            a.out_val[(obase + b) * a.rs] = val;
-            if (a.host_rec) store_host(a.host_rec, obase + b, ix, val);
+      const long long obase = (long long)row * nb;
+      if (small_keys) {
+        int cnt = 0;
+        for (int b = t; b < nb; b += T) {
+          const unsigned long long kk = keys[b];
+          long long ix = -1;
+          float2 val = make_float2(0.f, 0.f);
+          if (kk != 0ull) {
+            const int k = (int)(~(unsigned)kk);
+            ix = k;
+            val = buf[pad16(k)];
+            cnt++;
           }
-          if (a.out_cnt) {
-            const int c = __reduce_add_sync(gmask, cnt);
-            if (c && lane == (T >= 32 ? 0 : (lane & ~(T - 1)))) atomicAdd(a.out_cnt + row, c);
-          }
-        } else {
-          // Many bins: keys live in buf, so the lane holding each winner writes it.
-#pragma unroll
-          for (int q = 0; q < 16; q++) {
-            if (cand & (1u << q)) {
-              const int kq = t + T * q;
-              const int bin = bin_of(kq - a.ws, bs, inv_bs);
-              const unsigned long long kk = keys[bin];
-              if ((unsigned)(~(unsigned)kk) == (unsigned)kq) {
-                a.out_idx[(obase + bin) * a.rs] = kq;
-                a.out_val[(obase + bin) * a.rs] = make_float2(v[q].x, v[q].y);
-              }
-            }
-          }
-          int cnt = 0;
-          for (int b = t; b < nb; b += T) {
-            if (keys[b] == 0ull) {
-              a.out_idx[(obase + b) * a.rs] = -1;
-              a.out_val[(obase + b) * a.rs] = make_float2(0.f, 0.f);
-            } else {
-              cnt++;
-            }
-          }
-          if (a.out_cnt) {
-            const int c = __reduce_add_sync(gmask, cnt);
-            if (c && lane == (T >= 32 ? 0 : (lane & ~(T - 1)))) atomicAdd(a.out_cnt + row, c);
-          }
+          a.out_idx[(obase + b) * a.rs] = ix;
+          a.out_val[(obase + b) * a.rs] = val;
+          if (a.host_rec) store_host(a.host_rec, obase + b, ix, val);
+        }
+        if (a.out_cnt) {
+          const int c = __reduce_add_sync(gmask, cnt);
+          if (c && lane == (T >= 32 ? 0 : (lane & ~(T - 1)))) atomicAdd(a.out_cnt + row, c);
         }
       } else {
-        const unsigned long long kk = keys[0];
-        const float m2 = __uint_as_float((unsigned)(kk >> 32));
-        const bool fire = kk != 0ull && sqrtf(m2) >= a.gate;
-        if (a.coarse_out) {
-          if (t == 0) a.coarse_out[row] = kk != 0ull ? sqrtf(m2) : 0.f;
-        } else if (fire) {
-          if (t == 0) a.fire_list[atomicAdd(a.fire_count, 1)] = row;
-        } else {
-          const long long obase = (long long)row * a.full_nb;
-          for (int b = t; b < a.full_nb; b += T) {
+        // Many bins: keys live in buf, so the lane holding each winner writes it.
+#pragma unroll
+        for (int q = 0; q < 16; q++) {
+          if (cand & (1u << q)) {
+            const int kq = t + T * q;
+            const int bin = bin_of(kq - a.ws, bs, inv_bs);
+            const unsigned long long kk = keys[bin];
+            if ((unsigned)(~(unsigned)kk) == (unsigned)kq) {
+              a.out_idx[(obase + bin) * a.rs] = kq;
+              a.out_val[(obase + bin) * a.rs] = make_float2(v[q].x, v[q].y);
+            }
+          }
+        }
+        int cnt = 0;
+        for (int b = t; b < nb; b += T) {
+          if (keys[b] == 0ull) {
             a.out_idx[(obase + b) * a.rs] = -1;
             a.out_val[(obase + b) * a.rs] = make_float2(0.f, 0.f);
+          } else {
+            cnt++;
           }
+        }
+        if (a.out_cnt) {
+          const int c = __reduce_add_sync(gmask, cnt);
+          if (c && lane == (T >= 32 ? 0 : (lane & ~(T - 1)))) atomicAdd(a.out_cnt + row, c);
         }
       }
     }
@@ -817,6 +771,8 @@ flat_kernel(const FlatArgs a) {
 
 // Listed mode on its own: the output rows of a device row list (the
 // hierarchical refine, mfb_run_rows) with bins that flatw_kernel does not take.
+// A contiguous range per CTA: unlike a dense block's pairs, whose loud data rows are
+// neighbours, a list's rows come in arbitrary order and every one is a survivor.
 template <int N>
 __global__ void __launch_bounds__(FlatGeo<N>::CTA, FlatGeo<N>::MINB)
 rows_kernel(const FlatArgs a) {
@@ -828,7 +784,7 @@ rows_kernel(const FlatArgs a) {
   const long long per = items / gridDim.x, extra = items % gridDim.x;
   const long long ibeg = blockIdx.x * per + (blockIdx.x < extra ? blockIdx.x : extra);
   const long long iend = ibeg + per + (blockIdx.x < extra ? 1 : 0);
-  flat_range<N, MODE_PEAKS, false>(a, ibeg, iend, smem);
+  flat_range<N>(a, ibeg, iend, smem);
 }
 
 }  // namespace mfb
