@@ -618,3 +618,70 @@ def test_short_runs(n, nd, nt, nb, thr):
     assert (idx == -7).all()
     i, v = f.run_device(**kw)
     assert not (i == -7).any()
+
+
+@pytest.mark.parametrize("binsize, win, thr", [
+    ("n/16", None, 0.0),             # every warp's rows lie in one bin
+    ("n/16", None, 3.6),
+    ("n", None, 0.0),
+    ("n/50 + 3", (17, -9), 0.0),     # bins shared by lanes at random
+    ("n/50 + 3", (17, -9), 3.6),
+    ("n/3000", (5, -1), 3.6),        # more bins than a unit sees lags of
+])
+def test_longest_transform(binsize, win, thr):
+    """n = 2^20, where a row spans two warps and both passes exchange across the CTA: 37 pairs
+    (more items than ring slots, the last one half empty), dense against the same rows
+    listed and, for two pairs, against FP64; each twice, on the counters and records that the
+    first run left."""
+    import torch
+    mf = _mf()
+    from apogee_b200 import _lib
+    L = _lib.lib()
+    n, nd, nt = 1 << 20, 1, 37
+    binsize = eval(binsize.replace("/", "//"), {"n": n})
+    lo, hi = (0, n) if win is None else (win[0], n + win[1])
+    g = torch.Generator(device="cuda").manual_seed(20)
+    D = torch.randn(nd, n, dtype=torch.complex64, device="cuda", generator=g)
+    H = torch.randn(nt, n, dtype=torch.complex64, device="cuda", generator=g)
+    thr *= np.sqrt(n)
+    f = mf.MatchedFilter(n, nd, nt)
+    f.set_data(D)
+    f.set_templates(H)
+    nb = L.mfb_nbins(n, binsize, lo, hi)
+    rows = torch.randperm(nt, device="cuda", generator=g).to(torch.int32)
+    count = torch.tensor([nt], dtype=torch.int32, device="cuda")
+    for _ in range(2):
+        i, v = f.run_device(binsize=binsize, threshold=thr, window=(lo, hi))
+        li, lv = torch.full_like(i, -7), torch.zeros_like(v)
+        f._bind_stream()
+        _lib.check(L.mfb_run_rows(f._plan, 0, nd, 0, nt, rows.data_ptr(), count.data_ptr(), nt, binsize, thr,
+                                  lo, hi, li.data_ptr(), lv.data_ptr(), None))
+        assert torch.equal(i, li) and torch.equal(v, lv)
+        sel = [0, nt - 1]
+        z = oracle.correlate(D.cpu().numpy(), H[sel].cpu().numpy())
+        got = i[:, sel].cpu().numpy()
+        assert (got >= 0).any()
+        assert not parity.compare(got, v[:, sel].cpu().numpy(), z, binsize, thr, (lo, hi))
+
+
+def test_two_streams_at_32768():
+    """Blocks of more pairs than the cluster kernel takes, enqueued on two streams, share the
+    plan's scratch one after another."""
+    import torch
+    mf = _mf()
+    n, nd, nt = 32768, 2, 300
+    g = torch.Generator(device="cuda").manual_seed(7)
+    f = mf.MatchedFilter(n, nd, nt)
+    f.set_data(torch.randn(nd, n, dtype=torch.complex64, device="cuda", generator=g))
+    f.set_templates(torch.randn(nt, n, dtype=torch.complex64, device="cuda", generator=g))
+    want = [f.run_device(binsize=n // 16), f.run_device(binsize=n // 60 + 1, threshold=500.0)]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    got = []
+    for k in range(8):
+        with torch.cuda.stream(streams[k & 1]):
+            got.append(f.run_device(binsize=n // 16) if k % 3 else f.run_device(binsize=n // 60 + 1, threshold=500.0))
+    torch.cuda.synchronize()
+    for k, (i, v) in enumerate(got):
+        wi, wv = want[0 if k % 3 else 1]
+        assert torch.equal(i, wi) and torch.equal(v, wv)
