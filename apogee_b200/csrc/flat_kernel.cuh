@@ -505,10 +505,11 @@ __device__ __forceinline__ void flat_range(const FlatArgs &a, long long ibeg, lo
 // n = 4096, CUDA events, L2 flushed), while flat_range's short dynamic ranges
 // in the batched kernel need the entry barrier and the coherent-load switch.
 //
-// MINB: CTAs per SM.  A run with no more items than two CTAs per SM take at once has no
-// use for a third and takes the form with 128 registers, which has all 32 loads of a
+// MINB: CTAs per SM.  A run with no more items than one CTA per SM fewer takes at once has
+// no use for the last and takes the form with 128 registers, which has all 32 loads of a
 // pair in flight: us at threshold 0, three CTAs / two, n = 128, 4 x 100 pairs 12.5 / 10.6;
-// n = 256, 2 x 37 pairs of 64 bins 12.7 / 10.9; n = 1024, 1 x 16 of 64 14.5 / 12.7.
+// n = 256, 2 x 37 pairs of 64 bins 12.7 / 10.9; n = 1024, 1 x 16 of 64 14.5 / 12.7;
+// n = 8192, two / one, 9 x 16 of 64 14.7 / 10.6, of 128 24.9 / 18.8.
 template <int N, int MODE, int MINB = FlatGeo<N>::MINB>
 __global__ void __launch_bounds__(FlatGeo<N>::CTA, MINB)
 flat_kernel(const FlatArgs a) {

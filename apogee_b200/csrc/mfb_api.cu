@@ -105,7 +105,7 @@ struct NConst {
   int grid_peaks = 0, grid_gate = 0, grid_fwd = 0;
   int cta = 0, smem = 0, g = 0;
   int grid_rows = 0;
-  int grid_few = 0;             // items up to which flat_kernel runs two CTAs per SM
+  int grid_few = 0;             // items up to which flat_kernel runs one CTA per SM fewer
   // n = 128 ... 1024: the tables as (wr, wr, wi, wi) records for two pairs per
   // thread (the transforms of large2_kernel.cuh)
   float4 *twid2 = nullptr;
@@ -181,10 +181,10 @@ static int make_const(int device, NConst &c) {
     c.gridw = b5 * sms;
     c.gridw_gate = b6 * sms;
   }
-  if constexpr (Geo::MINB == 3) {
-    CUDA_TRY(cudaFuncSetAttribute(flat_kernel<N, MODE_PEAKS, 2>,
+  if constexpr (Geo::MINB > 1) {
+    CUDA_TRY(cudaFuncSetAttribute(flat_kernel<N, MODE_PEAKS, Geo::MINB - 1>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, Geo::SMEM));
-    c.grid_few = 2 * sms;
+    c.grid_few = (Geo::MINB - 1) * sms;
   }
   c.grid_rows = b4 * sms;
   c.grid_peaks = b1 * sms;
@@ -242,10 +242,10 @@ static cudaError_t launch_flatw(int n, const NConst &c, FlatArgs a, cudaStream_t
 template <int N>
 static void launch_peaks_n(const NConst &c, const FlatArgs &a, cudaStream_t s) {
   using Geo = FlatGeo<N>;
-  if constexpr (Geo::MINB == 3) {
+  if constexpr (Geo::MINB > 1) {
     const long long items = ((long long)a.nd * a.nt + Geo::G - 1) / Geo::G;
     if (items <= c.grid_few) {
-      flat_kernel<N, MODE_PEAKS, 2><<<(int)items, Geo::CTA, Geo::SMEM, s>>>(a);
+      flat_kernel<N, MODE_PEAKS, Geo::MINB - 1><<<(int)items, Geo::CTA, Geo::SMEM, s>>>(a);
       return;
     }
   }

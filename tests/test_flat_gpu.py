@@ -296,17 +296,16 @@ def _same_up_to_near_ties(i1, i2, z):
 
 
 @pytest.mark.parametrize("nd,nt,binsize,threshold", [
-    (16, 1024, 256, 0.0),     # the benchmark block: data rows shared by both pairs of an item
-    (5, 77, 512, 3.0),        # odd nt: items straddle data rows; thresholded
-    (3, 1, 64, 0.0),          # one template: every item mixes data rows; 64 bins
-    (1, 3, 4096, 2.0),        # odd pair count: the last item's second pair is absent
+    (16, 1024, 256, 0.0),     # the benchmark block
+    (5, 77, 512, 3.0),        # odd nt, thresholded
+    (3, 1, 768, 0.0),         # one template: every pair on its own data row; a short last bin
+    (1, 3, 4096, 2.0),        # fewer pairs than slots, one bin
 ])
 def test_packed_kernel_matches_one_pair_kernel_and_oracle(nd, nt, binsize, threshold):
-    """n = 4096 runs over the whole window use the kernel that carries two
-    pairs per thread in packed FP32x2 arithmetic.  It must meet the oracle's
-    bar and equal the one-pair kernel bit for bit (dense, listed and record
-    output, counts: both form their twiddles with the same operations); listed
-    rows equal the dense run's rows bit for bit."""
+    """n = 4096, bins of whole 256-lag blocks: the kernel that mfb_set_packed switches on
+    (flatw_kernel) must meet the oracle's bar and equal the general kernel bit
+    for bit (dense, listed and record output, counts: both form their twiddles
+    with the same operations); listed rows equal the dense run's rows bit for bit."""
     import torch
     import apogee_b200 as mf
     from apogee_b200 import _lib
@@ -457,15 +456,15 @@ def test_threshold_skips_only_pairs_without_candidates(n, win):
         assert (out["index"] >= 0).any(-1).sum() < 27
 
 
-@pytest.mark.parametrize("n", [64, 128, 256, 1024, 4096])
+@pytest.mark.parametrize("n", [64, 128, 256, 1024, 4096, 8192])
 @pytest.mark.parametrize("thr", [0.0, 4.0])
 def test_few_items_give_the_same_bits(n, thr):
-    """Runs of up to two CTAs per SM take flat_kernel's form with more registers: at the
-    line, one pair past it and in pieces, general bins, against each other."""
+    """Runs of up to two CTAs per SM (n = 8192: one) take flat_kernel's form with more
+    registers: at the line, one pair past it and in pieces, general bins, against each other."""
     import torch
     mf = _mf()
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    line = 2 * sms * max(1, 4096 // n)                 # pairs that fill two CTAs per SM
+    line = (2 if n <= 4096 else 1) * sms * max(1, 4096 // n)   # pairs that fill those CTAs
     g = torch.Generator(device="cuda").manual_seed(n)
     nt = line + 1
     D = torch.randn(1, n, dtype=torch.complex64, device="cuda", generator=g)
