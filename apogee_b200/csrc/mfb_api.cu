@@ -646,6 +646,7 @@ LargeScratch::~LargeScratch() {
 static int large_scratch(mfb_plan *p, long long pairs, size_t nb);
 extern "C" int mfb_destroy(mfb_plan *p);
 constexpr long long CLUSTER_PAIRS = 64;   // see cluster_mode
+constexpr size_t EAGER_BINS = 512;        // 2 x 6.7 MB of records
 
 // scratch: the large-n scratch to use, or nullptr for the plan's own; eager: allocate
 // what a run without an allocation needs.
@@ -682,9 +683,9 @@ static int create_plan(mfb_plan **out, size_t n, int ndata, int ntmpl, int devic
   CUDA_TRY(cudaDeviceSynchronize());
   if (is_large(n)) p->ls = scratch ? scratch : std::make_shared<LargeScratch>(device);
   if (eager && n == 32768 && (long long)ndata * ntmpl > CLUSTER_PAIRS) {
-    // runs at this length do not allocate (smaller blocks, lists and captured runs take
-    // the cluster kernel, which has no scratch)
-    r = large_scratch(p, (long long)ndata * ntmpl, 1);
+    // runs at this length do not allocate, up to EAGER_BINS bins (smaller blocks, lists and
+    // captured runs take the cluster kernel, which has no scratch)
+    r = large_scratch(p, (long long)ndata * ntmpl, EAGER_BINS);
     if (r != MFB_OK) { mfb_destroy(p); return r; }
   }
   *out = p;

@@ -60,10 +60,10 @@ int mfb_create(mfb_plan **out, size_t n, int ndata, int ntmpl, int device);
    uses owner's scratch for large n instead of one of its own.  Runs on different streams
    are ordered; the two plans must not be used from two threads at once.
    That scratch (of the persistent four-step kernel: n >= 65536, and n = 32768 in dense
-   blocks of more than 64 pairs) is allocated by mfb_create at n = 32768 and by a plan's
-   first run above, and grown by a run that needs more: rows of the pairs in flight, at
-   most 205 MiB (240 MiB at n = 2^20), and 64 bytes per bin of those pairs (0.4 MB at 16
-   bins and n = 65536, 27 MB at 1024).  A device with less room gets less, at some cost
+   blocks of more than 64 pairs) is allocated by mfb_create at n = 32768 (for 512 bins) and
+   by a plan's first run above, and grown by a run that needs more: rows of the pairs in flight, at
+   most 205 MiB (240 MiB at n = 2^20), and 32 bytes per bin of those pairs (0.2 MB at 16
+   bins and n = 65536, 13 MB at 1024).  A device with less room gets less, at some cost
    in speed. */
 int mfb_create_sharing(mfb_plan **out, size_t n, int ndata, int ntmpl, mfb_plan *owner);
 /* Replaces ap_mf_destroy (src/matchfilt.c:135-146). */
@@ -78,7 +78,11 @@ int mfb_set_templates(mfb_plan *p, int t0, int count, const void *spec);
    idx: int64 [nd*nt*nb]; val: complex64 [nd*nt*nb]; counts: int32 [nd*nt] or NULL.
    Returns 0, not the total of threshold crossings that ap_mf_run returns
    (matchedfilter.h:66-71): the run is only enqueued here, and the total would
-   need a host synchronisation.  Sum `counts` after synchronising instead. */
+   need a host synchronisation.  Sum `counts` after synchronising instead.
+   Runs of one plan on different streams are ordered where they share scratch
+   (n >= 32768).  A run captured by the caller is not: at n >= 65536 its graph must not
+   overlap another run of the plan (or of one that shares its scratch), or both give
+   wrong results; later runs are not affected. */
 int mfb_run(mfb_plan *p, int d0, int nd, int t0, int nt, size_t binsize, float threshold,
             size_t start, size_t end, int64_t *idx, void *val, int32_t *counts);
 /* Same as mfb_run, but the output is one array of 16-byte records laid out
@@ -106,7 +110,8 @@ int mfb_set_packed(mfb_plan *p, int on);
    threads, one per SM.  Same arithmetic, identical results.  Without a call, a
    run takes the faster on a B200: at n = 32768 mode 1 for row lists, dense blocks
    of up to 64 pairs and captured runs, mode 0 for larger blocks (1.7x faster
-   at 1024 pairs); at 65536 mode 0. */
+   at 1024 pairs); at 65536 mode 0.  A call fixes the mode for the plan's life, also
+   mode 1, which at n = 32768 then serves large blocks too. */
 int mfb_set_cluster(mfb_plan *p, int mode);
 /* MFB_ERR_CUDA, once, if a dependency wait inside a run of this plan ran out (the
    outputs of that run are then not valid).  Reads a host word: call it after

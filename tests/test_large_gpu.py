@@ -1,5 +1,5 @@
-"""Transforms larger than one CTA (n = 32768 ... 2^20): the two-pass four-step
-path, against the FP64 oracle."""
+"""Transforms larger than one CTA (n = 32768 ... 2^20): the four-step kernels, against
+the FP64 oracle and one another, and the scratch they share."""
 import numpy as np
 import pytest
 
@@ -358,6 +358,7 @@ def _held(make):
     free = torch.cuda.mem_get_info()[0]
     out = make()
     torch.cuda.synchronize()
+    torch.cuda.empty_cache()
     return free - torch.cuda.mem_get_info()[0], out
 
 
@@ -400,7 +401,9 @@ def test_scratch_is_what_the_runs_need():
     L.mfb_destroy(p)
     held, h = _held(lambda: mf.HierarchicalFilter(n, 2, 300, band=16384, coarse="fp32"))
     held_p, p = _held(lambda: _plan(n, 2, 300))
-    assert held_p <= rows(2, 300) + 213 * MB                     # 203.5 MiB of rows and few records
+    assert held_p <= rows(2, 300) + 213 * MB                     # rows, and records for 512 bins
+    allocated, _ = _held(lambda: [_run_plan(p, n, 2, 300, nb)[0].sum().item() for nb in (1, 64, 512)])
+    assert allocated <= 0                                        # no run at this length allocates
     L.mfb_destroy(p)
     del h
 
