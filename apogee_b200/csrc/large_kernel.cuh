@@ -1,5 +1,5 @@
 // Fused matched filter for transforms larger than one CTA holds
-// (n = 32768 ... 524288): a two-pass four-step through an L2-sized scratch.
+// (n = 32768 ... 2^20): a two-pass four-step, one launch per pass, through a scratch.
 //
 // With n = N1 * N2, f = f1 + N1 f2 and k = N2 k1 + k2 (f1, k1 < N1; f2, k2 < N2):
 //
@@ -15,8 +15,9 @@
 //           correlation series is never written.
 //   finalize  candidate records -> (index, value) outputs and crossing counts.
 //
-// These per-batch kernels serve mfb_run_large_static, whose fixed scratch of
-// 8 MiB has no room for large2_kernel's ring; plans run that kernel.  What it shares
+// These launches per batch serve mfb_run_large_static, whose fixed scratch of 8 MiB
+// has no room for large2_kernel's ring, and the short runs of plans that gain nothing
+// from that kernel (short_run, mfb_api.cu); all else runs there.  What it shares
 // (arguments, pair order, twiddle tables, keys, records) and the forward
 // transform of series blocks are here too.  Pairs run in batches that fit
 // the scratch and are ordered template-major so the data rows

@@ -47,8 +47,8 @@ FLOPS_PER_PAIR = lambda n: 5 * n * int(np.log2(n)) + 9 * n   # the reference's o
 TC_FLOPS_PER_PAIR = 12 * 128 * 64 * 16 * 2 / 8
 # DRAM bytes per launch from one ncu capture of the same kernels on this workload
 # (profiles/coarse_tc_ws_band512_16x1024.md, profiles/flatw_kernel.md).
-TRAFFIC_COARSE_TC = 4.347e6
-TRAFFIC_FLAT = 34.18e6
+TRAFFIC_COARSE_TC = 4.344e6
+TRAFFIC_FLAT = 34.12e6
 
 
 def measured_peaks():

@@ -2,9 +2,9 @@
 (tests/test_adversarial.py in the reference: peaks on bin and window edges,
 ragged bins, amplitude scale, zero inputs, a single frequency bin, a
 threshold equal to the peak, binsize 1), run through every kernel family
-here -- the one-pair kernel (n = 64 ... 16384), the packed n = 4096 kernel
-(whole window, bins a multiple of 32 lags) and the two-pass kernels
-(n >= 32768) -- against the FP64 oracle."""
+here -- the general single-block kernel (n = 64 ... 16384), the one for bins and
+windows of whole n/16 blocks, and the four-step kernels (n >= 32768) -- against
+the FP64 oracle."""
 import numpy as np
 import pytest
 

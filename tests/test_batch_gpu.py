@@ -134,7 +134,7 @@ def test_plan_errors():
 
 
 def test_own_launch_jobs_beside_the_persistent_launch():
-    """Jobs forced onto their own launches (single-CTA 8192/16384, two-pass
+    """Jobs forced onto their own launches (single-CTA 8192/16384, four-step
     65536, a series job) next to persistent ones: same results, also replayed
     from a graph."""
     import torch

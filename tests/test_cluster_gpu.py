@@ -1,6 +1,6 @@
 """The thread-block-cluster kernel (n = 32768 and 65536: one cluster per
 pair, the spectrum held in distributed shared memory between the passes)
-against the two-pass kernels it replaces (same arithmetic: identical outputs)
+against the other four-step kernels (same arithmetic: identical outputs)
 and against the FP64 oracle: dense blocks with more pairs than clusters,
 windows, thresholds, ragged bins, listed rows and the hierarchical refine."""
 import numpy as np
@@ -16,7 +16,7 @@ def noise(rng, shape):
 
 
 def _modes(f, **kw):
-    """Run with the two cluster geometries and with the two-pass kernels."""
+    """Run with the two cluster geometries and without clusters."""
     from apogee_b200 import _lib
     L = _lib.lib()
     outs = []
@@ -104,9 +104,8 @@ def test_cluster_listed_rows(n):
 
 def test_cluster_hierarchical_refine_and_host_table():
     """Hierarchical filter at n = 32768 with the cluster refine: its table
-    equals the two-pass refine's, and the host-table run (replayed as one
-    CUDA graph at this length, since no step reads the survivor count on the
-    host) matches the device table over changing data."""
+    equals the refine's without clusters, and the host-table run (replayed as one
+    CUDA graph) matches the device table over changing data."""
     import apogee_b200 as mf
     from apogee_b200 import _lib
     n, nd, nt = 32768, 4, 64

@@ -339,7 +339,7 @@ def test_packed_kernel_matches_one_pair_kernel_and_oracle(nd, nt, binsize, thres
     rows = np.random.default_rng(7).permutation(nd * nt)[: max(1, (nd * nt) // 2) | 1]
     rows_d = torch.as_tensor(rows.astype(np.int32), device="cuda")
     cnt_d = torch.tensor([rows.size], dtype=torch.int32, device="cuda")
-    nb = n // binsize
+    nb = -(-n // binsize)
     _lib.check(L.mfb_set_packed(f._plan, 1))
     f._bind_stream()
     idx = torch.full((nd * nt * nb,), -7, dtype=torch.int64, device="cuda")

@@ -218,8 +218,8 @@ def test_repeated_calls_replay_one_graph_with_fresh_inputs():
 @pytest.mark.parametrize("n,band,coarse", [(4096, 512, "fp16x3"), (4096, 1024, "fp32"),
                                            (65536, 4096, "fp32")])
 def test_host_table_other_kinds_and_lengths(n, band, coarse):
-    """The host-table run for the other coarse kinds and for the two-pass
-    large-n refine (no graph there: its batches are sized on the host)."""
+    """The host-table run for the other coarse kinds and for the
+    four-step refine of large n."""
     import torch
     nd, nt, bs = 3, 12, n // 16
     rng = np.random.default_rng(n + band)
