@@ -561,7 +561,7 @@ extern "C" size_t mfb_nbins(size_t n, size_t binsize, size_t start, size_t end) 
 }
 
 // ---------------------------------------------------------------- flat plan
-// large2_kernel's scratch, of one plan or shared (mfb_share_scratch): rows, and counters
+// large2_kernel's scratch, of one plan or shared (mfb_create_sharing): rows, and counters
 // and candidate records.  The latter are zero between launches, whatever the plan
 // and its layout of them, and are there twice: [0] for runs that follow one another and
 // [1] for runs captured by a caller, whose order nobody here knows.
@@ -874,6 +874,13 @@ static cudaError_t scratch_begin(const mfb_plan *p) {
 static cudaError_t scratch_end(const mfb_plan *p) {
   return capturing(p->stream) ? cudaSuccess : cudaEventRecord(p->ls->used, p->stream);
 }
+// Whether the plan's stream is being captured by a caller, whose graph then holds the
+// scratch's addresses.
+static bool note_capture(mfb_plan *p) {
+  const bool foreign = capturing(p->stream) && !p->own_capture;
+  if (foreign) p->ls->captured = true;
+  return foreign;
+}
 // Series blocks that fit the scratch.
 static int large_rows(const mfb_plan *p) { return (int)(p->ls->rows_bytes / (p->n * sizeof(float2))); }
 
@@ -913,7 +920,7 @@ static int run_batches(mfb_plan *p, LargeArgs a) {
   const LargeScratch &s = *p->ls;
   a.Y = reinterpret_cast<float2 *>(s.rows);
   a.rec = reinterpret_cast<uint4 *>(s.state[1]);
-  if (capturing(p->stream) && !p->own_capture) p->ls->captured = true;
+  note_capture(p);
   const int most = (int)std::min<size_t>(large_rows(p), s.state_bytes / ((size_t)a.nb * sizeof(uint4)));
   CUDA_TRY(scratch_begin(p));
   for (a.pair0 = 0; a.pair0 < a.total; a.pair0 += most) {
@@ -975,8 +982,7 @@ static int run_large(mfb_plan *p, int d0, int nd, int t0, int nt, const int32_t 
   g.tw2 = c.c2->twid2;
   g.anchors = c.anchors;
   g.Y = reinterpret_cast<float4 *>(p->ls->rows);
-  const int foreign = capturing(p->stream) && !p->own_capture;
-  if (foreign) p->ls->captured = true;
+  const int foreign = note_capture(p);
   g.ring = large_ring(p, list ? LLONG_MAX - 1 : a.total, nb);
   g.ctl = reinterpret_cast<Large2Ctl *>(p->ls->state[foreign]);
   g.rec = reinterpret_cast<uint4 *>(p->ls->state[foreign] + large_ctl_bytes(g.ring));
@@ -1145,6 +1151,7 @@ extern "C" int mfb_forward(mfb_plan *p, const void *series, size_t nseries,
     f.starts = (const unsigned long long *)starts_dev;
     f.spectra = (float2 *)spectra;
     f.scale = 1.0f / (float)p->n;
+    note_capture(p);
     CUDA_TRY(scratch_begin(p));
     for (long long p0 = 0; p0 < nblocks; p0 += large_rows(p)) {
       a.pair0 = p0;

@@ -623,6 +623,44 @@ def test_short_runs(n, nd, nt, nb, thr):
     assert not (i == -7).any()
 
 
+def test_outgrown_scratch_of_a_captured_forward_stays():
+    """The same for a captured forward transform, which is all that a plan at n = 32768 with few
+    pairs uses the scratch for."""
+    import torch
+    from apogee_b200 import _lib
+    L = _lib.lib()
+    n, nt = 32768, 2
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(50 * n, dtype=torch.complex64, device="cuda", generator=g)
+    st = np.arange(50, dtype=np.uint64) * n
+    st_d = torch.from_numpy(st.astype(np.int64)).cuda()
+    p = _plan(n, 1, nt)
+    spec = torch.zeros(2, n, dtype=torch.complex64, device="cuda")
+
+    def forward():
+        _lib.check(L.mfb_set_stream(p, torch.cuda.current_stream().cuda_stream))
+        _lib.check(L.mfb_forward(p, x.data_ptr(), x.numel(), st_d.data_ptr(), 2, spec.data_ptr()))
+    forward()
+    torch.cuda.synchronize()
+    want = spec.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        forward()
+    _lib.check(L.mfb_set_stream(p, torch.cuda.current_stream().cuda_stream))
+    H = torch.randn(nt, n, dtype=torch.complex64, device="cuda", generator=g)
+    _lib.check(L.mfb_set_templates(p, 0, nt, H.data_ptr()))
+    lo, hi = np.zeros(50, np.uint64), np.full(50, n, np.uint64)
+    rec = torch.empty(50 * nt * 16 * 2, dtype=torch.int64, device="cuda")
+    _lib.check(L.mfb_run_series_records(p, x.data_ptr(), x.numel(), st.ctypes.data, lo.ctypes.data, hi.ctypes.data,
+                                        50, 0, nt, n // 16, 0.0, rec.data_ptr(), None))   # the scratch grows
+    for _ in range(2):
+        spec.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(spec, want)
+    L.mfb_destroy(p)
+
+
 @pytest.mark.parametrize("binsize, win, thr", [
     ("n/16", None, 0.0),             # every warp's rows lie in one bin
     ("n/16", None, 3.6),
