@@ -884,18 +884,22 @@ static bool note_capture(mfb_plan *p) {
 // Series blocks that fit the scratch.
 static int large_rows(const mfb_plan *p) { return (int)(p->ls->rows_bytes / (p->n * sizeof(float2))); }
 
+constexpr int MANY_BINS = 1024;   // see short_run
 // The cluster kernel's geometry for a run (1 or 2), or 0 for large2_kernel.  At
 // n = 32768, unless mfb_set_cluster says otherwise, lists and dense runs of up to
 // CLUSTER_PAIRS pairs take the cluster kernel (one cluster per pair has the
 // shorter latency: 1 pair 16 against 19 us, 16 pairs 20 against 21, 51 listed rows
 // of 4096 56 against 62), larger blocks large2_kernel (128 pairs 34 against
-// 38 us, 1024 pairs 152 against 258).  A captured run at that length keeps to the
+// 38 us, 1024 pairs 152 against 258).  `loose` bins (up to MANY_BINS of them, not shared by
+// warps, at threshold 0) move the line to twice as many pairs: 96 pairs of 50 bins 38
+// against 45 us in the launches per batch (short_run) and 50 in large2_kernel, 128 51
+// against 51 and 57.  A captured run at that length keeps to the
 // cluster kernel, which has no scratch: its graph may run beside other runs of the
 // plan.
-static int cluster_mode(const mfb_plan *p, bool listed, long long pairs) {
+static int cluster_mode(const mfb_plan *p, bool listed, long long pairs, bool loose = false) {
   int mode = p->cluster;
   if (mode < 0)
-    mode = p->n == 32768 && (listed || pairs <= CLUSTER_PAIRS || capturing(p->stream)) ? 1 : 0;
+    mode = p->n == 32768 && (listed || pairs <= (loose ? 2 : 1) * CLUSTER_PAIRS || capturing(p->stream)) ? 1 : 0;
   return mode > 0 && p->lc && p->lc->cl[mode - 1].C > 0 ? mode : 0;
 }
 
@@ -903,16 +907,19 @@ static int cluster_mode(const mfb_plan *p, bool listed, long long pairs) {
 // large2_kernel, whose ring neither fills nor overlaps the two passes on so few items:
 // where bins are not whole multiples of N2 lags, either at threshold 0 (every lag a
 // candidate) or with so many bins that writing them out counts; and a pair or two of the
-// longest transform.  Up to SHORT_POINTS lags in all, where the two meet.  B200, us here
+// longest transform.  The limits, in lags of all pairs, are where the two meet.  B200, us here
 // against large2_kernel, 1 x pairs: 50 ragged bins at threshold 0, n = 65536, 16 pairs 30 / 38,
-// 128 92 / 98, 256 157 / 175 (one launch of 205 MB; in 64 MB batches 183); n = 524288, 4 pairs
-// 39 / 48; 4096 bins above it, n = 65536, 8 pairs 22 / 35; n = 2^20, one pair 28 / 34.  Above
-// a threshold with few bins large2_kernel wins from two pairs on (n = 65536, 16 pairs 24 / 19).
-constexpr long long SHORT_POINTS = 1ll << 23;
+// 128 92 / 98; n = 524288, 4 pairs 39 / 48; 4096 bins at threshold 0, n = 65536, 16 pairs 54 / 58, 32
+// 81 / 63; above it, n = 65536, 8 pairs 22 / 35, 256 154 / 186, n = 131072, 256 323 / 275; n = 2^20, one
+// pair 28 / 34.  Above a threshold with few bins large2_kernel wins from two pairs on
+// (n = 65536, 16 pairs 24 / 19).
 static bool short_run(const LargeArgs &a) {
-  if (a.list || a.n == 32768) return false;   // cluster_mode has that length's rule
+  if (a.list) return false;
   if (a.n == 1 << 20 && a.total <= 2) return true;
-  return a.seg == 0 && a.total * a.n <= SHORT_POINTS && (a.t2 > 0.f ? a.nb > 1024 : a.nb <= 1024);
+  const long long points = a.total * a.n;
+  if (a.seg > 0) return false;
+  if (a.t2 > 0.f) return a.nb > MANY_BINS && points <= 1 << 24;
+  return a.nb <= MANY_BINS ? points <= 1 << 23 : a.n <= 65536 && points <= 1 << 20;
 }
 // The launches per batch, in the scratch's rows, with the records of captured runs
 // (zeroed here first).
@@ -941,7 +948,9 @@ static int run_large(mfb_plan *p, int d0, int nd, int t0, int nt, const int32_t 
   if (nb > (size_t)LARGE_MAX_BINS)
     return fail(MFB_ERR_UNSUPPORTED, "n=%zu supports at most %d bins per pair", p->n, LARGE_MAX_BINS);
   const LargeConst &c = *p->lc;
-  const int cl = cluster_mode(p, list != nullptr, (long long)nd * nt);
+  const int bs = binsize > p->n ? (int)p->n : (int)binsize, seg = bin_lanes(bs, (int)start, c.N1, c.N2);
+  const bool loose = seg == 0 && !(threshold > 0.f) && nb <= (size_t)MANY_BINS;
+  const int cl = cluster_mode(p, list != nullptr, (long long)nd * nt, loose);
   if (!cl) {
     int sr = large_scratch(p, (long long)nd * nt, nb);
     if (sr) return sr;
@@ -962,9 +971,9 @@ static int run_large(mfb_plan *p, int d0, int nd, int t0, int nt, const int32_t 
   a.tw_lo = c.tw_lo;
   a.lo_bits = c.lo_bits;
   a.ws = (int)start; a.we = (int)end;
-  a.binsize = binsize > p->n ? (int)p->n : (int)binsize;
+  a.binsize = bs;
   a.nb = (int)nb;
-  a.seg = bin_lanes(a.binsize, a.ws, c.N1, c.N2);
+  a.seg = seg;
   a.t2 = threshold > 0.f ? threshold * threshold : 0.f;
   a.out_idx = (long long *)idx;
   a.out_val = (float2 *)val;

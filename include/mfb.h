@@ -109,8 +109,8 @@ int mfb_set_packed(mfb_plan *p, int on);
    in one launch with no scratch; mode 2 the same with 4 / 8 CTAs of 512
    threads, one per SM.  Same arithmetic, identical results.  Without a call, a
    run takes the faster on a B200: at n = 32768 mode 1 for row lists, dense blocks
-   of up to 64 pairs and captured runs, mode 0 for larger blocks (1.7x faster
-   at 1024 pairs); at 65536 mode 0.  A call fixes the mode for the plan's life, also
+   of up to 64 pairs (128 at threshold 0 with bins that warps do not share) and captured
+   runs, mode 0 for larger blocks (1.7x faster at 1024 pairs); at 65536 mode 0.  A call fixes the mode for the plan's life, also
    mode 1, which at n = 32768 then serves large blocks too. */
 int mfb_set_cluster(mfb_plan *p, int mode);
 /* MFB_ERR_CUDA, once, if a dependency wait inside a run of this plan ran out (the

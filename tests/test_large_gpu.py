@@ -563,6 +563,12 @@ def test_many_bins(n, binsize, win):
 
 @pytest.mark.parametrize("n, nd, nt, nb, thr", [
     (65536, 1, 1, 50, 0.0),
+    (32768, 1, 128, 50, 0.0),        # the last on clusters
+    (32768, 1, 129, 50, 0.0),        # on the launches per batch
+    (32768, 1, 65, 50, 600.0),       # in the persistent kernel
+    (32768, 1, 96, 4090, 0.0),
+    (65536, 1, 16, 4090, 0.0),       # 2^20 lags of many bins, and one pair more
+    (65536, 1, 17, 4090, 0.0),
     (65536, 2, 64, 50, 0.0),         # 2^23 lags: the last on the launches per batch
     (65536, 3, 43, 50, 0.0),         # the first in the persistent kernel
     (65536, 1, 1, 4090, 900.0),
