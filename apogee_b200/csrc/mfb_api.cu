@@ -337,7 +337,7 @@ static int large2_attr(LargeConst &c, int sms) {
   if (b < 1) return fail(MFB_ERR_CUDA, "large kernel (%d x %d) cannot be resident", N1, N2);
   c.units_a = N1 / large2_cols<N2>();
   c.units_b = N2 / (256 / (N1 / 16));
-  c.grid2 = 2 * sms;      // two CTAs per SM (registers, and shared memory at any number of bins)
+  c.grid2 = 2 * sms;      // two CTAs per SM (registers, and shared memory but for some runs of many bins)
   LargeArgs a;
   memset(&a, 0, sizeof a);
   a.n = N1 * N2;
