@@ -567,7 +567,8 @@ extern "C" size_t mfb_nbins(size_t n, size_t binsize, size_t start, size_t end) 
 // [1] for runs captured by a caller, whose order nobody here knows.
 struct LargeScratch {
   int device;
-  char *rows = nullptr, *state[2] = {nullptr, nullptr};   // state: one allocation
+  char *rows = nullptr, *state[2] = {nullptr, nullptr};   // one allocation, until state grows
+  char *grown = nullptr;                                  // state's own, after that
   size_t rows_bytes = 0, state_bytes = 0;                 // state_bytes: each
   size_t refused = SIZE_MAX;                              // rows the device had no room for
   cudaEvent_t used = nullptr;         // after the last use outside a capture
@@ -638,7 +639,7 @@ struct DeviceGuard {
 LargeScratch::~LargeScratch() {
   DeviceGuard dg(device);
   cudaFree(rows);
-  cudaFree(state[0]);
+  cudaFree(grown);
   for (char *k : kept) cudaFree(k);
   if (used) cudaEventDestroy(used);
 }
@@ -815,7 +816,8 @@ static int large_status(const mfb_plan *p) {
 }
 // Keeps or frees an outgrown allocation.
 static void large_drop(LargeScratch &s, char *block) {
-  if (s.captured && block) { s.kept.push_back(block); return; }
+  if (!block) return;
+  if (s.captured) { s.kept.push_back(block); return; }
   cudaDeviceSynchronize();
   cudaFree(block);
 }
@@ -830,32 +832,41 @@ static int large_scratch(mfb_plan *p, long long pairs, size_t nb) {
   cudaError_t e = cudaSuccess;
   if (!s.used) e = cudaEventCreateWithFlags(&s.used, cudaEventDisableTiming);
   if (e == cudaSuccess && !p->err) e = take_err_word(&p->err);
+  // records: as many as the bins ask for, two slots of LARGE_MAX_BINS at least
+  const size_t state = std::max(std::max(large_state_bytes(ring, nb), large_state_bytes(2, LARGE_MAX_BINS)),
+                                s.state_bytes);
+  char *fresh = nullptr;
   if (e == cudaSuccess && s.rows_bytes < rows) {
+    // one block for rows and state: an allocation costs a first run about 0.3 ms
     large_drop(s, s.rows);
-    s.rows = nullptr;
-    s.rows_bytes = 0;
+    large_drop(s, s.grown);
+    s.rows = s.grown = s.state[0] = s.state[1] = nullptr;
+    s.rows_bytes = s.state_bytes = 0;
+    s.captured = false;
     s.generation++;
-    while ((e = cudaMalloc(&s.rows, rows)) == cudaErrorMemoryAllocation && rows > 2 * slot) {
+    while ((e = cudaMalloc(&s.rows, rows + 2 * state)) == cudaErrorMemoryAllocation && rows > 2 * slot) {
       cudaGetLastError();             // a shorter ring is slower, no more
       s.refused = rows;
       rows = std::max(2 * slot, rows / 2);
     }
-    if (e == cudaSuccess) s.rows_bytes = rows;
-  }
-  // records: as many as the bins ask for, two slots of LARGE_MAX_BINS at least
-  const size_t state = std::max(large_state_bytes(ring, nb), large_state_bytes(2, LARGE_MAX_BINS));
-  if (e == cudaSuccess && s.state_bytes < state) {
-    large_drop(s, s.state[0]);
-    s.state[0] = s.state[1] = nullptr;
+    if (e == cudaSuccess) {
+      s.rows_bytes = rows;
+      fresh = s.rows + rows;
+    }
+  } else if (e == cudaSuccess && s.state_bytes < state) {
+    large_drop(s, s.grown);
+    s.grown = s.state[0] = s.state[1] = nullptr;
     s.state_bytes = 0;
     s.generation++;
-    e = cudaMalloc(&s.state[0], 2 * state);
-    if (e == cudaSuccess) {
-      s.state[1] = s.state[0] + state;
-      s.state_bytes = state;
-      e = cudaMemset(s.state[0], 0, 2 * state);
-      if (e == cudaSuccess) e = cudaDeviceSynchronize();   // before any stream uses it
-    }
+    e = cudaMalloc(&s.grown, 2 * state);
+    fresh = s.grown;
+  }
+  if (e == cudaSuccess && fresh) {
+    s.state[0] = fresh;
+    s.state[1] = fresh + state;
+    s.state_bytes = state;
+    e = cudaMemset(fresh, 0, 2 * state);
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();   // before any stream uses it
   }
   if (e != cudaSuccess) {
     cudaGetLastError();
