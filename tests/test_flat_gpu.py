@@ -300,12 +300,14 @@ def _same_up_to_near_ties(i1, i2, z):
     (5, 77, 512, 3.0),        # odd nt, thresholded
     (3, 1, 768, 0.0),         # one template: every pair on its own data row; a short last bin
     (1, 3, 4096, 2.0),        # fewer pairs than slots, one bin
+    (3, 1, 64, 0.0),          # 64 bins of a quarter block: the general kernel either way
 ])
 def test_packed_kernel_matches_one_pair_kernel_and_oracle(nd, nt, binsize, threshold):
     """n = 4096, bins of whole 256-lag blocks: the kernel that mfb_set_packed switches on
     (flatw_kernel) must meet the oracle's bar and equal the general kernel bit
     for bit (dense, listed and record output, counts: both form their twiddles
-    with the same operations); listed rows equal the dense run's rows bit for bit."""
+    with the same operations); listed rows equal the dense run's rows bit for bit.
+    Bins off the grid run on the general kernel whatever the switch says."""
     import torch
     import apogee_b200 as mf
     from apogee_b200 import _lib
